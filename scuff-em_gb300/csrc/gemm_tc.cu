@@ -24,8 +24,6 @@
 //            (C loads issued before the TMEM read so they overlap)
 // Every mbarrier wait is bounded; on timeout the CTA records an error code,
 // drains its outstanding TMA copies (bounded), frees its TMEM and exits.
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cstdint>
@@ -33,6 +31,7 @@
 #include <cstdlib>
 #include "bem_math.cuh"
 #include "gbem_internal.h"
+#include "tc_ptx.cuh"
 
 namespace gbem {
 
@@ -42,87 +41,10 @@ constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTE
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 static_assert((2 * STAGES + 5) * 8 + 4 <= 256, "barrier area");
 constexpr uint32_t TMEM_COLS = 256;
-constexpr long long SPIN_LIMIT = 1ll << 20;  // bounded waits (about a second at most)
+constexpr uint32_t IDESC = idesc_bf16(BM, BN);
 }  // namespace tc
 
 __device__ int g_tc_error = 0;
-
-// ---------------- PTX helpers ----------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait; returns false on timeout
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (long long it = 0; it < tc::SPIN_LIMIT; it++)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-          smem_u32(dst)),
-      "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
-}
-
-__device__ __forceinline__ uint64_t sdesc_sw128(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)(16 >> 4) << 16;    // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;  // stride byte offset: 8 rows x 128 B
-  d |= (uint64_t)1 << 46;            // descriptor version for tcgen05
-  d |= (uint64_t)2 << 61;            // 128-byte swizzle
-  return d;
-}
-
-// instruction descriptor: D f32, A/B bf16, both K-major, M = 128, N = 256
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tc::BN >> 3) << 17) |
-                           ((uint32_t)(tc::BM >> 4) << 24);
-
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(IDESC), "r"(accumulate));
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
-}
 
 // ---------------- split packing ----------------
 __device__ __forceinline__ void split_bf16(float x, __nv_bfloat16* hi, __nv_bfloat16* lo) {
@@ -282,7 +204,7 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_kernel(const __grid_constant__
           uint32_t a0 = smem_u32(tiles + s * tc::STAGE_BYTES), b0 = a0 + tc::A_BYTES;
           for (int kk = 0; kk < tc::BK / 16; kk++) {
             uint64_t da = sdesc_sw128(a0 + kk * 32), db = sdesc_sw128(b0 + kk * 32);
-            umma_f16(d, da, db, (kb > 0 || kk > 0) ? 1u : 0u);
+            umma_f16(d, da, db, tc::IDESC, (kb > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(&empty[s]);
         }
@@ -342,24 +264,24 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_kernel(const __grid_constant__
 }
 
 // ---------------- host side ----------------
-static PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
     cudaDriverEntryPointQueryResult q;
     void* p = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-  }
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return (PFN_cuTensorMapEncodeTiled_v12000)p;
+  }();
   return fn;
 }
 
-static bool make_map(CUtensorMap* map, const void* ptr, int rows, int Kp, int box_rows) {
-  auto enc = get_encode();
+bool make_bf16_map(CUtensorMap* map, const void* ptr, long long rows, int cols, int box_rows) {
+  auto enc = tensor_map_encoder();
   if (!enc) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)Kp * 2};
-  cuuint32_t box[2] = {(cuuint32_t)tc::BK, (cuuint32_t)box_rows};
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -403,7 +325,7 @@ bool tc_gemm_update(cx<float>* C, long long ldc, const cx<float>* A, long long l
     launch_pdl(zero_pad, dim3((unsigned)(((long long)2 * n * pw + 255) / 256)), dim3(256), 0, s, pb, 2LL * n, 6 * k, Kp);
   }
   CUtensorMap ma, mb;
-  if (!make_map(&ma, pa, m, Kp, tc::BM) || !make_map(&mb, pb, 2 * n, Kp, tc::BN)) return false;
+  if (!make_bf16_map(&ma, pa, m, Kp, tc::BM) || !make_bf16_map(&mb, pb, 2 * n, Kp, tc::BN)) return false;
   static bool attr = false;
   if (!attr) {
     *err = allow_max_smem(tc_gemm_kernel);
