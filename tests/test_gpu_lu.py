@@ -164,3 +164,41 @@ def test_panel_width_tuning_is_reported():
     # normwise backward error of the complex-FP32 solve (split-BF16 updates
     # keep ~16 bits per product: 1.0e-4 measured at this size)
     assert np.linalg.norm(A @ x - b) / (np.linalg.norm(A, 2) * np.linalg.norm(x)) < 1e-3
+
+
+def _strip(n):
+    """An open PEC strip of n + 1 triangles: n interior edges, N = n."""
+    from gbem import RWGGeometry
+    V = np.array([[0.5 * i, i % 2, 0.01 * i * i / (n + 1)] for i in range(n + 3)], dtype=np.float64)
+    P = np.array([[i, i + 1, i + 2] if i % 2 == 0 else [i + 1, i, i + 2] for i in range(n + 1)], dtype=np.int32)
+    return RWGGeometry([{"V": V, "P": P, "material": None}])
+
+
+@pytest.mark.parametrize("N", [1, 2, 15, 16, 17, 31, 33, 48, 63, 64, 65, 511, 512, 513, 529, 1030])
+def test_complex64_leaf_edges(N):
+    """C64 LU where a 16-column leaf, a pair of leaves, a one-CTA leaf or a
+    panel ends.  Up to N = 65 every update is FP32 arithmetic: backward error
+    within N 2^-24 times 4 (complex products) of |L||U|; larger sizes have
+    split-BF16 updates (2^-16 per product)."""
+    import scipy.linalg as sl
+    from gbem import C64
+    from gbem.api import HMatrix
+    G = _strip(N)
+    M = HMatrix(G, C64)
+    assert M.N == N
+    rng = np.random.default_rng(N)
+    A = (rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))).astype(np.complex64)
+    M.set(A)
+    assert M.LUFactorize() == 0
+    LU = M.numpy().astype(np.complex128)
+    L, U = np.tril(LU, -1) + np.eye(N), np.triu(LU)
+    perm = np.arange(N)
+    for i, p in enumerate(M.ipiv - 1):
+        assert i <= p < N
+        perm[[i, p]] = perm[[p, i]]
+    u = 2.0 ** -24 if N <= 65 else 2.0 ** -16
+    err = np.abs(A.astype(np.complex128)[perm] - L @ U)
+    assert (err <= 4 * N * u * (np.abs(L) @ np.abs(U))).all()
+    assert np.abs(L).max() <= np.sqrt(2.0) * (1 + 1e-5)
+    if N <= 65:
+        assert np.array_equal(M.ipiv - 1, sl.lu_factor(A)[1])
