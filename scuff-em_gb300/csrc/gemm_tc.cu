@@ -164,31 +164,35 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_kernel(const __grid_constant__
   if (warp == 0) {
     if (lane == 0) {
       // producer: one ring of STAGES slots across all of this CTA's tiles
-      long long g = 0, issued = 0;
+      RingPos<tc::STAGES> r;
+      int issued = 0;  // stages in use
       bool ok = true;
       for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-        const int tm = t % mt, tn = t / mt;
-        for (int kb = 0; kb < kblocks; kb++, g++) {
-          const int s = (int)(g % tc::STAGES);
-          if (g >= tc::STAGES) {
-            if (!mbar_wait(&empty[s], (uint32_t)(((g / tc::STAGES) - 1) & 1))) { atomicExch(&s_fail, 1); ok = false; break; }
-          }
-          unsigned char* sa = tiles + s * tc::STAGE_BYTES;
-          mbar_arrive_expect_tx(&full[s], tc::STAGE_BYTES);
-          tma_load_2d(sa, &mapA, &full[s], kb * tc::BK, tm * tc::BM);
-          tma_load_2d(sa + tc::A_BYTES, &mapB, &full[s], kb * tc::BK, tn * tc::BN);
-          issued = g + 1;
+        const int ya = (t % mt) * tc::BM, yb = (t / mt) * tc::BN;
+        for (int kb = 0; kb < kblocks; kb++, r.next()) {
+          // a fresh barrier's previous phase counts as complete
+          if (!mbar_wait(&empty[r.s], r.phase ^ 1u)) { atomicExch(&s_fail, 1); ok = false; break; }
+          unsigned char* sa = tiles + r.s * tc::STAGE_BYTES;
+          mbar_arrive_expect_tx(&full[r.s], tc::STAGE_BYTES);
+          tma_load_3d(sa, &mapA, &full[r.s], 0, ya, kb);
+          tma_load_3d(sa + tc::A_BYTES, &mapB, &full[r.s], 0, yb, kb);
+          issued = min(issued + 1, tc::STAGES);
         }
       }
-      // drain: no TMA write may still be in flight when the CTA exits
-      for (long long q = (issued > tc::STAGES ? issued - tc::STAGES : 0); q < issued; q++)
-        mbar_wait(&full[q % tc::STAGES], (uint32_t)((q / tc::STAGES) & 1));
+      // drain: no TMA write may still be in flight when the CTA exits (the
+      // last pass of every stage used)
+      for (int q = 0; q < issued; q++) {
+        if (r.s == 0) { r.s = tc::STAGES; r.phase ^= 1u; }
+        r.s--;
+        mbar_wait(&full[r.s], r.phase);
+      }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      long long g = 0;
+      RingPos<tc::STAGES> r;
       bool ok = true;
       int i = 0;
+      const uint64_t desc0 = sdesc_sw128(smem_u32(tiles));  // addresses count 16 bytes in the low bits
       for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, i++) {
         const int acc = i & 1;
         if (i >= 2 && !mbar_wait(&acc_empty[acc], (uint32_t)(((i >> 1) - 1) & 1))) {
@@ -197,16 +201,14 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_kernel(const __grid_constant__
         }
         tc_fence_after();
         const uint32_t d = tmem + (uint32_t)(acc * tc::TMEM_COLS);
-        for (int kb = 0; kb < kblocks; kb++, g++) {
-          const int s = (int)(g % tc::STAGES);
-          if (!mbar_wait(&full[s], (uint32_t)((g / tc::STAGES) & 1))) { atomicExch(&s_fail, 1); ok = false; break; }
+        for (int kb = 0; kb < kblocks; kb++, r.next()) {
+          if (!mbar_wait(&full[r.s], r.phase)) { atomicExch(&s_fail, 1); ok = false; break; }
           tc_fence_after();
-          uint32_t a0 = smem_u32(tiles + s * tc::STAGE_BYTES), b0 = a0 + tc::A_BYTES;
-          for (int kk = 0; kk < tc::BK / 16; kk++) {
-            uint64_t da = sdesc_sw128(a0 + kk * 32), db = sdesc_sw128(b0 + kk * 32);
-            umma_f16(d, da, db, tc::IDESC, (kb > 0 || kk > 0) ? 1u : 0u);
-          }
-          umma_commit(&empty[s]);
+          const uint64_t da = desc0 + (uint32_t)(r.s * (tc::STAGE_BYTES >> 4)), db = da + (tc::A_BYTES >> 4);
+#pragma unroll
+          for (int kk = 0; kk < tc::BK / 16; kk++)
+            umma_f16(d, da + 2 * kk, db + 2 * kk, tc::IDESC, (kb | kk) ? 1u : 0u);
+          umma_commit(&empty[r.s]);
         }
         if (ok) umma_commit(&acc_full[acc]);
       }
@@ -276,14 +278,14 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-bool make_bf16_map(CUtensorMap* map, const void* ptr, long long rows, int cols, int box_rows) {
+bool make_bf16_map(CUtensorMap* map, const void* ptr, long long rows, int cols, int box_rows, int kbox) {
   auto enc = tensor_map_encoder();
   if (!enc) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+  cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)};
+  cuuint64_t strides[2] = {(cuuint64_t)cols * 2, 128};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, (cuuint32_t)kbox};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
@@ -325,7 +327,7 @@ bool tc_gemm_update(cx<float>* C, long long ldc, const cx<float>* A, long long l
     launch_pdl(zero_pad, dim3((unsigned)(((long long)2 * n * pw + 255) / 256)), dim3(256), 0, s, pb, 2LL * n, 6 * k, Kp);
   }
   CUtensorMap ma, mb;
-  if (!make_bf16_map(&ma, pa, m, Kp, tc::BM) || !make_bf16_map(&mb, pb, 2 * n, Kp, tc::BN)) return false;
+  if (!make_bf16_map(&ma, pa, m, Kp, tc::BM, 1) || !make_bf16_map(&mb, pb, 2 * n, Kp, tc::BN, 1)) return false;
   static bool attr = false;
   if (!attr) {
     *err = allow_max_smem(tc_gemm_kernel);

@@ -7,7 +7,7 @@
 
 namespace gbem {
 
-constexpr long long TC_SPIN_LIMIT = 1ll << 20;  // bounded waits (about a second at most)
+constexpr int TC_SPIN_LIMIT = 1 << 20;  // bounded waits (about a second at most)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -31,16 +31,27 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 // bounded wait; returns false on timeout
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (long long it = 0; it < TC_SPIN_LIMIT; it++)
+  for (int it = 0; it < TC_SPIN_LIMIT; it++)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
 
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
+// Position in a ring of N stages and the parity of its current pass, stepped
+// instead of divided out: the producer's and the MMA issuer's single threads
+// bound a k-step by their own instruction chains.
+template <int N> struct RingPos {
+  int s = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next() {
+    if (++s == N) { s = 0; phase ^= 1u; }
+  }
+};
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
           smem_u32(dst)),
-      "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
 
@@ -82,14 +93,27 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
 }
 
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
 // instruction descriptor of kind::f16: D f32, A and B bf16, both K-major
 constexpr uint32_t idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 // host: the driver's tensor-map encoder, and the map of a row-major bf16
-// matrix (rows x cols) read in boxes of 64 columns x box_rows rows, 128-byte swizzle
+// matrix (rows x cols, cols a multiple of 64) read in boxes of box_rows rows
+// and kbox blocks of 64 columns (block after block in shared memory, 128-byte
+// swizzle); coordinates {0, row, block}
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
-bool make_bf16_map(CUtensorMap* map, const void* ptr, long long rows, int cols, int box_rows);
+bool make_bf16_map(CUtensorMap* map, const void* ptr, long long rows, int cols, int box_rows, int kbox);
 
 }  // namespace gbem
