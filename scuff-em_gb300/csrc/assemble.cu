@@ -11,18 +11,19 @@
 //  near_kernel    per frequency: every other pair with rRel <= 4 (FP64,
 //                 desingularised 6x6 rule + static table, or high-order rule
 //                 in the short-wavelength regime).
-//  tile_kernel<T> per frequency: one CTA per tile of TE x TE edge pairs.
-//                 Computes the 6x6-rule bilinear moments of every panel pair
-//                 the tile touches once (T = float for the mixed form,
-//                 double for the plain form), forms the up-to-9 (Qa,Qb)
-//                 combinations, and writes the tile's matrix entries (and
-//                 the mirrored tile) with coalesced stores.  Each edge-pair
-//                 entry gathers its four panel-pair contributions from
-//                 per-(edge pair, P/M side) slots in shared memory, so the
-//                 sum is deterministic and needs no atomics.
+//  ppair_kernel   per frequency: the 6x6-rule integrals of every far panel
+//  ppair64_kernel pair, once, for the nine (Qa,Qb) combinations (float-float
+//                 for the mixed form, FP64 for the plain form).
+//  stamp_kernel   per frequency: one CTA per tile of TE x TE edge pairs sums
+//  stamp64_kernel each entry's four panel-pair values in a fixed order (no
+//                 atomics) and writes the tile and its mirror with coalesced
+//                 stores.
+//  tile_kernel    both passes of the plain form in one, where the pair values
+//                 find no room.
 #include <cstdio>
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <vector>
 #include "adjoint.cuh"
 #include "bem_math.cuh"
@@ -38,6 +39,10 @@ namespace gbem {
 __constant__ double c_lo64[18];
 __constant__ FFRule c_ffrule;      // the LO rule as float-float (mixed far field)
 __constant__ SinCosTab c_sctab;    // cos, sin of j pi/64 as float-float
+struct SinCosTab64 {
+  double c[128], s[128];  // cos, sin of j pi/64
+};
+__constant__ SinCosTab64 c_sctab64;
 static const double h_lo[18] = {
     0.0915762135098, 0.0915762135098, 0.0549758718276, 0.8168475729805, 0.0915762135098, 0.0549758718276,
     0.0915762135098, 0.8168475729805, 0.0549758718276, 0.1081030181681, 0.4459484909160, 0.1116907948390,
@@ -92,7 +97,13 @@ static gbem_status init_rules() {
   fill_ff_rule(h_lo, &ffr);
   SinCosTab sct;
   fill_sincos_tab(&sct);
+  SinCosTab64 sct64;
+  for (int j = 0; j < 128; j++) {
+    sct64.c[j] = cos(j * (3.14159265358979323846 / 64.0));
+    sct64.s[j] = sin(j * (3.14159265358979323846 / 64.0));
+  }
   cudaError_t e = cudaMemcpyToSymbol(c_lo64, h_lo, sizeof h_lo);
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_sctab64, &sct64, sizeof sct64);
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_ffrule, &ffr, sizeof ffr);
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_sctab, &sct, sizeof sct);
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_ho, ho, sizeof ho);
@@ -149,6 +160,8 @@ struct DevBlock {
   int4* edge_a = nullptr;  // per row edge: P panel, its Q index, M panel, its Q index
   int4* edge_b = nullptr;  // per column edge, likewise
   int2* ecol = nullptr;    // per column edge: stripe-local P, M panel index
+  int* emin = nullptr;     // per row panel: its first edge (ne: none)
+  int* emax = nullptr;     // per column panel: its last edge (-1: none)
 };
 
 template <typename Tp>
@@ -229,6 +242,16 @@ gbem_status upload_geometry(Geometry* g) {
     if (e == cudaSuccess) e = dupload(&db->edge_a, ea.data(), ea.size());
     if (e == cudaSuccess) e = dupload(&db->edge_b, eb.data(), eb.size());
     if (e == cudaSuccess) e = dupload(&db->ecol, b.ecol.data(), b.ecol.size());
+    const Surface &Sa = g->S[b.sa], &Sb = g->S[b.sb];
+    std::vector<int> emin(Sa.np, Sa.ne), emax(Sb.np, -1);
+    for (int i = 0; i < Sa.ne; i++)
+      for (int c = 4; c < 6; c++)
+        if (Sa.E[8 * i + c] >= 0) emin[Sa.E[8 * i + c]] = std::min(emin[Sa.E[8 * i + c]], i);
+    for (int i = 0; i < Sb.ne; i++)
+      for (int c = 4; c < 6; c++)
+        if (Sb.E[8 * i + c] >= 0) emax[Sb.E[8 * i + c]] = std::max(emax[Sb.E[8 * i + c]], i);
+    if (e == cudaSuccess) e = dupload(&db->emin, emin.data(), emin.size());
+    if (e == cudaSuccess) e = dupload(&db->emax, emax.data(), emax.size());
     for (const Stripe& st : b.stripes) {
       DevBlock::DevStripe ds;
       ds.nrow = st.nrow; ds.ncp = (int)st.cpan.size(); ds.ntiles = (int)st.tiles.size();
@@ -273,7 +296,7 @@ void free_geometry_device(Geometry* g) {
     cudaFree(db->rows); cudaFree(db->cols); cudaFree(db->tiles); cudaFree(db->elen_a); cudaFree(db->elen_b);
     cudaFree(db->nptr); cudaFree(db->ncol); cudaFree(db->nidx); cudaFree(db->near); cudaFree(db->self_list);
     cudaFree(db->other_list); cudaFree(db->fippi); cudaFree(db->nearval);
-    cudaFree(db->edge_a); cudaFree(db->edge_b); cudaFree(db->ecol);
+    cudaFree(db->edge_a); cudaFree(db->edge_b); cudaFree(db->ecol); cudaFree(db->emin); cudaFree(db->emax);
     for (auto& st : db->stripes) { cudaFree(st.cpan); cudaFree(st.tiles); }
     delete db;
   }
@@ -998,6 +1021,285 @@ __global__ void __launch_bounds__(256) stamp_kernel(StampArgs sp) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// FP64 far field, in the same two passes: ppair64_kernel integrates every far
+// panel pair of a stripe once (the tile kernel integrates it in every tile
+// that touches it, 2.4 times on an icosphere, and forms each of its nine
+// combinations from scratch), stamp64_kernel sums the entries.  The FP64 pipe
+// bounds the first pass (2 operations per cycle and SM, everything else hides
+// behind it), so its operations are what was cut, per sample 54 (lossless
+// region) from about 95: positions from per-panel node offsets, one reciprocal
+// square root, e^{i k r} by a 128-entry table and a short Taylor series; the
+// combinations of all nine (Qa, Qb) from eight scalars of the pair (h0_all,
+// h1_all), 180 operations from 2100; real arithmetic where the wavenumber is
+// imaginary (REALK); pairs below the diagonal skipped.  Measured against the
+// tile kernel: dielectric sphere, N = 3840, 36.7 -> 10.2 ms; PEC sphere, N =
+// 480, 1.13 -> 0.32; rounded cube, N = 6084, 97.1 -> 26.1.
+// ---------------------------------------------------------------------------
+constexpr double PI64_HI = 0x1.921fb54400000p-5;  // pi/64, leading 33 bits
+constexpr double PI64_LO = 0x1.0b4611a626331p-39;
+constexpr double EXPI_MAX = 5.0e4;                // j < 2^20: j PI64_HI is exact
+
+// e^{ix}: x = j pi/64 + t, |t| <= pi/128, the Taylor series of sin t and
+// cos t - 1 to t^7 and t^6 (remainders below 4e-18), added onto the table's
+// values; error about one unit in the last place
+__device__ __forceinline__ void expi64(double x, const SinCosTab64& tab, double* c, double* s) {
+  if ((__double2hiint(x) & 0x7fffffff) >= 0x40e86a00) {  // |x| >= EXPI_MAX, infinite or NaN
+    sincos(x, s, c);
+    return;
+  }
+  const double magic = 6755399441055744.0;  // 1.5 * 2^52: rounds to an integer in the low word
+  const double y = fma(x, 64.0 / 3.14159265358979323846, magic);
+  const int j = __double2loint(y) & 127;
+  const double jf = y - magic;
+  const double t = fma(-jf, PI64_LO, fma(-jf, PI64_HI, x));
+  const double t2 = t * t;
+  const double sn = fma(t * t2, fma(t2, fma(t2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), t);
+  const double cm = t2 * fma(t2, fma(t2, -1.0 / 720.0, 1.0 / 24.0), -0.5);
+  const double c0 = tab.c[j], s0 = tab.s[j];
+  *c = c0 + fma(c0, cm, -(s0 * sn));
+  *s = s0 + fma(s0, cm, c0 * sn);
+}
+
+// the 6x6-rule moments of one far pair (definition of pair_moments).
+// KIND 0: k real, 1: any k, 2: k imaginary (G and Psi real, E = double).
+// pa0/A/B: the row panel's V0 - V0 of the column panel and edges; ob: the
+// column panel's node offsets u' Ab + v' Bb; w4: the rule's weights over 4 pi.
+template <int KIND, typename E>
+__device__ __forceinline__ void moments64(const double* D0, const double* A, const double* B, const double* ob, double kre,
+                                          double kim, const double* w4, const SinCosTab64& tab, E* MG, E* MP) {
+#pragma unroll
+  for (int m = 0; m < 9; m++) MG[m] = MP[m] = E{};
+#pragma unroll 1
+  for (int i = 0; i < 6; i++) {
+    const double u = c_lo64[3 * i], v = c_lo64[3 * i + 1], wi = c_lo64[3 * i + 2];
+    double pa[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) pa[c] = fma(v, B[c], fma(u, A[c], D0[c]));
+    E SG[3], SP[3];
+#pragma unroll
+    for (int b = 0; b < 3; b++) SG[b] = SP[b] = E{};
+#pragma unroll 2
+    for (int j = 0; j < 6; j++) {
+      const double x = pa[0] - ob[3 * j], y = pa[1] - ob[3 * j + 1], z = pa[2] - ob[3 * j + 2];
+      const double r2 = fma(z, z, fma(y, y, x * x));
+      const double rinv = rsqrt(r2), r = r2 * rinv;
+      const double up = c_lo64[3 * j], vp = c_lo64[3 * j + 1];
+      double amp = w4[j] * rinv;
+      if (KIND != 0) amp *= exp(-kim * r);
+      E phi, psi;
+      const double fre = (KIND == 0 ? -rinv : -kim - rinv) * rinv;  // (ik - 1/r)/r
+      if constexpr (KIND == 2) {
+        phi = amp;
+        psi = amp * fre;
+      } else {
+        double c, s;
+        expi64(kre * r, tab, &c, &s);
+        phi = mk(amp * c, amp * s);
+        psi = phi * mk(fre, kre * rinv);
+      }
+      SG[0] = SG[0] + phi; SP[0] = SP[0] + psi;
+      SG[1] = SG[1] + up * phi; SP[1] = SP[1] + up * psi;
+      SG[2] = SG[2] + vp * phi; SP[2] = SP[2] + vp * psi;
+    }
+    const double a[3] = {wi, wi * u, wi * v};
+#pragma unroll
+    for (int al = 0; al < 3; al++)
+#pragma unroll
+      for (int b = 0; b < 3; b++) {
+        MG[3 * al + b] = MG[3 * al + b] + a[al] * SG[b];
+        MP[3 * al + b] = MP[3 * al + b] + a[al] * SP[b];
+      }
+  }
+}
+
+struct PPair64Args {
+  const double* pv;   // per global panel: 9 vertex coordinates
+  const double* pc;   // per global panel: centroid, radius
+  const int* cpan;    // the stripe's column panels (surface-local)
+  const int* emin;    // per row panel: its first edge; per column panel: its last
+  const int* emax;
+  int offa, offb;     // global index of the first panel of each surface
+  int nrow, ncp, sym;
+  double2* out;       // [NC][9][ncp][nrow]; x = NaN: a near pair
+};
+constexpr int PP64_COLS = 8, PP64_SLOTS = 32 + PP64_COLS, PP64_THREADS = 32 * PP64_COLS;
+
+__device__ __forceinline__ cx<double> scaled(cx<double> f, cx<double> h) { return f * h; }
+__device__ __forceinline__ cx<double> scaled(cx<double> f, double h) { return h * f; }
+
+template <int NC, bool REALK>
+__global__ void __launch_bounds__(PP64_THREADS, 1) ppair64_kernel(PPair64Args p, RegionArgs ra) {
+  using E = typename std::conditional<REALK, double, cx<double>>::type;
+  __shared__ double s_pv[PP64_SLOTS][9];
+  __shared__ double s_ob[PP64_COLS][18];
+  __shared__ double s_pcd[PP64_SLOTS][4];
+  __shared__ float s_cf[PP64_SLOTS][4];
+  __shared__ SinCosTab64 s_tab;
+  __shared__ double s_w4[6];
+  const int tid = threadIdx.y * 32 + threadIdx.x;
+  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * PP64_COLS;
+  auto panel_of = [&](int sl) -> int {
+    if (sl < 32) return r0 + sl < p.nrow ? p.offa + r0 + sl : -1;
+    return c0 + sl - 32 < p.ncp ? p.offb + p.cpan[c0 + sl - 32] : -1;
+  };
+  for (int q = tid; q < PP64_SLOTS * 9; q += PP64_THREADS) {
+    const int sl = q / 9, f = q - sl * 9, gp = panel_of(sl);
+    s_pv[sl][f] = gp >= 0 ? p.pv[9 * (size_t)gp + f] : 0.0;
+  }
+  for (int q = tid; q < PP64_SLOTS * 4; q += PP64_THREADS) {
+    const int sl = q / 4, f = q - sl * 4, gp = panel_of(sl);
+    if (gp >= 0) { s_pcd[sl][f] = p.pc[4 * (size_t)gp + f]; s_cf[sl][f] = (float)p.pc[4 * (size_t)gp + f]; }
+  }
+  if (!REALK)
+    for (int q = tid; q < (int)(sizeof(SinCosTab64) / 8); q += PP64_THREADS)
+      reinterpret_cast<double*>(&s_tab)[q] = reinterpret_cast<const double*>(&c_sctab64)[q];
+  if (tid < 6) s_w4[tid] = c_lo64[3 * tid + 2] * 0.079577471545947667884;  // 1/(4 pi)
+  __syncthreads();
+  for (int q = tid; q < PP64_COLS * 18; q += PP64_THREADS) {
+    const int cl = q / 18, j = (q - cl * 18) / 3, c = q % 3;
+    const double* V = s_pv[32 + cl];
+    s_ob[cl][3 * j + c] = fma(c_lo64[3 * j + 1], V[6 + c] - V[c], c_lo64[3 * j] * (V[3 + c] - V[c]));
+  }
+  __syncthreads();
+
+  const int pa = r0 + threadIdx.x, cl = c0 + threadIdx.y;
+  if (pa >= p.nrow || cl >= p.ncp) return;
+  // entries on and above the diagonal only: no edge of pa precedes one of the column panel
+  if (p.sym && p.emin[pa] > p.emax[p.cpan[cl]]) return;
+  const int ia = threadIdx.x, ib = 32 + threadIdx.y;
+  const size_t cs = (size_t)p.ncp * p.nrow;  // stride of one (field, combination) plane
+  double2* out = p.out + (size_t)cl * p.nrow + pa;
+  if (!tile_pair_far(s_cf[ia], s_cf[ib], s_pcd[ia], s_pcd[ib])) {
+    const double marker = __longlong_as_double(0x7ff8000000000000ll);  // quiet NaN: a near pair
+    for (int c = 0; c < 9; c++) out[c * cs] = make_double2(marker, 0.0);
+    return;
+  }
+  PairGeom<double> g;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    g.D0[c] = s_pv[ia][c] - s_pv[ib][c];
+    g.Aa[c] = s_pv[ia][3 + c] - s_pv[ia][c]; g.Ba[c] = s_pv[ia][6 + c] - s_pv[ia][c];
+  }
+  bool first = true;
+#pragma unroll 1
+  for (int r = 0; r < ra.nreg; r++) {
+    const cx<double> k = ra.k[r];
+    if (k.re == 0.0 && k.im == 0.0) continue;
+    E MG[9], MP[9];
+    if constexpr (REALK) {
+      moments64<2>(g.D0, g.Aa, g.Ba, s_ob[threadIdx.y], 0.0, k.im, s_w4, s_tab, MG, MP);
+    } else {
+      if (k.im == 0.0) moments64<0>(g.D0, g.Aa, g.Ba, s_ob[threadIdx.y], k.re, 0.0, s_w4, s_tab, MG, MP);
+      else moments64<1>(g.D0, g.Aa, g.Ba, s_ob[threadIdx.y], k.re, k.im, s_w4, s_tab, MG, MP);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      g.Ab[c] = s_pv[ib][3 + c] - s_pv[ib][c]; g.Bb[c] = s_pv[ib][6 + c] - s_pv[ib][c];
+    }
+    PairScalars<double> ps;
+    pair_scalars(g, &ps);
+    const cx<double> m4 = cdiv(mk(-4.0, 0.0), k * k);
+    E H[9], m4e;
+    if constexpr (REALK) m4e = m4.re; else m4e = m4;
+    h0_all(ps, MG, m4e, H);
+    const size_t fs = 9 * cs;  // stride of one field
+    auto put = [&](int f, int c, cx<double> v) {
+      double2* o = out + f * fs + c * cs;
+      if (!first) { const double2 z = *o; v = v + mk(z.x, z.y); }
+      *o = make_double2(v.re, v.im);
+    };
+#pragma unroll
+    for (int c = 0; c < 9; c++) {
+      put(0, c, scaled(ra.pf1[r], H[c]));
+      if (NC > 2) put(2, c, scaled(ra.pf3[r], H[c]));
+    }
+    if (NC > 1) {
+      h1_all(ps, MP, H);
+#pragma unroll
+      for (int c = 0; c < 9; c++) put(1, c, scaled(ra.pfc[r], H[c]));
+    }
+    first = false;
+  }
+  if (first)  // every common region has k = 0: zero contribution
+    for (int c = 0; c < 9 * NC; c++) out[c * cs] = make_double2(0.0, 0.0);
+}
+
+struct Stamp64Args {
+  TileArgs ta;            // output placement, near table, edge blocks
+  const int2* tiles;      // the stripe's tiles
+  const int4* edge_a;     // per row edge: P panel, its Q index, M panel, its Q index (surface-local; -1: none)
+  const int4* edge_b;     // per column edge, likewise
+  const int2* ecol;       // per column edge: stripe-local index of its P, M panel
+  int offb;               // global index of the first column-surface panel
+  const double2* ppv;     // pass-1 values [NC][9][ncp][nrow]
+  int nrow, ncp;
+};
+
+// pass 2, as stamp_kernel: La Lb ((PP - PM) - (MP - MM)), a missing panel's value zero
+template <int NC>
+__global__ void __launch_bounds__(256) stamp64_kernel(Stamp64Args sp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cx<double>* s_val = reinterpret_cast<cx<double>*>(smem_raw);  // [TE][TE][NC]
+  const TileArgs& a = sp.ta;
+  const int2 tile = sp.tiles[blockIdx.x];
+  const DevEdgeBlock* RB = a.rows + tile.x;
+  const DevEdgeBlock* CB = a.cols + tile.y;
+  const int NR = RB->ne, NCc = CB->ne;
+  const bool diag = a.sym && tile.x == tile.y;
+  const size_t cs = (size_t)sp.ncp * sp.nrow, fs = 9 * cs;
+  for (int q = threadIdx.x; q < NR * NCc; q += blockDim.x) {
+    const int i = q % NR, j = q / NR;
+    if (diag && i > j) continue;
+    const int ea = RB->e0 + i, eb = CB->e0 + j;
+    const int4 A = sp.edge_a[ea], B = sp.edge_b[eb];
+    const int2 C = sp.ecol[eb];
+    cx<double> row[2][NC];  // P - M over the column panels, per row panel
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const int pa = u ? A.z : A.x, ja = u ? A.w : A.y;
+      cx<double> v[2][NC];
+#pragma unroll
+      for (int w = 0; w < 2; w++) {
+        const int pb = w ? B.z : B.x, jb = w ? B.w : B.y, cl = w ? C.y : C.x;
+#pragma unroll
+        for (int c = 0; c < NC; c++) v[w][c] = mk(0.0, 0.0);
+        if (pa < 0 || pb < 0) continue;
+        const double2* src = sp.ppv + (size_t)(3 * ja + jb) * cs + (size_t)cl * sp.nrow + pa;
+        const double2 f0 = src[0];
+        if (!isnan(f0.x)) {
+          v[w][0] = mk(f0.x, f0.y);
+#pragma unroll
+          for (int c = 1; c < NC; c++) { const double2 f = src[c * fs]; v[w][c] = mk(f.x, f.y); }
+        } else {
+          // near pair: values of near_kernel / self_kernel
+          const int hit = near_hit(a, a.row_panel_offset + pa, sp.offb + pb);
+          if (hit < 0) continue;  // cannot happen: every rRel<=4 pair is listed
+          const double* nv = a.nearval + 54 * (size_t)(hit >> 1) + 6 * ((hit & 1) ? (3 * jb + ja) : (3 * ja + jb));
+#pragma unroll
+          for (int c = 0; c < NC; c++) v[w][c] = mk(nv[2 * c], nv[2 * c + 1]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < NC; c++) row[u][c] = v[0][c] - v[1][c];
+    }
+    const double L = a.elen_a[ea] * a.elen_b[eb];
+#pragma unroll
+    for (int c = 0; c < NC; c++) s_val[(size_t)(i * TE + j) * NC + c] = L * (row[0][c] - row[1][c]);
+  }
+  __syncthreads();
+  cx<double>* out = reinterpret_cast<cx<double>*>(a.out);
+  for (int pass = 0; pass < 2; pass++) {
+    if (!(a.passes & (1 << pass))) continue;
+    for (int q = threadIdx.x; q < NR * NCc; q += blockDim.x) {
+      int i, j;
+      if (!tile_entry(pass, q, NR, NCc, diag, &i, &j)) continue;
+      const cx<double>* v = s_val + (size_t)(i * TE + j) * NC;
+      store_entry(a, out, pass, RB->e0 + i, CB->e0 + j, v[0], NC > 1 ? v[1] : v[0], NC > 2 ? v[2] : v[0]);
+    }
+  }
+}
+
 static inline cx<double> cxd(double r, double i) { return mk(r, i); }
 
 template <int NC>
@@ -1009,15 +1311,12 @@ static cudaError_t launch_tiles64(const TileArgs& ta, const RegionArgs& ra, int 
   return cudaGetLastError();
 }
 
-// the two passes of the mixed far field over a block's column stripes
-template <int NC>
-static cudaError_t far_mixed(Geometry* g, const Block& b, DevBlock* db, const TileArgs& ta, const RegionArgs& ra,
-                             cudaStream_t s) {
-  const size_t need = b.max_stripe_pairs * 9 * ppair_fields<NC>() * sizeof(float);
+// the pair-value scratch of the two-pass far fields, kept on the geometry
+static cudaError_t pair_scratch(Geometry* g, size_t need) {
   cudaError_t e = cudaSuccess;
   if (need > g->ppv_bytes) {
-    // grow the scratch (kept on the geometry; the old one may still be read
-    // by earlier launches, so wait for the device before freeing it)
+    // grow (the old one may still be read by earlier launches, so wait for
+    // the device before freeing it)
     if (g->ppv) {
       e = cudaDeviceSynchronize();
       cudaFree(g->ppv);
@@ -1028,6 +1327,50 @@ static cudaError_t far_mixed(Geometry* g, const Block& b, DevBlock* db, const Ti
     if (e != cudaSuccess) return e;
     g->ppv_bytes = need;
   }
+  return e;
+}
+
+// the two passes of the FP64 far field; without room for the pair values, the
+// tile kernel, which needs none
+template <int NC>
+static cudaError_t far_fp64(Geometry* g, const Block& b, DevBlock* db, const TileArgs& ta, const RegionArgs& ra,
+                            cudaStream_t s) {
+  cudaError_t e = pair_scratch(g, b.max_stripe_pairs * 9 * NC * sizeof(double2));
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    stats_launch(ST_FAR);
+    return launch_tiles64<NC>(ta, ra, db->ntiles, s);
+  }
+  if (e == cudaSuccess) e = allow_max_smem(stamp64_kernel<NC>);
+  if (e != cudaSuccess) return e;
+  bool realk = true;
+  for (int r = 0; r < ra.nreg; r++) realk = realk && ra.k[r].re == 0.0;
+  for (const DevBlock::DevStripe& st : db->stripes) {
+    if (st.ntiles == 0 || st.ncp == 0) continue;
+    PPair64Args pp;
+    pp.pv = g->d_pv; pp.pc = g->d_pc; pp.cpan = st.cpan; pp.emin = db->emin; pp.emax = db->emax;
+    pp.offa = g->S[b.sa].panel_offset; pp.offb = g->S[b.sb].panel_offset;
+    pp.nrow = st.nrow; pp.ncp = st.ncp; pp.sym = b.sym; pp.out = (double2*)g->ppv;
+    const dim3 grid((st.nrow + 31) / 32, (st.ncp + PP64_COLS - 1) / PP64_COLS), block(32, PP64_COLS);
+    if (realk) ppair64_kernel<NC, true><<<grid, block, 0, s>>>(pp, ra);
+    else ppair64_kernel<NC, false><<<grid, block, 0, s>>>(pp, ra);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    Stamp64Args sp;
+    sp.ta = ta; sp.tiles = st.tiles; sp.edge_a = db->edge_a; sp.edge_b = db->edge_b; sp.ecol = db->ecol;
+    sp.offb = pp.offb; sp.ppv = pp.out; sp.nrow = st.nrow; sp.ncp = st.ncp;
+    stamp64_kernel<NC><<<st.ntiles, 256, TE * TE * NC * sizeof(cx<double>), s>>>(sp);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    stats_launch(ST_FAR, 2);
+  }
+  return cudaSuccess;
+}
+
+// the two passes of the mixed far field over a block's column stripes
+template <int NC>
+static cudaError_t far_mixed(Geometry* g, const Block& b, DevBlock* db, const TileArgs& ta, const RegionArgs& ra,
+                             cudaStream_t s) {
+  cudaError_t e = pair_scratch(g, b.max_stripe_pairs * 9 * ppair_fields<NC>() * sizeof(float));
+  if (e != cudaSuccess) return e;
   for (const DevBlock::DevStripe& st : db->stripes) {
     if (st.ntiles == 0 || st.ncp == 0) continue;
     PPairArgs pp;
@@ -1231,12 +1574,10 @@ gbem_status assemble_device(Geometry* g, double wr, double wi, const double* eps
     ta.out = dM; ta.ld = ld;
     int nc = (b.bpe_a == 2 && b.bpe_b == 2) ? 3 : ((b.bpe_a == 1 && b.bpe_b == 1) ? 1 : 2);
     StatTimer tf(ST_FAR, s);
-    if (precision != GBEM_PREC_MIXED) stats_launch(ST_FAR);
     if (precision == GBEM_PREC_MIXED) {
       e = nc == 1 ? far_mixed<1>(g, b, db, ta, ra, s) : nc == 2 ? far_mixed<2>(g, b, db, ta, ra, s) : far_mixed<3>(g, b, db, ta, ra, s);
     } else {
-      e = nc == 1 ? launch_tiles64<1>(ta, ra, db->ntiles, s)
-                  : nc == 2 ? launch_tiles64<2>(ta, ra, db->ntiles, s) : launch_tiles64<3>(ta, ra, db->ntiles, s);
+      e = nc == 1 ? far_fp64<1>(g, b, db, ta, ra, s) : nc == 2 ? far_fp64<2>(g, b, db, ta, ra, s) : far_fp64<3>(g, b, db, ta, ra, s);
     }
     if (e != cudaSuccess) return cuda_status(e, "tile_kernel");
   }

@@ -301,6 +301,73 @@ GB_HD void vec_combine(const PairGeom<T>& g, const VecMoments<T>& vm, int ja, in
   *H1 = h1;
 }
 
+// The same combinations from eight scalars of the pair.  With a_i in {Aa, Ba},
+// b_j in {Ab, Bb}, alpha = -a_k or 0 and beta = -b_l or 0, every product in
+// vec_combine is one of
+//   D_ij = a_i.b_j,  T_ij = D0.(a_i x b_j),  U_j = (Aa x Ba).b_j,  V_i = a_i.(Ab x Bb)
+// (triple products with a repeated vector vanish), so that all nine H0 and H1
+// cost about 180 operations on the moments in place of 230 per (Qa, Qb).
+template <typename T> struct PairScalars {
+  T D[2][2], Tr[2][2], U[2], V[2];
+};
+
+template <typename T> GB_HD void pair_scalars(const PairGeom<T>& g, PairScalars<T>* p) {
+  const T* a[2] = {g.Aa, g.Ba};
+  const T* b[2] = {g.Ab, g.Bb};
+  const T na[3] = {g.Aa[1] * g.Ba[2] - g.Aa[2] * g.Ba[1], g.Aa[2] * g.Ba[0] - g.Aa[0] * g.Ba[2],
+                   g.Aa[0] * g.Ba[1] - g.Aa[1] * g.Ba[0]};
+  const T nb[3] = {g.Ab[1] * g.Bb[2] - g.Ab[2] * g.Bb[1], g.Ab[2] * g.Bb[0] - g.Ab[0] * g.Bb[2],
+                   g.Ab[0] * g.Bb[1] - g.Ab[1] * g.Bb[0]};
+  for (int i = 0; i < 2; i++) {
+    // D0.(a_i x b_j) = b_j.(D0 x a_i)
+    const T x[3] = {g.D0[1] * a[i][2] - g.D0[2] * a[i][1], g.D0[2] * a[i][0] - g.D0[0] * a[i][2],
+                    g.D0[0] * a[i][1] - g.D0[1] * a[i][0]};
+    for (int j = 0; j < 2; j++) {
+      p->D[i][j] = a[i][0] * b[j][0] + a[i][1] * b[j][1] + a[i][2] * b[j][2];
+      p->Tr[i][j] = x[0] * b[j][0] + x[1] * b[j][1] + x[2] * b[j][2];
+    }
+    p->U[i] = na[0] * b[i][0] + na[1] * b[i][1] + na[2] * b[i][2];
+    p->V[i] = nb[0] * a[i][0] + nb[1] * a[i][1] + nb[2] * a[i][2];
+  }
+}
+
+// H0[3 ja + jb] for all nine (Qa, Qb); E is cx<T>, or T where the moments are real
+template <typename T, typename E> GB_HD void h0_all(const PairScalars<T>& p, const E* MG, E m4ok2, E* H0) {
+  const E base = p.D[0][0] * MG[4] + p.D[0][1] * MG[5] + p.D[1][0] * MG[7] + p.D[1][1] * MG[8] + m4ok2 * MG[0];
+  const E z{};
+  const E X[3] = {z, p.D[0][0] * MG[3] + p.D[1][0] * MG[6], p.D[0][1] * MG[3] + p.D[1][1] * MG[6]};  // by jb
+  const E Y[3] = {z, p.D[0][0] * MG[1] + p.D[0][1] * MG[2], p.D[1][0] * MG[1] + p.D[1][1] * MG[2]};  // by ja
+  for (int ja = 0; ja < 3; ja++) {
+    const E r = ja ? base - Y[ja] : base;
+    H0[3 * ja] = r;
+    for (int jb = 1; jb < 3; jb++) {
+      const E h = r - X[jb];
+      H0[3 * ja + jb] = ja ? h + p.D[ja - 1][jb - 1] * MG[0] : h;
+    }
+  }
+}
+
+// H1[3 ja + jb] for all nine (Qa, Qb)
+template <typename T, typename E> GB_HD void h1_all(const PairScalars<T>& p, const E* MP, E* H1) {
+  const E S0 = p.Tr[0][0] * MP[4] + p.Tr[0][1] * MP[5] + p.Tr[1][0] * MP[7] + p.Tr[1][1] * MP[8];
+  // alpha = -a_k: + U_j M_{1j} (k = 0) or - U_j M_{0j} (k = 1), - T_kj MP[1 + j]
+  const E X0 = p.U[0] * MP[7] + p.U[1] * MP[8] - p.Tr[0][0] * MP[1] - p.Tr[0][1] * MP[2];
+  const E X1 = E{} - p.U[0] * MP[4] - p.U[1] * MP[5] - p.Tr[1][0] * MP[1] - p.Tr[1][1] * MP[2];
+  // beta = -b_l: + V_i M_{i1} (l = 0) or - V_i M_{i0} (l = 1), - T_il MP[3 (i + 1)]
+  const E Y0 = p.V[0] * MP[5] + p.V[1] * MP[8] - p.Tr[0][0] * MP[3] - p.Tr[1][0] * MP[6];
+  const E Y1 = E{} - p.V[0] * MP[4] - p.V[1] * MP[7] - p.Tr[0][1] * MP[3] - p.Tr[1][1] * MP[6];
+  H1[0] = S0;
+  H1[1] = S0 + Y0;
+  H1[2] = S0 + Y1;
+  H1[3] = S0 + X0;
+  H1[6] = S0 + X1;
+  // both: - sgn_k U_l MP[u of the other a], - sgn_l V_k MP[v of the other b], + T_kl MP[0]
+  H1[4] = H1[3] + Y0 - p.U[0] * MP[6] - p.V[0] * MP[2] + p.Tr[0][0] * MP[0];
+  H1[5] = H1[3] + Y1 - p.U[1] * MP[6] + p.V[0] * MP[1] + p.Tr[0][1] * MP[0];
+  H1[7] = H1[6] + Y0 + p.U[0] * MP[3] - p.V[1] * MP[2] + p.Tr[1][0] * MP[0];
+  H1[8] = H1[6] + Y1 + p.U[1] * MP[3] + p.V[1] * MP[1] + p.Tr[1][1] * MP[0];
+}
+
 // H0 = sum c MG - (4/k^2) MG[0];  H1 = sum d MP.
 template <typename T>
 GB_HD void combine(const cx<T>* MG, const cx<T>* MP, const T* c, const T* d, cx<T> m4ok2, cx<T>* H0, cx<T>* H1) {

@@ -151,3 +151,37 @@ def test_f64_matrix_and_lu(golden):
     b = np.random.default_rng(5).standard_normal((A.shape[0], 2))
     x = R.LUSolve(b)
     assert np.abs(A @ x - b).max() / np.abs(b).max() < 1e-10
+
+
+@pytest.mark.parametrize("omega", [0.8, 0.9j, 0.7 + 0.2j])
+def test_two_surfaces_every_pair_form_matches_oracle(omega):
+    """FP64 far field over every form its rules take: a PEC and a dielectric
+    body (blocks with one, two and three channels, with and without a
+    mirror), panel counts off the 32 x 8 pair tiles (80 and 36), and a real, an
+    imaginary and a complex wavenumber, against the oracle."""
+    from gbem import RWGGeometry, mesh
+    from gbem.api import Material
+    from oracle import oracle
+    V1, P1 = mesh.icosphere(1)
+    V2, P2 = mesh.rounded_cube(48, seed=3)
+    V2 = V2 + [0.0, 0.4, 2.1]
+    m = Material(2.5) if omega == 0.9j else Material(2.25 + 0.01j)
+    G = RWGGeometry([{"V": V1, "P": P1, "material": None}, {"V": V2, "P": P2, "material": m}])
+    A = G.AssembleBEMMatrix(omega).numpy()
+    Ao = oracle.assemble([oracle.Surface(V1, P1), oracle.Surface(V2, P2)], [(0, -1), (0, 1)], [True, False], omega,
+                         [1.0, m.eps], [1.0, 1.0])
+    assert np.array_equal(A, A.T)
+    # entries whose four panel pairs are all far (rRel > 4): the same rule in
+    # the same arithmetic, 144 samples of a few units in the last place
+    T = np.concatenate([V1[P1], V2[P2]])
+    c = T.mean(axis=1)
+    rad = np.linalg.norm(T - c[:, None], axis=2).max(axis=1)
+    far = np.linalg.norm(c[:, None] - c[None], axis=2) > 4.0 * np.maximum(rad[:, None], rad[None])
+    bf = np.array([(off + e[4], off + e[5]) for i, off, n in ((0, 0, 1), (1, len(P1), 2)) for e in G.edges(i)[0]
+                   for _ in range(n)])
+    ok = np.ones(A.shape, dtype=bool)
+    for a in (0, 1):
+        for b in (0, 1):
+            ok &= far[bf[:, a]][:, bf[:, b]]
+    assert ok.mean() > 0.3
+    assert np.abs(A - Ao)[ok].max() <= 1e-13 * np.abs(Ao).max()
