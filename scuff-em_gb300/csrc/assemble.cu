@@ -814,8 +814,10 @@ struct PPairArgs {
   const float* geo;   // per global panel: 18 floats (float-float V0 - O, A, B)
   const double* pc;   // per global panel: centroid, radius
   const int* cpan;    // the stripe's column panels (surface-local)
+  const int* emin;    // per row panel: its first edge; per column panel: its last
+  const int* emax;
   int offa, offb;     // global index of the first panel of each surface
-  int nrow, ncp;
+  int nrow, ncp, sym;
   float* out;         // [NF][9][ncp][nrow]
 };
 
@@ -874,6 +876,9 @@ __global__ void __launch_bounds__(PP_THREADS, 1) ppair_kernel(PPairArgs p, Regio
 
   const int pa = r0 + threadIdx.x, cl = c0 + threadIdx.y;
   if (pa >= p.nrow || cl >= p.ncp) return;
+  // entries on and above the diagonal only: no edge of pa precedes one of the
+  // column panel (44 % of the pairs of a one-stripe icosphere)
+  if (p.sym && p.emin[pa] > p.emax[p.cpan[cl]]) return;
   const int ia = threadIdx.x, ib = 32 + threadIdx.y;
   const size_t cs = (size_t)p.ncp * p.nrow;  // stride of one (field, combination) plane
   float* out = p.out + (size_t)cl * p.nrow + pa;
@@ -1374,9 +1379,9 @@ static cudaError_t far_mixed(Geometry* g, const Block& b, DevBlock* db, const Ti
   for (const DevBlock::DevStripe& st : db->stripes) {
     if (st.ntiles == 0 || st.ncp == 0) continue;
     PPairArgs pp;
-    pp.node = g->d_ffnode; pp.geo = g->d_ffgeo; pp.pc = g->d_pc; pp.cpan = st.cpan;
+    pp.node = g->d_ffnode; pp.geo = g->d_ffgeo; pp.pc = g->d_pc; pp.cpan = st.cpan; pp.emin = db->emin; pp.emax = db->emax;
     pp.offa = g->S[b.sa].panel_offset; pp.offb = g->S[b.sb].panel_offset;
-    pp.nrow = st.nrow; pp.ncp = st.ncp; pp.out = (float*)g->ppv;
+    pp.nrow = st.nrow; pp.ncp = st.ncp; pp.sym = b.sym; pp.out = (float*)g->ppv;
     ppair_kernel<NC><<<dim3((st.nrow + 31) / 32, (st.ncp + PP_COLS - 1) / PP_COLS), dim3(32, PP_COLS), 0, s>>>(pp, ra);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     StampArgs sp;
