@@ -1241,8 +1241,13 @@ struct Stamp64Args {
   int nrow, ncp;
 };
 
-// pass 2, as stamp_kernel: La Lb ((PP - PM) - (MP - MM)), a missing panel's value zero
-template <int NC>
+template <typename TO> __device__ __forceinline__ TO kept(cx<double> v);
+template <> __device__ __forceinline__ cx<double> kept<cx<double>>(cx<double> v) { return v; }
+template <> __device__ __forceinline__ double kept<double>(cx<double> v) { return v.re; }
+
+// pass 2, as stamp_kernel: La Lb ((PP - PM) - (MP - MM)), a missing panel's
+// value zero; TO = double keeps the real part
+template <int NC, typename TO>
 __global__ void __launch_bounds__(256) stamp64_kernel(Stamp64Args sp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<double>* s_val = reinterpret_cast<cx<double>*>(smem_raw);  // [TE][TE][NC]
@@ -1293,14 +1298,15 @@ __global__ void __launch_bounds__(256) stamp64_kernel(Stamp64Args sp) {
     for (int c = 0; c < NC; c++) s_val[(size_t)(i * TE + j) * NC + c] = L * (row[0][c] - row[1][c]);
   }
   __syncthreads();
-  cx<double>* out = reinterpret_cast<cx<double>*>(a.out);
+  TO* out = reinterpret_cast<TO*>(a.out);
   for (int pass = 0; pass < 2; pass++) {
     if (!(a.passes & (1 << pass))) continue;
     for (int q = threadIdx.x; q < NR * NCc; q += blockDim.x) {
       int i, j;
       if (!tile_entry(pass, q, NR, NCc, diag, &i, &j)) continue;
       const cx<double>* v = s_val + (size_t)(i * TE + j) * NC;
-      store_entry(a, out, pass, RB->e0 + i, CB->e0 + j, v[0], NC > 1 ? v[1] : v[0], NC > 2 ? v[2] : v[0]);
+      store_entry(a, out, pass, RB->e0 + i, CB->e0 + j, kept<TO>(v[0]), kept<TO>(NC > 1 ? v[1] : v[0]),
+                  kept<TO>(NC > 2 ? v[2] : v[0]));
     }
   }
 }
@@ -1346,7 +1352,7 @@ static cudaError_t far_fp64(Geometry* g, const Block& b, DevBlock* db, const Til
     stats_launch(ST_FAR);
     return launch_tiles64<NC>(ta, ra, db->ntiles, s);
   }
-  if (e == cudaSuccess) e = allow_max_smem(stamp64_kernel<NC>);
+  if (e == cudaSuccess) e = allow_max_smem(stamp64_kernel<NC, cx<double>>);
   if (e != cudaSuccess) return e;
   bool realk = true;
   for (int r = 0; r < ra.nreg; r++) realk = realk && ra.k[r].re == 0.0;
@@ -1363,7 +1369,7 @@ static cudaError_t far_fp64(Geometry* g, const Block& b, DevBlock* db, const Til
     Stamp64Args sp;
     sp.ta = ta; sp.tiles = st.tiles; sp.edge_a = db->edge_a; sp.edge_b = db->edge_b; sp.ecol = db->ecol;
     sp.offb = pp.offb; sp.ppv = pp.out; sp.nrow = st.nrow; sp.ncp = st.ncp;
-    stamp64_kernel<NC><<<st.ntiles, 256, TE * TE * NC * sizeof(cx<double>), s>>>(sp);
+    stamp64_kernel<NC, cx<double>><<<st.ntiles, 256, TE * TE * NC * sizeof(cx<double>), s>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     stats_launch(ST_FAR, 2);
   }
@@ -1783,6 +1789,219 @@ __global__ void __launch_bounds__(128) grad_kernel(GradArgs a, RegionArgs ra) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// Gradient of a block without near pairs: as the far field, every panel pair
+// once (grad_pair_kernel) and its nine (Qa, Qb) combinations into the entries
+// (stamp64_kernel), per component mu.  With F = x - Qa, F' = x' - Qb,
+//   G0 = int int R_mu (F.F' - 4/k^2) Psi          is H0 with R_mu Psi for G,
+//   G1 = int int R_mu ((F x F').R) Zeta           is H1 with R_mu Zeta for Psi,
+//      + int int (F x F')_mu Psi                  H0 with (a_i x b_j)_mu for a_i.b_j,
+// so the moments are those of three kernels.  grad_kernel integrates each of
+// an edge pair's four panel pairs afresh, all components, in complex
+// arithmetic: two PEC spheres, N = 3840 real, dM/dz: 134 ms there, 4.9 here.
+// ---------------------------------------------------------------------------
+template <int KIND, bool H1, typename E>
+__device__ __forceinline__ void grad_moments64(const double* D0, const double* A, const double* B, const double* ob,
+                                               double kre, double kim, const double* w4, const SinCosTab64& tab, int mu,
+                                               E* M0, E* M1, E* M2) {
+  const int NF = H1 ? 9 : 0;
+#pragma unroll
+  for (int m = 0; m < 9; m++) {
+    M0[m] = E{};
+    if (m < NF) M1[m] = M2[m] = E{};
+  }
+#pragma unroll 1
+  for (int i = 0; i < 6; i++) {
+    const double u = c_lo64[3 * i], v = c_lo64[3 * i + 1], wi = c_lo64[3 * i + 2];
+    double pa[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) pa[c] = fma(v, B[c], fma(u, A[c], D0[c]));
+    E S0[3], S1[3], S2[3];
+#pragma unroll
+    for (int b = 0; b < 3; b++) S0[b] = S1[b] = S2[b] = E{};
+#pragma unroll 2
+    for (int j = 0; j < 6; j++) {
+      const double x = pa[0] - ob[3 * j], y = pa[1] - ob[3 * j + 1], z = pa[2] - ob[3 * j + 2];
+      const double Rm = mu == 0 ? x : (mu == 1 ? y : z);
+      const double r2 = fma(z, z, fma(y, y, x * x));
+      const double rinv = rsqrt(r2), r = r2 * rinv;
+      const double up = c_lo64[3 * j], vp = c_lo64[3 * j + 1];
+      double amp = w4[j] * rinv;
+      if (KIND != 0) amp *= exp(-kim * r);
+      E psi, f1{};
+      // Psi = Phi (ik - 1/r)/r, Zeta = Phi ((ik)^2 - 3 ik/r + 3/r^2)/r^2
+      if constexpr (KIND == 2) {
+        psi = amp * ((-kim - rinv) * rinv);
+        if (H1) f1 = Rm * (amp * (fma(3.0 * rinv, kim + rinv, kim * kim) * (rinv * rinv)));
+      } else {
+        double c, s;
+        expi64(kre * r, tab, &c, &s);
+        const cx<double> phi = mk(amp * c, amp * s);
+        psi = phi * mk((-kim - rinv) * rinv, kre * rinv);
+        if (H1) {
+          const double ri2 = rinv * rinv;
+          f1 = Rm * (phi * mk(fma(3.0 * rinv, kim + rinv, kim * kim - kre * kre) * ri2,
+                              (-2.0 * kre * kim - 3.0 * kre * rinv) * ri2));
+        }
+      }
+      const E f0 = Rm * psi;
+      S0[0] = S0[0] + f0; S0[1] = S0[1] + up * f0; S0[2] = S0[2] + vp * f0;
+      if (H1) {
+        S1[0] = S1[0] + f1; S1[1] = S1[1] + up * f1; S1[2] = S1[2] + vp * f1;
+        S2[0] = S2[0] + psi; S2[1] = S2[1] + up * psi; S2[2] = S2[2] + vp * psi;
+      }
+    }
+    const double a[3] = {wi, wi * u, wi * v};
+#pragma unroll
+    for (int al = 0; al < 3; al++)
+#pragma unroll
+      for (int b = 0; b < 3; b++) {
+        const int m = 3 * al + b;
+        M0[m] = M0[m] + a[al] * S0[b];
+        if (H1) {
+          M1[m] = M1[m] + a[al] * S1[b];
+          M2[m] = M2[m] + a[al] * S2[b];
+        }
+      }
+  }
+}
+
+template <int NC, bool REALK>
+__global__ void __launch_bounds__(PP64_THREADS, 1) grad_pair_kernel(PPair64Args p, RegionArgs ra, int mu, double sign) {
+  using E = typename std::conditional<REALK, double, cx<double>>::type;
+  __shared__ double s_pv[PP64_SLOTS][9];
+  __shared__ double s_ob[PP64_COLS][18];
+  __shared__ SinCosTab64 s_tab;
+  __shared__ double s_w4[6];
+  const int tid = threadIdx.y * 32 + threadIdx.x;
+  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * PP64_COLS;
+  for (int q = tid; q < PP64_SLOTS * 9; q += PP64_THREADS) {
+    const int sl = q / 9, f = q - sl * 9;
+    const int gp = sl < 32 ? (r0 + sl < p.nrow ? p.offa + r0 + sl : -1)
+                           : (c0 + sl - 32 < p.ncp ? p.offb + p.cpan[c0 + sl - 32] : -1);
+    s_pv[sl][f] = gp >= 0 ? p.pv[9 * (size_t)gp + f] : 0.0;
+  }
+  if (!REALK)
+    for (int q = tid; q < (int)(sizeof(SinCosTab64) / 8); q += PP64_THREADS)
+      reinterpret_cast<double*>(&s_tab)[q] = reinterpret_cast<const double*>(&c_sctab64)[q];
+  if (tid < 6) s_w4[tid] = c_lo64[3 * tid + 2] * 0.079577471545947667884;  // 1/(4 pi)
+  __syncthreads();
+  for (int q = tid; q < PP64_COLS * 18; q += PP64_THREADS) {
+    const int cl = q / 18, j = (q - cl * 18) / 3, c = q % 3;
+    const double* V = s_pv[32 + cl];
+    s_ob[cl][3 * j + c] = fma(c_lo64[3 * j + 1], V[6 + c] - V[c], c_lo64[3 * j] * (V[3 + c] - V[c]));
+  }
+  __syncthreads();
+  const int pa = r0 + threadIdx.x, cl = c0 + threadIdx.y;
+  if (pa >= p.nrow || cl >= p.ncp) return;
+  const int ia = threadIdx.x, ib = 32 + threadIdx.y;
+  const size_t cs = (size_t)p.ncp * p.nrow, fs = 9 * cs;
+  double2* out = p.out + (size_t)cl * p.nrow + pa;
+  PairGeom<double> g;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    g.D0[c] = s_pv[ia][c] - s_pv[ib][c];
+    g.Aa[c] = s_pv[ia][3 + c] - s_pv[ia][c]; g.Ba[c] = s_pv[ia][6 + c] - s_pv[ia][c];
+  }
+  bool first = true;
+#pragma unroll 1
+  for (int r = 0; r < ra.nreg; r++) {
+    const cx<double> k = ra.k[r];
+    if (k.re == 0.0 && k.im == 0.0) continue;
+    E M0[9], M1[9], M2[9];
+    const double* ob = s_ob[threadIdx.y];
+    if constexpr (REALK) {
+      grad_moments64<2, (NC > 1)>(g.D0, g.Aa, g.Ba, ob, 0.0, k.im, s_w4, s_tab, mu, M0, M1, M2);
+    } else {
+      if (k.im == 0.0) grad_moments64<0, (NC > 1)>(g.D0, g.Aa, g.Ba, ob, k.re, 0.0, s_w4, s_tab, mu, M0, M1, M2);
+      else grad_moments64<1, (NC > 1)>(g.D0, g.Aa, g.Ba, ob, k.re, k.im, s_w4, s_tab, mu, M0, M1, M2);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      g.Ab[c] = s_pv[ib][3 + c] - s_pv[ib][c]; g.Bb[c] = s_pv[ib][6 + c] - s_pv[ib][c];
+    }
+    PairScalars<double> ps;
+    pair_scalars(g, &ps);
+    const cx<double> m4 = cdiv(mk(-4.0, 0.0), k * k);
+    E H[9], m4e;
+    if constexpr (REALK) m4e = m4.re; else m4e = m4;
+    h0_all(ps, M0, m4e, H);
+    auto put = [&](int f, int c, cx<double> v) {
+      double2* o = out + f * fs + c * cs;
+      if (!first) { const double2 z = *o; v = v + mk(z.x, z.y); }
+      *o = make_double2(v.re, v.im);
+    };
+#pragma unroll
+    for (int c = 0; c < 9; c++) {
+      put(0, c, scaled(sign * ra.pf1[r], H[c]));
+      if (NC > 2) put(2, c, scaled(sign * ra.pf3[r], H[c]));
+    }
+    if (NC > 1) {
+      E Hx[9];
+      h1_all(ps, M1, H);
+      // (F x F')_mu: the dot products of h0_all replaced by cross-product components
+      const int n1 = (mu + 1) % 3, n2 = (mu + 2) % 3;
+      const double* a[2] = {g.Aa, g.Ba};
+      const double* b[2] = {g.Ab, g.Bb};
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) ps.D[i][j] = a[i][n1] * b[j][n2] - a[i][n2] * b[j][n1];
+      h0_all(ps, M2, E{}, Hx);
+#pragma unroll
+      for (int c = 0; c < 9; c++) put(1, c, scaled(sign * ra.pfc[r], H[c] + Hx[c]));
+    }
+    first = false;
+  }
+  if (first)  // every common region has k = 0: zero contribution
+    for (int c = 0; c < 9 * NC; c++) out[c * cs] = make_double2(0.0, 0.0);
+}
+
+// dM/dx_mu of the (nsa, nsb) block, without near pairs, nsa != nsb; the block
+// is stored with rows of the lower surface, and a displacement of the higher
+// one is minus that of the lower
+template <int NC>
+static cudaError_t grad_far(Geometry* g, const Block& b, DevBlock* db, const RegionArgs& ra, const BlockSel& sel, int mu,
+                            void* dst, int ld, bool real, cudaStream_t s) {
+  cudaError_t e = pair_scratch(g, b.max_stripe_pairs * 9 * NC * sizeof(double2));
+  if (e == cudaSuccess) e = allow_max_smem(stamp64_kernel<NC, cx<double>>);
+  if (e == cudaSuccess) e = allow_max_smem(stamp64_kernel<NC, double>);
+  if (e != cudaSuccess) return e;
+  bool realk = true;
+  for (int r = 0; r < ra.nreg; r++) realk = realk && ra.k[r].re == 0.0;
+  const bool same = sel.nsa == b.sa;
+  TileArgs ta = {};
+  ta.rows = db->rows; ta.cols = db->cols;
+  ta.pv = g->d_pv; ta.pc = g->d_pc; ta.elen_a = db->elen_a; ta.elen_b = db->elen_b;
+  ta.nptr = db->nptr; ta.ncol = db->ncol; ta.nidx = db->nidx; ta.nearval = db->nearval;
+  ta.row_panel_offset = g->S[b.sa].panel_offset;
+  ta.bpe_a = b.bpe_a; ta.bpe_b = b.bpe_b;
+  ta.row_off = ta.mrow_off = sel.row0; ta.col_off = ta.mcol_off = sel.col0;
+  ta.passes = same ? 1 : 2;
+  ta.sym = 0;
+  ta.out = dst; ta.ld = ld;
+  for (const DevBlock::DevStripe& st : db->stripes) {
+    if (st.ntiles == 0 || st.ncp == 0) continue;
+    PPair64Args pp = {};
+    pp.pv = g->d_pv; pp.pc = g->d_pc; pp.cpan = st.cpan;
+    pp.offa = g->S[b.sa].panel_offset; pp.offb = g->S[b.sb].panel_offset;
+    pp.nrow = st.nrow; pp.ncp = st.ncp; pp.out = (double2*)g->ppv;
+    const dim3 grid((st.nrow + 31) / 32, (st.ncp + PP64_COLS - 1) / PP64_COLS), block(32, PP64_COLS);
+    if (realk) grad_pair_kernel<NC, true><<<grid, block, 0, s>>>(pp, ra, mu, same ? 1.0 : -1.0);
+    else grad_pair_kernel<NC, false><<<grid, block, 0, s>>>(pp, ra, mu, same ? 1.0 : -1.0);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    Stamp64Args sp;
+    sp.ta = ta; sp.tiles = st.tiles; sp.edge_a = db->edge_a; sp.edge_b = db->edge_b; sp.ecol = db->ecol;
+    sp.offb = pp.offb; sp.ppv = pp.out; sp.nrow = st.nrow; sp.ncp = st.ncp;
+    const size_t smem = TE * TE * NC * sizeof(cx<double>);
+    if (real) stamp64_kernel<NC, double><<<st.ntiles, 256, smem, s>>>(sp);
+    else stamp64_kernel<NC, cx<double>><<<st.ntiles, 256, smem, s>>>(sp);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    stats_launch(ST_OTHER, 2);
+  }
+  return cudaSuccess;
+}
+
 gbem_status assemble_gradient_device(Geometry* g, double wr, double wi, const double* eps, const double* mu,
                                      const BlockSel& sel, void* const out[3], int ld, int dtype, cudaStream_t s,
                                      int nta, const double* gamma, void* const* outT) {
@@ -1807,6 +2026,24 @@ gbem_status assemble_gradient_device(Geometry* g, double wr, double wi, const do
   }
   if (e != cudaSuccess) return cuda_status(e, "gradient memset");
   if (bp->nreg == 0 || A.ne == 0 || B.ne == 0) return GBEM_OK;
+  if (nta == 0 && !bp->sym && bp->near.empty()) {
+    // every panel pair is far: the two-pass form (grad_kernel where its pair
+    // values find no room)
+    const RegionArgs ra = region_args(*bp, wr, wi, eps, mu);
+    DevBlock* db = g->dblocks[bp - g->blocks.data()];
+    const int nc = (bp->bpe_a == 2 && bp->bpe_b == 2) ? 3 : ((bp->bpe_a == 1 && bp->bpe_b == 1) ? 1 : 2);
+    for (int m = 0; m < 3 && e == cudaSuccess; m++) {
+      if (!out[m]) continue;
+      const bool real = dtype == GBEM_F64;
+      e = nc == 1 ? grad_far<1>(g, *bp, db, ra, sel, m, out[m], ld, real, s)
+                  : nc == 2 ? grad_far<2>(g, *bp, db, ra, sel, m, out[m], ld, real, s)
+                            : grad_far<3>(g, *bp, db, ra, sel, m, out[m], ld, real, s);
+    }
+    if (e == cudaSuccess) return cuda_status(cudaStreamSynchronize(s), "gradient block");
+    if (e != cudaErrorMemoryAllocation) return cuda_status(e, "gradient block");
+    cudaGetLastError();
+    e = cudaSuccess;
+  }
   double *dVa = nullptr, *dVb = nullptr, *dLa = nullptr, *dLb = nullptr;
   int *dEa = nullptr, *dEb = nullptr;
   e = dupload(&dVa, A.V.data(), A.V.size());

@@ -146,3 +146,41 @@ def test_torque_matches_finite_differences(golden):
     fd = (Ms[0] - Ms[1]) / (2 * h)
     tz = RWGGeometry(gs).AssembleBEMMatrixBlockTorque(0, 1, w, [(0.0, 0.0, 1.0)])[0]
     assert np.abs(tz - fd).max() / np.abs(tz).max() < 1e-5
+
+
+@pytest.mark.parametrize("omega", [1.1, 0.6j, 0.8 + 0.3j])
+@pytest.mark.parametrize("pec", [(True, True), (False, False), (True, False)])
+def test_gradient_of_distant_bodies_in_every_form(omega, pec):
+    """Blocks without near pairs (every pair once, combinations from moments):
+    both orientations, one to three channels, each component, a real, an
+    imaginary and a complex wavenumber, panel counts off the 32 x 8 tiles.
+    Block and gradient use the same 6x6 rule here, so the gradient equals
+    central differences of the block: truncation h^2 |d3| / 6 of a kernel that
+    varies over distances above 3, 2e-9 at h = 1e-4, and rounding 1e-16 / h."""
+    from gbem import RWGGeometry, mesh
+    from gbem.api import Material
+    V0, P0 = mesh.icosphere(1)
+    V1, P1 = mesh.rounded_cube(108, seed=2)
+    V1 = V1 + [0.3, -0.5, 6.0]
+    m = Material(2.5) if omega == 0.6j else Material(2.25 + 0.02j)
+
+    def geo(d0, d1):
+        return RWGGeometry([{"V": V0 + d0, "P": P0, "material": None if pec[0] else m},
+                            {"V": V1 + d1, "P": P1, "material": None if pec[1] else m}])
+
+    G = geo(np.zeros(3), np.zeros(3))
+    h = 1e-4
+    for (a, b) in ((0, 1), (1, 0)):
+        grads = G.AssembleBEMMatrixBlockGradient(a, b, omega)
+        scale = max(np.abs(g).max() for g in grads)
+        for mu in range(3):
+            d = np.zeros(3)
+            d[mu] = h
+            z = np.zeros(3)
+            Mp = (geo(d, z) if a == 0 else geo(z, d)).AssembleBEMMatrixBlock(a, b, omega)
+            Mm = (geo(-d, z) if a == 0 else geo(z, -d)).AssembleBEMMatrixBlock(a, b, omega)
+            assert np.abs(grads[mu] - (Mp - Mm) / (2 * h)).max() <= 1e-7 * scale
+        if omega == 0.6j:
+            real = G.AssembleBEMMatrixBlockGradient(a, b, omega, real=True)
+            for mu in range(3):
+                assert np.array_equal(real[mu], grads[mu].real)
