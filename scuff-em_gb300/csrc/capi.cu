@@ -205,14 +205,18 @@ static __global__ void emt_grad(const cx<double>* M, long long ld, int N, const 
 }
 
 namespace gbem {
-template <typename T>
-static __global__ void trace_diag(const cx<T>* X, long long ldx, int n, double* out) {
+template <typename T> __device__ __forceinline__ double re_of(cx<T> z) { return (double)z.re; }
+template <typename T> __device__ __forceinline__ double im_of(cx<T> z) { return (double)z.im; }
+__device__ __forceinline__ double re_of(double x) { return x; }
+__device__ __forceinline__ double im_of(double) { return 0.0; }
+template <typename E>
+static __global__ void trace_diag(const E* X, long long ldx, int n, double* out) {
   __shared__ double sr[1024], si[1024];
   double ar = 0.0, ai = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const cx<T> v = X[i + (long long)i * ldx];
-    ar += (double)v.re;
-    ai += (double)v.im;
+    const E v = X[i + (long long)i * ldx];
+    ar += re_of(v);
+    ai += im_of(v);
   }
   sr[threadIdx.x] = ar;
   si[threadIdx.x] = ai;
@@ -814,19 +818,23 @@ gbem_status gbem_lu_factor(gbem_matrix* M, int* ipiv, int* info) {
   int h_info = 0;
   gbem_status st;
   if (M->dtype == GBEM_F64) {
-    // real matrix (dgetrf semantics): factored as complex128 with zero
-    // imaginary parts, which stay exactly zero; |Re|+|Im| is then IDAMAX's |x|
+    // real matrix (dgetrf semantics): in real arithmetic, or, beyond the rows
+    // that takes, as complex128 with zero imaginary parts, which stay exactly
+    // zero; |Re|+|Im| is then IDAMAX's |x|
     const int N = M->N;
-    void* tmp = nullptr;
-    CHECK_CUDA(cudaMallocAsync(&tmp, (size_t)N * N * 16, M->stream), "F64 LU scratch");
-    const unsigned nb = (unsigned)(((long long)N * N + 255) / 256);
-    make_complex<<<nb, 256, 0, M->stream>>>((const double*)M->d, M->ld, (double2*)tmp, N, N, N);
-    st = lu_factor_device(tmp, N, N, GBEM_C128, M->d_ipiv, &h_info, M->stream, &M->ws, &M->ws_bytes);
-    if (st == GBEM_OK) take_real<<<nb, 256, 0, M->stream>>>((const double2*)tmp, N, (double*)M->d, M->ld, N, N);
-    stats_launch(ST_OTHER, 2);
-    cudaFreeAsync(tmp, M->stream);
-    cudaError_t e = cudaStreamSynchronize(M->stream);
-    if (st == GBEM_OK && e != cudaSuccess) st = cuda_status(e, "F64 LU");
+    st = lu_factor_device(M->d, N, M->ld, GBEM_F64, M->d_ipiv, &h_info, M->stream, &M->ws, &M->ws_bytes);
+    if (st == GBEM_ENOTSUP) {
+      void* tmp = nullptr;
+      CHECK_CUDA(cudaMallocAsync(&tmp, (size_t)N * N * 16, M->stream), "F64 LU scratch");
+      const unsigned nb = (unsigned)(((long long)N * N + 255) / 256);
+      make_complex<<<nb, 256, 0, M->stream>>>((const double*)M->d, M->ld, (double2*)tmp, N, N, N);
+      st = lu_factor_device(tmp, N, N, GBEM_C128, M->d_ipiv, &h_info, M->stream, &M->ws, &M->ws_bytes);
+      if (st == GBEM_OK) take_real<<<nb, 256, 0, M->stream>>>((const double2*)tmp, N, (double*)M->d, M->ld, N, N);
+      stats_launch(ST_OTHER, 2);
+      cudaFreeAsync(tmp, M->stream);
+      cudaError_t e = cudaStreamSynchronize(M->stream);
+      if (st == GBEM_OK && e != cudaSuccess) st = cuda_status(e, "F64 LU");
+    }
   } else {
     st = lu_factor_device(M->d, M->N, M->ld, M->dtype, M->d_ipiv, &h_info, M->stream, &M->ws, &M->ws_bytes);
   }
@@ -908,54 +916,29 @@ static gbem_status trace_impl(gbem_matrix* M, const void* B, int ldb, int ncols,
   CHECK_CUDA(cudaSetDevice(M->g->device), "cudaSetDevice");
   const int N = M->N;
   cudaStream_t s = M->stream;
-  const bool real = M->dtype == GBEM_F64;
-  const int dt = real ? GBEM_C128 : M->dtype;           // element type of the solve
-  const size_t es = dt == GBEM_C64 ? 8 : 16, ein = real ? 8 : es;
-  void *A = M->d, *tA = nullptr, *X = nullptr, *tB = nullptr;
+  const int dt = M->dtype;
+  const size_t es = esize(dt);
+  void* X = nullptr;
   double* d_out = nullptr;
-  int lda = M->ld;
   gbem_status st = GBEM_OK;
   cudaError_t e = cudaMallocAsync(&X, (size_t)N * ncols * es, s);
   if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_out, 2 * sizeof(double), s);
-  if (e == cudaSuccess && real) e = cudaMallocAsync(&tA, (size_t)N * N * 16, s);
-  if (e == cudaSuccess && real && host) e = cudaMallocAsync(&tB, (size_t)N * ncols * 8, s);
-  if (e == cudaSuccess) {
-    const void* src = B;
-    long long lds = ldb;
-    if (host) {
-      // the host B goes through a device buffer: the real one, or X itself
-      void* dst = real ? tB : X;
-      e = cudaMemcpy2DAsync(dst, (size_t)N * ein, B, (size_t)ldb * ein, (size_t)N * ein, ncols, cudaMemcpyHostToDevice, s);
-      src = dst;
-      lds = N;
-    } else if (!real) {
-      e = cudaMemcpy2DAsync(X, (size_t)N * es, B, (size_t)ldb * es, (size_t)N * es, ncols, cudaMemcpyDeviceToDevice, s);
-    }
-    if (e == cudaSuccess && real) {
-      // real factors and B: solved as complex128 with zero imaginary parts
-      make_complex<<<(unsigned)(((long long)N * N + 255) / 256), 256, 0, s>>>((const double*)M->d, M->ld, (double2*)tA,
-                                                                              N, N, N);
-      make_complex<<<(unsigned)(((long long)N * ncols + 255) / 256), 256, 0, s>>>((const double*)src, lds, (double2*)X,
-                                                                                  N, N, ncols);
-      stats_launch(ST_OTHER, 2);
-      A = tA;
-      lda = N;
-      e = cudaGetLastError();
-    }
-  }
+  if (e == cudaSuccess)
+    e = cudaMemcpy2DAsync(X, (size_t)N * es, B, (size_t)ldb * es, (size_t)N * es, ncols,
+                          host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s);
   if (e != cudaSuccess) st = cuda_status(e, "gbem_lu_trace setup");
-  if (st == GBEM_OK) st = lu_solve_many_device(A, N, lda, dt, M->d_perm, ncols, X, N, s);
+  if (st == GBEM_OK) st = lu_solve_many_device(M->d, N, M->ld, dt, M->d_perm, ncols, X, N, s);
   if (st == GBEM_OK) {
-    if (dt == GBEM_C64) trace_diag<float><<<1, 1024, 0, s>>>((const cx<float>*)X, N, ncols, d_out);
-    else trace_diag<double><<<1, 1024, 0, s>>>((const cx<double>*)X, N, ncols, d_out);
+    if (dt == GBEM_C64) trace_diag<<<1, 1024, 0, s>>>((const cx<float>*)X, N, ncols, d_out);
+    else if (dt == GBEM_F64) trace_diag<<<1, 1024, 0, s>>>((const double*)X, N, ncols, d_out);
+    else trace_diag<<<1, 1024, 0, s>>>((const cx<double>*)X, N, ncols, d_out);
     stats_launch(ST_OTHER);
     e = cudaMemcpyAsync(trace, d_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) st = cuda_status(e, "gbem_lu_trace");
   }
-  cudaFreeAsync(X, s); cudaFreeAsync(d_out, s);
-  if (tA) cudaFreeAsync(tA, s);
-  if (tB) cudaFreeAsync(tB, s);
+  if (X) cudaFreeAsync(X, s);
+  if (d_out) cudaFreeAsync(d_out, s);
   cudaStreamSynchronize(s);
   return st;
 }

@@ -79,3 +79,60 @@ def test_factor_keeps_non_finite_visible():
     assert np.array_equal(LU[:, :256], ref[:, :256])
     assert np.abs(LU[:, :N - 1] - ref[:, :N - 1]).max() <= 1e-12 * np.abs(ref).max()
     assert not np.isfinite(LU[:, N - 1]).any()
+
+
+def _strip(n):
+    """An open PEC strip of n + 1 triangles: n interior edges, N = n."""
+    from gbem import RWGGeometry
+    V = np.array([[0.5 * i, i % 2, 0.01 * i * i / (n + 1)] for i in range(n + 3)], dtype=np.float64)
+    P = np.array([[i, i + 1, i + 2] if i % 2 == 0 else [i + 1, i, i + 2] for i in range(n + 1)], dtype=np.int32)
+    return RWGGeometry([{"V": V, "P": P, "material": None}])
+
+
+@pytest.mark.parametrize("N", [1, 2, 15, 16, 17, 31, 33, 65, 255, 257, 320, 513, 777])
+def test_real_factor_solve_and_trace_edges(N):
+    """F64 matrices in real arithmetic: dgetrf's pivots and factors, and
+    Tr[M^-1 B] over the first columns, at leaf, panel and tile edges."""
+    import scipy.linalg as sl
+    from gbem._lib import F64
+    from gbem.api import HMatrix
+    G = _strip(N)
+    M = HMatrix(G, F64)
+    rng = np.random.default_rng(N)
+    A = rng.standard_normal((N, N))
+    M.set(A)
+    assert M.LUFactorize() == 0
+    lu_ref, piv_ref = sl.lu_factor(A)
+    assert np.array_equal(M.ipiv - 1, piv_ref)
+    LU = M.numpy()
+    assert np.abs(LU - lu_ref).max() <= 1e-11 * np.abs(lu_ref).max()
+    _check_backward(A, LU, M.ipiv - 1)
+    nc = max(1, (2 * N) // 3)
+    B = rng.standard_normal((N, nc))
+    t = M.TraceMInvdM(B)
+    X = sl.lu_solve((lu_ref, piv_ref), B)
+    # forward error of one solution: cond(A) N u, times the root of nc terms
+    tol = np.linalg.cond(A) * N * U * np.linalg.norm(X)
+    assert t.imag == 0.0 and abs(t.real - np.trace(X[:nc])) <= tol
+
+
+@pytest.mark.parametrize("pec", [True, False])
+def test_complex_trace_matches_lapack(pec):
+    """Tr[M^-1 B] of a complex128 matrix: halves of 32-row blocks with
+    remainders (N = 400 and 800, a panel and three quarters)."""
+    import scipy.linalg as sl
+    from gbem import RWGGeometry, mesh
+    from gbem._lib import C128
+    from gbem.api import HMatrix, Material
+    V, P = mesh.rounded_cube(270, seed=1)
+    G = RWGGeometry([{"V": V, "P": P, "material": None if pec else Material(2.0)}])
+    M = HMatrix(G, C128)
+    N = M.N
+    rng = np.random.default_rng(N)
+    A = rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))
+    M.set(A)
+    assert M.LUFactorize() == 0
+    B = rng.standard_normal((N, 100)) + 1j * rng.standard_normal((N, 100))
+    X = sl.solve(A, B)
+    tol = np.linalg.cond(A) * N * U * np.linalg.norm(X)
+    assert abs(M.TraceMInvdM(B) - np.trace(X[:100])) <= tol
