@@ -82,7 +82,8 @@ constexpr int HO_N = 11;                 // collapsed Gauss rule, degree 20
 __constant__ double c_ho[3 * HO_N * HO_N];
 constexpr int NT_SELF = 16;              // 1-D rule of the common-triangle reduction
 constexpr int N_FIP = 12;                // rules of the static near-pair integrals
-__constant__ double c_gx16[NT_SELF], c_gw16[NT_SELF], c_gx12[N_FIP], c_gw12[N_FIP];
+__device__ double g_self_tab[SELF_ROWS * 6 * NT_SELF];  // common-triangle table (self_table)
+__constant__ double c_gx12[N_FIP], c_gw12[N_FIP];
 // static integrals inside the adjoint's central differences: 8 points per
 // dimension move their derivatives by < 1e-8 (relative) against 12, at a
 // third of the cost (touching pairs are the worst case)
@@ -135,8 +136,9 @@ static gbem_status init_rules() {
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_ffrule, &ffr, sizeof ffr);
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_sctab, &sct, sizeof sct);
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_ho, ho, sizeof ho);
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_gx16, gx16, sizeof gx16);
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_gw16, gw16, sizeof gw16);
+  std::vector<double> stab(SELF_ROWS * 6 * NT_SELF);
+  self_table(gx16, gw16, NT_SELF, stab.data());
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_self_tab, stab.data(), sizeof(double) * stab.size());
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_gx12, gx12, sizeof gx12);
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_gw12, gw12, sizeof gw12);
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_gx8, gx8, sizeof gx8);
@@ -390,12 +392,12 @@ __device__ void fippi_warp(const DevNear& d, const double* Va, const double* Vb,
                            int n, int lane, Fippi& F) {
   fippi_zero(&F);
   if (d.ncv == 0) {
-    double A[3], B[3], Ap[3], Bp[3], dV[3], a2;
-    fippi_far_setup(Va, Vb, A, B, Ap, Bp, dV, &a2);
+    double A[3], B[3], Ap[3], Bp[3], dV[3], a2, ia;
+    fippi_far_setup(Va, Vb, A, B, Ap, Bp, dV, &a2, &ia);
     for (int q = lane; q < n * n * n; q += 32) {
       const int i1 = q / (n * n), j = (q / n) % n, l = q % n;
       const double u = sgx[i1];
-      fippi_far_acc(A, B, Ap, Bp, dV, a2, u, u * sgx[j], sgx[l], sgw[i1] * sgw[j] * sgw[l] * u, F);
+      fippi_far_acc(A, B, Ap, Bp, dV, a2, ia, u, u * sgx[j], sgx[l], sgw[i1] * sgw[j] * sgw[l] * u, F);
     }
   } else {
     double Ea[9], Eb[9];
@@ -426,12 +428,12 @@ __global__ void __launch_bounds__(FIPPI_THREADS) fippi_kernel(const DevNear* nea
   Fippi F;
   fippi_zero(&F);
   if (d.ncv == 0) {
-    double A[3], B[3], Ap[3], Bp[3], dV[3], a2;
-    fippi_far_setup(Va, Vb, A, B, Ap, Bp, dV, &a2);
+    double A[3], B[3], Ap[3], Bp[3], dV[3], a2, ia;
+    fippi_far_setup(Va, Vb, A, B, Ap, Bp, dV, &a2, &ia);
     for (int q = lane; q < N_FIP * N_FIP * N_FIP; q += 32) {
       const int i1 = q / (N_FIP * N_FIP), j = (q / N_FIP) % N_FIP, l = q % N_FIP;
       const double u = sgx[i1];
-      fippi_far_acc(A, B, Ap, Bp, dV, a2, u, u * sgx[j], sgx[l], sgw[i1] * sgw[j] * sgw[l] * u, F);
+      fippi_far_acc(A, B, Ap, Bp, dV, a2, ia, u, u * sgx[j], sgx[l], sgw[i1] * sgw[j] * sgw[l] * u, F);
     }
   } else {
     double Ea[9], Eb[9];
@@ -459,10 +461,6 @@ __device__ void store_near(double* dst, int ja, int jb, cx<double> kk, cx<double
 // over the lanes and the moments reduced with shuffles
 __global__ void __launch_bounds__(128) self_kernel(const DevNear* near, const int* list, int n, const double* pv,
                                                    RegionArgs ra, double* nearval) {
-  // the 1-D rule in shared memory: the lanes read different nodes at once
-  __shared__ double sgx[NT_SELF], sgw[NT_SELF];
-  if (threadIdx.x < NT_SELF) { sgx[threadIdx.x] = c_gx16[threadIdx.x]; sgw[threadIdx.x] = c_gw16[threadIdx.x]; }
-  __syncthreads();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= n) return;  // whole warps exit together
   int i = list[warp];
@@ -476,7 +474,7 @@ __global__ void __launch_bounds__(128) self_kernel(const DevNear* near, const in
     cx<double> k = ra.k[r];
     if (k.re == 0.0 && k.im == 0.0) continue;
     cx<double> MG[9], MP[9];
-    self_moments(V, k, sgx, sgw, NT_SELF, MG, lane, 32);
+    self_moments(V, k, g_self_tab, 6 * NT_SELF, MG, lane, 32);
     for (int m = 0; m < 9; m++) {
       for (int o = 16; o > 0; o >>= 1) {
         MG[m].re += __shfl_xor_sync(0xffffffff, MG[m].re, o);
@@ -502,52 +500,75 @@ __global__ void __launch_bounds__(128) self_kernel(const DevNear* near, const in
   }
 }
 
-__global__ void near_kernel(const DevNear* near, const int* list, int n, const double* pv, const Fippi* fippi,
-                            RegionArgs ra, double* nearval, int* status) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  int i = list[t];
-  DevNear d = near[i];
-  double Va[9], Vb[9];
-  for (int c = 0; c < 9; c++) { Va[c] = pv[9 * (size_t)d.pa + c]; Vb[c] = pv[9 * (size_t)d.pb + c]; }
+// Two lanes per pair and region, half of the first panel's points each: the
+// FP64 pipe issues a warp's operation in 64 cycles, so a pair's chain of
+// operations is what bounds a few thousand pairs (13400 operations per pair in
+// one lane: 0.71 ms at N = 960, 0.98 at 3840; 2200 in each of four: 0.17 and
+// 0.52).  After the moments are summed each lane forms five of the nine
+// (Qa, Qb) values; the regions' lanes add theirs.
+template <int NREG>
+__global__ void __launch_bounds__(64) near_kernel(const DevNear* near, const int* list, int n, const double* pv,
+                                                  const Fippi* fippi, RegionArgs ra, double* nearval) {
+  constexpr int LP = 2 * NREG;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = t / LP < n;  // the others keep the warp's shuffles company
+  const int i = list[live ? t / LP : n - 1], half = t & 1, r = NREG == 2 ? (t >> 1) & 1 : 0;
+  const DevNear d = near[i];
   PairGeom<double> g;
   for (int c = 0; c < 3; c++) {
+    const double* Va = pv + 9 * (size_t)d.pa;
+    const double* Vb = pv + 9 * (size_t)d.pb;
     g.D0[c] = Va[c] - Vb[c];
     g.Aa[c] = Va[3 + c] - Va[c]; g.Ba[c] = Va[6 + c] - Va[c];
     g.Ab[c] = Vb[3 + c] - Vb[c]; g.Bb[c] = Vb[6 + c] - Vb[c];
   }
-  double* dst = nearval + 54 * (size_t)i;
-  for (int c = 0; c < 54; c++) dst[c] = 0.0;
   const Fippi& F = fippi[i];  // read where used: keeps 33 doubles out of registers
-  for (int r = 0; r < ra.nreg; r++) {
-    cx<double> k = ra.k[r];
-    if (k.re == 0.0 && k.im == 0.0) continue;
-    // short-wavelength test of PanelPanelInteractions.cc:416-418
-    cx<double> kr = mk(k.re * d.rmax, k.im * d.rmax);
-    bool sw = hypot(kr.re, kr.im) > M_PI;
-    cx<double> MG[9], MP[9];
-    bool desing = false;
-    if (!sw) {
-      pair_moments<double, 1>(g, k, c_lo64, 6, MG, MP);
-      add_taylor_terms(F, k, MG, MP);
-      desing = true;
-    } else if (d.ncv == 0) {
-      pair_moments<double, 0>(g, k, c_ho, HO_N * HO_N, MG, MP);
-    } else {
-      // touching pair in the short-wavelength regime: td_touch_kernel adds
-      // this region's full-kernel Taylor-Duffy values after this kernel
-      continue;
-    }
-    cx<double> m4ok2 = cdiv(mk(-4.0, 0.0), k * k);
-    VecMoments<double> vm;
-    vec_moments(g, MG, MP, &vm);
-    for (int ja = 0; ja < 3; ja++)
-      for (int jb = 0; jb < 3; jb++) {
-        cx<double> H0, H1;
-        vec_combine(g, vm, ja, jb, m4ok2, &H0, &H1);
-        if (desing) H1 = H1 + mk(-0.079577471545947667884 * htimes_rm3(F, Va, Vb, ja, jb), 0.0);
-        store_near(dst, ja, jb, ra.pf1[r] * H0, ra.pfc[r] * H1, ra.pf3[r] * H0);
+  const cx<double> k = ra.k[r];
+  const bool on = !(k.re == 0.0 && k.im == 0.0);
+  // short-wavelength test of PanelPanelInteractions.cc:416-418
+  const bool sw = hypot(k.re * d.rmax, k.im * d.rmax) > M_PI;
+  // a touching pair in the short-wavelength regime: td_touch_kernel adds this
+  // region's full-kernel Taylor-Duffy values after this kernel
+  const bool sum = on && !(sw && d.ncv != 0);
+  cx<double> MG[9], MP[9];
+  if (sum && sw) {
+    constexpr int NP = HO_N * HO_N, HP = (NP + 1) / 2;
+    pair_moments_rows<double, 0>(g, k, c_ho, NP, half ? HP : 0, half ? NP : HP, MG, MP);
+  } else {
+    pair_moments_rows<double, 1>(g, on ? k : mk(1.0, 0.0), c_lo64, 6, half ? 3 : 0, half ? 6 : 3, MG, MP);
+  }
+#pragma unroll
+  for (int m = 0; m < 9; m++) {
+    MG[m].re += __shfl_xor_sync(0xffffffffu, MG[m].re, 1); MG[m].im += __shfl_xor_sync(0xffffffffu, MG[m].im, 1);
+    MP[m].re += __shfl_xor_sync(0xffffffffu, MP[m].re, 1); MP[m].im += __shfl_xor_sync(0xffffffffu, MP[m].im, 1);
+  }
+  if (!sw) add_taylor_terms(F, k, MG, MP);
+  PairScalars<double> ps;
+  pair_scalars(g, &ps);
+  cx<double> H0[9], H1[9];
+  h0_all(ps, MG, cdiv(mk(-4.0, 0.0), k * k), H0);
+  h1_all(ps, MP, H1);
+  if (!sw) {
+    double h[9];
+    htimes_rm3_all(F, g, h);
+#pragma unroll
+    for (int c = 0; c < 9; c++) H1[c].re -= 0.079577471545947667884 * h[c];
+  }
+  double* dst = nearval + 54 * (size_t)i;
+#pragma unroll
+  for (int q = 0; q < 5; q++) {  // combinations 0 .. 4 or 5 .. 8
+    const int c1 = q < 4 ? 5 + q : 8, c = half ? c1 : q;
+    const cx<double> h0 = half ? H0[c1] : H0[q], h1 = half ? H1[c1] : H1[q];
+    cx<double> v[3] = {ra.pf1[r] * h0, ra.pfc[r] * h1, ra.pf3[r] * h0};
+#pragma unroll
+    for (int f = 0; f < 3; f++) {
+      if (!sum) v[f] = mk(0.0, 0.0);
+      if (NREG == 2) {
+        v[f].re += __shfl_xor_sync(0xffffffffu, v[f].re, 2);
+        v[f].im += __shfl_xor_sync(0xffffffffu, v[f].im, 2);
       }
+      if (live && r == 0 && (q < 4 || !half)) *reinterpret_cast<double2*>(dst + 6 * c + 2 * f) = make_double2(v[f].re, v[f].im);
+    }
   }
 }
 
@@ -1552,10 +1573,7 @@ gbem_status assemble_device(Geometry* g, double wr, double wi, const double* eps
     }
     if (e != cudaSuccess) return cuda_status(e, "memset matrix");
   }
-  int* d_status = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&d_status, sizeof(int), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_status, 0, sizeof(int), s);
-  if (e != cudaSuccess) return cuda_status(e, "status word");
+  cudaError_t e = cudaSuccess;
   for (size_t bi = 0; bi < g->blocks.size(); bi++) {
     const Block& b = g->blocks[bi];
     DevBlock* db = g->dblocks[bi];
@@ -1575,8 +1593,11 @@ gbem_status assemble_device(Geometry* g, double wr, double wi, const double* eps
       }
       if (db->nother) {
         stats_launch(ST_NEAR);
-        near_kernel<<<(db->nother + 63) / 64, 64, 0, s>>>(db->near, db->other_list, db->nother, g->d_pv, db->fippi,
-                                                          ra, db->nearval, d_status);
+        const int blocks = (2 * ra.nreg * db->nother + 63) / 64;
+        if (ra.nreg == 2)
+          near_kernel<2><<<blocks, 64, 0, s>>>(db->near, db->other_list, db->nother, g->d_pv, db->fippi, ra, db->nearval);
+        else
+          near_kernel<1><<<blocks, 64, 0, s>>>(db->near, db->other_list, db->nother, g->d_pv, db->fippi, ra, db->nearval);
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "near_kernel");
         // touching pairs in the short-wavelength regime (only when some k |r| can exceed pi)
         double kmax = 0.0;
@@ -1620,16 +1641,8 @@ gbem_status assemble_device(Geometry* g, double wr, double wi, const double* eps
     }
     if (e != cudaSuccess) return cuda_status(e, "tile_kernel");
   }
-  int h_status = 0;
-  e = cudaMemcpyAsync(&h_status, d_status, sizeof(int), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaFreeAsync(d_status, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_status(e, "assembly");
-  if (h_status) {
-    set_error("touching panel pairs in the short-wavelength regime (|k r| > pi) need the full-kernel "
-              "Taylor-Duffy path, which this build does not implement");
-    return GBEM_ENOTSUP;
-  }
   return GBEM_OK;
 }
 
@@ -2358,8 +2371,7 @@ __global__ void __launch_bounds__(128) vjp_far_kernel(VjpFarArgs a, RegionArgs r
 // the edge lengths taken from the positions.  Every lane returns the value.
 __device__ double near_pair_energy(const DevNear& d, const double* Va, const double* Vb, const double* sgA,
                                    const double* sgB, const RegionArgs& ra, const cx<double> (*W)[9], int lane,
-                                   const double* sgx8, const double* sgw8, const double* srule6,
-                                   const double* srule16) {
+                                   const double* sgx8, const double* sgw8, const double* srule6) {
   const bool self = d.pa == d.pb;
   // lane m < 9 forms the (Qa, Qb) combination m = 3 ja + jb; the sums over
   // cubature points before it are spread over all lanes
@@ -2391,7 +2403,7 @@ __device__ double near_pair_energy(const DevNear& d, const double* Va, const dou
     cx<double> H0, H1;
     if (self) {
       cx<double> MG[9], MP[9];
-      self_moments(Va, k, srule16, srule16 + NT_SELF, NT_SELF, MG, lane, 32);
+      self_moments(Va, k, g_self_tab, 6 * NT_SELF, MG, lane, 32);
       cx_warp_sum(MG, 9);
       for (int q = 0; q < 9; q++) MP[q] = mk(0.0, 0.0);
       double c[9], dd[9];
@@ -2450,11 +2462,10 @@ __global__ void __launch_bounds__(128) vjp_near_kernel(VjpNearArgs a, RegionArgs
   // vertex 0 follows from the others) x 3 coordinates; each warp evaluates
   // its two displaced pairs with the lanes over the cubature points
   // the rules in shared memory: the lanes read different nodes at once
-  __shared__ double sgx[N_FIP_ADJ], sgw[N_FIP_ADJ], srule6[18], srule16[2 * NT_SELF];
+  __shared__ double sgx[N_FIP_ADJ], sgw[N_FIP_ADJ], srule6[18];
   __shared__ cx<double> sW[4][3][9];  // per warp: the pair's weights (kept out of registers)
   if (threadIdx.x < N_FIP_ADJ) { sgx[threadIdx.x] = c_gx8[threadIdx.x]; sgw[threadIdx.x] = c_gw8[threadIdx.x]; }
   if (threadIdx.x < 18) srule6[threadIdx.x] = c_lo64[threadIdx.x];
-  if (threadIdx.x < NT_SELF) { srule16[threadIdx.x] = c_gx16[threadIdx.x]; srule16[NT_SELF + threadIdx.x] = c_gw16[threadIdx.x]; }
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const long long wid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
@@ -2496,7 +2507,7 @@ __global__ void __launch_bounds__(128) vjp_near_kernel(VjpNearArgs a, RegionArgs
       if (t.pvi[3 * d.pa + q] == gv) Va[3 * q + c] += dv;
       if (t.pvi[3 * d.pb + q] == gv) Vb[3 * q + c] += dv;
     }
-    E[s] = near_pair_energy(d, Va, Vb, sgA, sgB, ra, W, lane, sgx, sgw, srule6, srule16);
+    E[s] = near_pair_energy(d, Va, Vb, sgA, sgB, ra, W, lane, sgx, sgw, srule6);
   }
   const double dE = (E[0] - E[1]) / (2.0 * h);
   if (lane == 0) {

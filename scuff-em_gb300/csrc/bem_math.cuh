@@ -126,6 +126,14 @@ GB_HD float rsqrt_t(float x) {
 }
 GB_HD double rsqrt_t(double x) { return 1.0 / sqrt(x); }
 
+GB_HD double rsqrt_d(double x) {
+#ifdef __CUDA_ARCH__
+  return rsqrt(x);
+#else
+  return 1.0 / sqrt(x);
+#endif
+}
+
 // Phi = e^{ikr}/(4 pi r), Psi = Phi (ik - 1/r)/r, both times the weight w.
 template <typename T>
 GB_HD void helmholtz_pp(T r2, cx<T> k, T w, cx<T>* phi, cx<T>* psi) {
@@ -143,21 +151,53 @@ GB_HD void helmholtz_pp(T r2, cx<T> k, T w, cx<T>* phi, cx<T>* psi) {
   *psi = p * f;
 }
 
+// exprel4 of i y and of a real x: the same terms, the same truncation rule, in
+// real arithmetic (7 operations per term in place of 17)
+GB_HD cx<double> exprel4_imag(double y) {
+  double t = 1.0;
+  for (int m = 1; m < 4; m++) t = recip_int(m) * (t * y);
+  double s[2] = {0.0, 0.0};  // i^m by m mod 4: 1, i, -1, -i
+  for (int m = 4; m < 100; m += 2) {
+    const double sg = (m & 2) ? -1.0 : 1.0;
+    t = recip_int(m) * (t * y);
+    s[0] = s[0] + sg * t;
+    if (t * t < 1.0e-16 * (s[0] * s[0] + s[1] * s[1])) break;
+    t = recip_int(m + 1) * (t * y);
+    s[1] = s[1] + sg * t;
+    if (t * t < 1.0e-16 * (s[0] * s[0] + s[1] * s[1])) break;
+  }
+  return mk(s[0], s[1]);
+}
+GB_HD double exprel4_real(double x) {
+  double t = 1.0, s = 0.0;
+  for (int m = 1; m < 4; m++) t = recip_int(m) * (t * x);
+  for (int m = 4; m < 100; m++) {
+    t = recip_int(m) * (t * x);
+    s = s + t;
+    if (t * t < 1.0e-16 * (s * s)) break;
+  }
+  return s;
+}
+
 GB_HD void desing_pp(double r2, cx<double> k, double w, cx<double>* phi, cx<double>* psi) {
   const double inv4pi = 0.079577471545947667884;
-  double r = sqrt(r2), rinv = 1.0 / r;
-  cx<double> ikr = mk(-k.im * r, k.re * r);
-  cx<double> p = (w * inv4pi * rinv) * exprel4(ikr);
-  cx<double> f = mk((-k.im - rinv) * rinv, k.re * rinv);
+  const double rinv = rsqrt_d(r2), r = r2 * rinv;
+  cx<double> e;
+  if (k.im == 0.0) e = exprel4_imag(k.re * r);
+  else if (k.re == 0.0) e = mk(exprel4_real(-k.im * r), 0.0);
+  else e = exprel4(mk(-k.im * r, k.re * r));
+  const cx<double> p = (w * inv4pi * rinv) * e;
+  const cx<double> f = mk((-k.im - rinv) * rinv, k.re * rinv);
   *phi = p;
   *psi = p * f;
 }
 
-// rule: npts triples (u, v, w)
+// rule: npts triples (u, v, w); the first panel's points i0 .. i1-1
 template <typename T, int DESING>
-GB_HD void pair_moments(const PairGeom<T>& g, cx<T> k, const T* rule, int npts, cx<T>* MG, cx<T>* MP) {
+GB_HD void pair_moments_rows(const PairGeom<T>& g, cx<T> k, const T* rule, int npts, int i0, int i1, cx<T>* MG,
+                             cx<T>* MP) {
   for (int m = 0; m < 9; m++) { MG[m] = mk((T)0, (T)0); MP[m] = mk((T)0, (T)0); }
-  for (int i = 0; i < npts; i++) {
+  for (int i = i0; i < i1; i++) {
     T u = rule[3 * i], v = rule[3 * i + 1], wi = rule[3 * i + 2];
     T pa[3];
     for (int c = 0; c < 3; c++) pa[c] = g.D0[c] + u * g.Aa[c] + v * g.Ba[c];
@@ -183,6 +223,11 @@ GB_HD void pair_moments(const PairGeom<T>& g, cx<T> k, const T* rule, int npts, 
         MP[3 * al + b] = MP[3 * al + b] + a[al] * SP[b];
       }
   }
+}
+
+template <typename T, int DESING>
+GB_HD void pair_moments(const PairGeom<T>& g, cx<T> k, const T* rule, int npts, cx<T>* MG, cx<T>* MP) {
+  pair_moments_rows<T, DESING>(g, k, rule, npts, 0, npts, MG, MP);
 }
 
 // pair_moments with the npts x npts samples dealt out: this call adds the
@@ -392,13 +437,9 @@ GB_HD void expint_moments(cx<double> z, cx<double>* E) {
     for (int n = 0; n <= NMAX; n++) E[n] = mk(recip_int(n + 1), 0.0);
     for (int m = 1; m < 60; m++) {
       term = recip_int(m) * (term * z);
-      double worst = 0.0;
-      for (int n = 0; n <= NMAX; n++) {
-        const cx<double> t = recip_int(n + m + 1) * term;
-        E[n] = E[n] + t;
-        worst = fmax(worst, cnorm2(t) / cnorm2(E[n]));
-      }
-      if (worst < 1e-36) break;
+      for (int n = 0; n <= NMAX; n++) E[n] = E[n] + recip_int(n + m + 1) * term;
+      // |z| < 2 keeps |E_n| above 0.1 / (n + 1): the terms left out are below 1e-18 of it
+      if (cnorm2(term) < 1e-40) break;
     }
   } else {
     const cx<double> ez = cexpo(z), zi = cdiv(mk(1.0, 0.0), z);
@@ -456,63 +497,79 @@ GB_HD rpoly rp_mul(const rpoly& a, const rpoly& b) {
 // ---------------------------------------------------------------------------
 // Outer points (sector, t) with linear index p = sector*nt + t are visited
 // for p = p0, p0 + pstride, ... (a warp can split them over its lanes).
-GB_HD void self_moments(const double* V, cx<double> k, const double* gx, const double* gw, int nt, cx<double>* MG,
-                        int p0 = 0, int pstride = 1) {
-  const double inv4pi = 0.079577471545947667884;
-  double E1[3], E2[3];
-  for (int i = 0; i < 3; i++) { E1[i] = V[3 + i] - V[i]; E2[i] = V[6 + i] - V[3 + i]; }
+// The polynomial part of outer point (sector sct, parameter t): summed over the
+// three s' points, om ma mb = sum_n Q[m][n] w^n per monomial pair m.  It does not
+// depend on the triangle, so a table of it (self_table) serves every pair.
+GB_HD void self_poly(int sct, double t, double* zz, double Q[9][5]) {
   const double H[7][2] = {{1, 0}, {1, 1}, {0, 1}, {-1, 0}, {-1, -1}, {0, -1}, {1, 0}};
   const double TP[3][2] = {{0.5, 0.0}, {1.0, 0.5}, {0.5, 0.5}};
-  for (int m = 0; m < 9; m++) MG[m] = mk(0.0, 0.0);
-  for (int pp = p0; pp < 6 * nt; pp += pstride) {
-      const int sct = pp / nt, it = pp - sct * nt;
-      {
-      double t = gx[it];
-      double z0 = H[sct][0] + t * (H[sct + 1][0] - H[sct][0]);
-      double z1 = H[sct][1] + t * (H[sct + 1][1] - H[sct][1]);
-      double am = z1 < 0 ? -z1 : 0.0, bm = z0 > 0 ? z0 : 0.0, cm = (z0 - z1) < 0 ? (z0 - z1) : 0.0;
-      double sig = bm + am - cm;
-      double D[3];
-      for (int i = 0; i < 3; i++) D[i] = z0 * E1[i] + z1 * E2[i];
-      double X = sqrt(vdot(D, D));
-      cx<double> E[5];
-      expint_moments<4>(mk(-k.im * X, k.re * X), E);
-      // om = lambda^2 = (1 - sig w)^2 (the w lambda^2 of the Jacobian over the 1/w of G)
-      const double om0 = 1.0, om1 = -2.0 * sig, om2 = sig * sig;
-      const double W = gw[it] * (1.0 / 6.0) * inv4pi / X;
-      // sum over the three s' points of the degree-4 polynomials om * ma * mb, then
-      // one combination with E_0..E_4 per monomial pair
-      double Q[9][5];
-      for (int m = 0; m < 9; m++)
-        for (int n = 0; n < 5; n++) Q[m][n] = 0.0;
-      for (int ip = 0; ip < 3; ip++) {
-        double p1 = TP[ip][0], p2 = TP[ip][1];
-        // s' = (p1, p2) + w ((am - cm) - sig p1, am - sig p2);  s = s' + w z
-        double sb0 = p1, sb1 = (am - cm) - sig * p1, tb0 = p2, tb1 = am - sig * p2;
-        double sa0 = sb0, sa1 = sb1 + z0, ta0 = tb0, ta1 = tb1 + z1;
-        // TCR coordinates u = s1 - s2, v = s2, affine in w: (c0, c1)
-        const double ma[3][2] = {{1.0, 0.0}, {sa0 - ta0, sa1 - ta1}, {ta0, ta1}};
-        const double mb[3][2] = {{1.0, 0.0}, {sb0 - tb0, sb1 - tb1}, {tb0, tb1}};
-        for (int al = 0; al < 3; al++) {
-          const double P0 = om0 * ma[al][0], P1 = om0 * ma[al][1] + om1 * ma[al][0],
-                       P2 = om1 * ma[al][1] + om2 * ma[al][0], P3 = om2 * ma[al][1];
-          for (int be = 0; be < 3; be++) {
-            const double n0 = mb[be][0], n1 = mb[be][1];
-            double* q = Q[3 * al + be];
-            q[0] += P0 * n0;
-            q[1] += P0 * n1 + P1 * n0;
-            q[2] += P1 * n1 + P2 * n0;
-            q[3] += P2 * n1 + P3 * n0;
-            q[4] += P3 * n1;
-          }
-        }
-      }
-      for (int m = 0; m < 9; m++) {
-        cx<double> sm = mk(0.0, 0.0);
-        for (int n = 0; n < 5; n++) sm = sm + Q[m][n] * E[n];
-        MG[m] = MG[m] + W * sm;
+  const double z0 = H[sct][0] + t * (H[sct + 1][0] - H[sct][0]);
+  const double z1 = H[sct][1] + t * (H[sct + 1][1] - H[sct][1]);
+  const double am = z1 < 0 ? -z1 : 0.0, bm = z0 > 0 ? z0 : 0.0, cm = (z0 - z1) < 0 ? (z0 - z1) : 0.0;
+  const double sig = bm + am - cm;
+  // om = lambda^2 = (1 - sig w)^2 (the w lambda^2 of the Jacobian over the 1/w of G)
+  const double om0 = 1.0, om1 = -2.0 * sig, om2 = sig * sig;
+  zz[0] = z0;
+  zz[1] = z1;
+  for (int m = 0; m < 9; m++)
+    for (int n = 0; n < 5; n++) Q[m][n] = 0.0;
+  for (int ip = 0; ip < 3; ip++) {
+    const double p1 = TP[ip][0], p2 = TP[ip][1];
+    // s' = (p1, p2) + w ((am - cm) - sig p1, am - sig p2);  s = s' + w z
+    const double sb0 = p1, sb1 = (am - cm) - sig * p1, tb0 = p2, tb1 = am - sig * p2;
+    const double sa0 = sb0, sa1 = sb1 + z0, ta0 = tb0, ta1 = tb1 + z1;
+    // TCR coordinates u = s1 - s2, v = s2, affine in w: (c0, c1)
+    const double ma[3][2] = {{1.0, 0.0}, {sa0 - ta0, sa1 - ta1}, {ta0, ta1}};
+    const double mb[3][2] = {{1.0, 0.0}, {sb0 - tb0, sb1 - tb1}, {tb0, tb1}};
+    for (int al = 0; al < 3; al++) {
+      const double P0 = om0 * ma[al][0], P1 = om0 * ma[al][1] + om1 * ma[al][0],
+                   P2 = om1 * ma[al][1] + om2 * ma[al][0], P3 = om2 * ma[al][1];
+      for (int be = 0; be < 3; be++) {
+        const double n0 = mb[be][0], n1 = mb[be][1];
+        double* q = Q[3 * al + be];
+        q[0] += P0 * n0;
+        q[1] += P0 * n1 + P1 * n0;
+        q[2] += P1 * n1 + P2 * n0;
+        q[3] += P2 * n1 + P3 * n0;
+        q[4] += P3 * n1;
       }
     }
+  }
+}
+
+// The table: 48 rows of 6 nt outer points -- Q[m][n] at row 5 m + n, then the
+// weight over 24 pi, z0 and z1 (consecutive points adjacent: lanes read them together).
+constexpr int SELF_ROWS = 48;
+inline void self_table(const double* gx, const double* gw, int nt, double* tab) {
+  const int np = 6 * nt;
+  for (int p = 0; p < np; p++) {
+    double z[2], Q[9][5];
+    self_poly(p / nt, gx[p % nt], z, Q);
+    for (int m = 0; m < 9; m++)
+      for (int n = 0; n < 5; n++) tab[(5 * m + n) * np + p] = Q[m][n];
+    tab[45 * np + p] = gw[p % nt] * (1.0 / 6.0) * 0.079577471545947667884;
+    tab[46 * np + p] = z[0];
+    tab[47 * np + p] = z[1];
+  }
+}
+
+// the common-triangle moments: outer points p0, p0 + pstride, ... of the table
+GB_HD void self_moments(const double* V, cx<double> k, const double* tab, int np, cx<double>* MG, int p0 = 0,
+                        int pstride = 1) {
+  double E1[3], E2[3];
+  for (int i = 0; i < 3; i++) { E1[i] = V[3 + i] - V[i]; E2[i] = V[6 + i] - V[3 + i]; }
+  for (int m = 0; m < 9; m++) MG[m] = mk(0.0, 0.0);
+  for (int pp = p0; pp < np; pp += pstride) {
+    const double z0 = tab[46 * np + pp], z1 = tab[47 * np + pp];
+    double D[3];
+    for (int i = 0; i < 3; i++) D[i] = z0 * E1[i] + z1 * E2[i];
+    const double X = sqrt(vdot(D, D));
+    cx<double> E[5];
+    expint_moments<4>(mk(-k.im * X, k.re * X), E);
+    const double W = tab[45 * np + pp] / X;
+    for (int n = 0; n < 5; n++) E[n] = W * E[n];
+    for (int m = 0; m < 9; m++)
+      for (int n = 0; n < 5; n++) MG[m] = MG[m] + tab[(5 * m + n) * np + pp] * E[n];
   }
 }
 
@@ -531,27 +588,31 @@ struct Fippi {
 // Segment integrals along the second panel's v' direction (closed forms of
 // int (t^2+b2)^{p/2} t^j dt), p = -3, -1, 1, 2; j = 0, 1
 // (QIFIPPICubature.cc:240-300 evaluates the same integrals).
-GB_HD void seg_integrals(double a2, double v0, double b2, double up, double J[4][2]) {
-  double a = sqrt(a2);
-  double t1 = -v0, t2 = up - v0;
-  double S1 = sqrt(t1 * t1 + b2), S2 = sqrt(t2 * t2 + b2);
-  double L;
-  if (t1 >= 0) L = log((t2 + S2) / (t1 + S1));
-  else if (t2 <= 0) L = log((S1 - t1) / (S2 - t2));
-  else L = log((t2 + S2) * (S1 - t1) / b2);
-  double Im3_0;
-  if (t1 * t2 > 0) Im3_0 = (t2 * t2 - t1 * t1) / (S1 * S2 * (t2 * S1 + t1 * S2));
-  else Im3_0 = (t2 / S2 - t1 / S1) / b2;
-  double Im3_1 = 1.0 / S1 - 1.0 / S2;
-  double Im1_0 = L, Im1_1 = S2 - S1;
-  double I1_0 = 0.5 * (t2 * S2 - t1 * S1 + b2 * L), I1_1 = (S2 * S2 * S2 - S1 * S1 * S1) / 3.0;
-  double I2_0 = (t2 * t2 * t2 - t1 * t1 * t1) / 3.0 + b2 * (t2 - t1);
-  double q1 = t1 * t1 + b2, q2 = t2 * t2 + b2;
-  double I2_1 = (q2 * q2 - q1 * q1) / 4.0;
-  J[0][0] = Im3_0 / (a2 * a); J[0][1] = (Im3_1 + v0 * Im3_0) / (a2 * a);
-  J[1][0] = Im1_0 / a;        J[1][1] = (Im1_1 + v0 * Im1_0) / a;
-  J[2][0] = I1_0 * a;         J[2][1] = (I1_1 + v0 * I1_0) * a;
-  J[3][0] = I2_0 * a2;        J[3][1] = (I2_1 + v0 * I2_0) * a2;
+// ia: 1/|Bp|, a2 = |Bp|^2.  Two reciprocal square roots, two divisions and a
+// logarithm per point (the rest is products): FP64 divisions and square roots
+// cost 10 to 20 operations each.
+GB_HD void seg_integrals(double a2, double ia, double v0, double b2, double up, double J[4][2]) {
+  const double t1 = -v0, t2 = up - v0;
+  const double q1 = t1 * t1 + b2, q2 = t2 * t2 + b2;
+  const double i1 = rsqrt_d(q1), i2 = rsqrt_d(q2), S1 = q1 * i1, S2 = q2 * i2;
+  double num, den;
+  if (t1 >= 0) { num = t2 + S2; den = t1 + S1; }
+  else if (t2 <= 0) { num = S1 - t1; den = S2 - t2; }
+  else { num = (t2 + S2) * (S1 - t1); den = b2; }
+  const double L = log(num / den);
+  double n3, d3;
+  if (t1 * t2 > 0) { n3 = (t2 * t2 - t1 * t1) * (i1 * i2); d3 = t2 * S1 + t1 * S2; }
+  else { n3 = t2 * i2 - t1 * i1; d3 = b2; }
+  const double Im3_0 = n3 / d3, Im3_1 = i1 - i2;
+  const double Im1_1 = S2 - S1;
+  const double I1_0 = 0.5 * (t2 * S2 - t1 * S1 + b2 * L), I1_1 = (S2 * q2 - S1 * q1) * (1.0 / 3.0);
+  const double I2_0 = (t2 * t2 * t2 - t1 * t1 * t1) * (1.0 / 3.0) + b2 * (t2 - t1);
+  const double I2_1 = (q2 * q2 - q1 * q1) * 0.25;
+  const double a = a2 * ia, ia3 = ia * ia * ia;
+  J[0][0] = Im3_0 * ia3; J[0][1] = (Im3_1 + v0 * Im3_0) * ia3;
+  J[1][0] = L * ia;      J[1][1] = (Im1_1 + v0 * L) * ia;
+  J[2][0] = I1_0 * a;    J[2][1] = (I1_1 + v0 * I1_0) * a;
+  J[3][0] = I2_0 * a2;   J[3][1] = (I2_1 + v0 * I2_0) * a2;
 }
 
 GB_HD void fippi_zero(Fippi* F) {
@@ -563,9 +624,9 @@ GB_HD void fippi_zero(Fippi* F) {
 // tensor Gauss-Legendre rule (the 3-D scheme of QIFIPPICubature.cc:187-325).
 // Va, Vb: 9 doubles each, mesh vertex order.  fippi_far_acc adds one point
 // (u, v = u t, u') of weight W; A, B, Ap, Bp are the panels' edge vectors,
-// dV = V0b - V0a, a2 = |Bp|^2.
+// dV = V0b - V0a, a2 = |Bp|^2, ia = 1/|Bp|.
 GB_HD void fippi_far_acc(const double* A, const double* B, const double* Ap, const double* Bp, const double* dV,
-                         double a2, double u, double v, double up, double W, Fippi& F) {
+                         double a2, double ia, double u, double v, double up, double W, Fippi& F) {
   double Y[3], Xo[3], Zo[3];
 #pragma unroll
   for (int m = 0; m < 3; m++) {
@@ -573,11 +634,12 @@ GB_HD void fippi_far_acc(const double* A, const double* B, const double* Ap, con
     Zo[m] = dV[m] + up * Ap[m];    // z - V0a
     Y[m] = Xo[m] - Zo[m];
   }
-  double v0 = vdot(Bp, Y) / a2;
-  double b2 = vdot(Y, Y) / a2 - v0 * v0;
+  const double ia2 = ia * ia;
+  double v0 = vdot(Bp, Y) * ia2;
+  double b2 = vdot(Y, Y) * ia2 - v0 * v0;
   if (b2 < 0) b2 = 0;
   double J[4][2];
-  seg_integrals(a2, v0, b2, up, J);
+  seg_integrals(a2, ia, v0, b2, up, J);
 #pragma unroll
   for (int m = 0; m < 3; m++) F.XM[m] += W * (Y[m] * J[0][0] - Bp[m] * J[0][1]);
   double XZ[3], XB[3];
@@ -586,34 +648,36 @@ GB_HD void fippi_far_acc(const double* A, const double* B, const double* Ap, con
   for (int m = 0; m < 3; m++) F.XX[m] += W * (XZ[m] * J[0][0] + XB[m] * J[0][1]);
   // TCR a-side monomials {1, u - v, v}; b-side {1, u' - v', v'}
   const double ma[3] = {1.0, u - v, v};
+  const double K1 = up * J[1][0] - J[1][1], K2 = up * J[2][0] - J[2][1], K3 = up * J[3][0] - J[3][1];
 #pragma unroll
   for (int al = 0; al < 3; al++) {
     double f = W * ma[al];
-    F.RM1[3 * al + 0] += f * J[1][0]; F.RM1[3 * al + 1] += f * (up * J[1][0] - J[1][1]); F.RM1[3 * al + 2] += f * J[1][1];
-    F.R1[3 * al + 0] += f * J[2][0];  F.R1[3 * al + 1] += f * (up * J[2][0] - J[2][1]);  F.R1[3 * al + 2] += f * J[2][1];
-    F.R2[3 * al + 0] += f * J[3][0];  F.R2[3 * al + 1] += f * (up * J[3][0] - J[3][1]);  F.R2[3 * al + 2] += f * J[3][1];
+    F.RM1[3 * al + 0] += f * J[1][0]; F.RM1[3 * al + 1] += f * K1; F.RM1[3 * al + 2] += f * J[1][1];
+    F.R1[3 * al + 0] += f * J[2][0];  F.R1[3 * al + 1] += f * K2;  F.R1[3 * al + 2] += f * J[2][1];
+    F.R2[3 * al + 0] += f * J[3][0];  F.R2[3 * al + 1] += f * K3;  F.R2[3 * al + 2] += f * J[3][1];
   }
 }
 
 GB_HD void fippi_far_setup(const double* Va, const double* Vb, double* A, double* B, double* Ap, double* Bp, double* dV,
-                           double* a2) {
+                           double* a2, double* ia) {
   for (int i = 0; i < 3; i++) {
     A[i] = Va[3 + i] - Va[i]; B[i] = Va[6 + i] - Va[3 + i];
     Ap[i] = Vb[3 + i] - Vb[i]; Bp[i] = Vb[6 + i] - Vb[3 + i];
     dV[i] = Vb[i] - Va[i];
   }
   *a2 = vdot(Bp, Bp);
+  *ia = 1.0 / sqrt(*a2);
 }
 
 GB_HD void fippi_far(const double* Va, const double* Vb, const double* gx, const double* gw, int n, Fippi* F) {
-  double A[3], B[3], Ap[3], Bp[3], dV[3], a2;
-  fippi_far_setup(Va, Vb, A, B, Ap, Bp, dV, &a2);
+  double A[3], B[3], Ap[3], Bp[3], dV[3], a2, ia;
+  fippi_far_setup(Va, Vb, A, B, Ap, Bp, dV, &a2, &ia);
   fippi_zero(F);
   for (int i = 0; i < n; i++)
     for (int j = 0; j < n; j++)
       for (int l = 0; l < n; l++) {
         double u = gx[i];
-        fippi_far_acc(A, B, Ap, Bp, dV, a2, u, u * gx[j], gx[l], gw[i] * gw[j] * gw[l] * u, *F);
+        fippi_far_acc(A, B, Ap, Bp, dV, a2, ia, u, u * gx[j], gx[l], gw[i] * gw[j] * gw[l] * u, *F);
       }
 }
 
@@ -693,7 +757,7 @@ GB_HD void fippi_touch_acc(const double* Ea, const double* Eb, const int* pa, co
     Ap[i] = Eb[3 + i] - Eb[i]; Bp[i] = Eb[6 + i] - Eb[3 + i];
     D[i] = pt.sa1[0] * A[i] + pt.sa1[1] * B[i] - pt.sb1[0] * Ap[i] - pt.sb1[1] * Bp[i];
   }
-  const double X = sqrt(vdot(D, D));
+  const double X2 = vdot(D, D), iX = rsqrt_d(X2), X = X2 * iX;
   const double o2 = pt.om.c[2], o3 = pt.om.c[3];
   rpoly ua, va, ub, vb;
   tcr_from_edge(pa, pt.sa0, pt.sa1, &ua, &va);
@@ -706,17 +770,21 @@ GB_HD void fippi_touch_acc(const double* Ea, const double* Eb, const int* pa, co
   const double hm1[3] = {h(0), h(1), h(2)};   // r^-1
   const double h1[3] = {h(2), h(3), h(4)};    // r
   const double h2[3] = {h(3), h(4), h(5)};    // r^2
-  const double iX = 1.0 / X;
-  const double WX = pt.W * X, WXX = pt.W * X * X, WoX = pt.W * iX;
-#pragma unroll
-  for (int al = 0; al < 3; al++)
+  // with the b side first: g0 = b0 h0 + b1 h1 and g1 = b0 h1 + b1 h2 give a0 g0 + a1 g1
+  auto add = [&](const double* hh, double w, double* S) {
+    const double p0 = w * hh[0], p1 = w * hh[1], p2 = w * hh[2];
+    const double g0[3] = {p0, b0[1] * p0 + b1[1] * p1, b0[2] * p0 + b1[2] * p1};
+    const double g1[3] = {p1, b0[1] * p1 + b1[1] * p2, b0[2] * p1 + b1[2] * p2};
 #pragma unroll
     for (int be = 0; be < 3; be++) {
-      const double m0 = a0[al] * b0[be], m1 = a0[al] * b1[be] + a1[al] * b0[be], m2 = a1[al] * b1[be];
-      F.RM1[3 * al + be] += WoX * (m0 * hm1[0] + m1 * hm1[1] + m2 * hm1[2]);
-      F.R1[3 * al + be] += WX * (m0 * h1[0] + m1 * h1[1] + m2 * h1[2]);
-      F.R2[3 * al + be] += WXX * (m0 * h2[0] + m1 * h2[1] + m2 * h2[2]);
+      S[be] += g0[be];
+      S[3 + be] += a0[1] * g0[be] + a1[1] * g1[be];
+      S[6 + be] += a0[2] * g0[be] + a1[2] * g1[be];
     }
+  };
+  add(hm1, pt.W * iX, F.RM1);
+  add(h1, pt.W * X, F.R1);
+  add(h2, pt.W * X2, F.R2);
   // (x - x')/r^3 = D / (w^2 X^3): int om w^-2 = o2 + o3 / 2
   const double iX3 = iX * iX * iX;
   const double om2 = o2 + 0.5 * o3;
@@ -883,6 +951,27 @@ GB_HD void add_taylor_terms(const Fippi& F, cx<double> k, cx<double>* MG, cx<dou
   for (int m = 0; m < 9; m++) {
     MG[m] = MG[m] + F.RM1[m] * PF[0] + R0[m] * PF[1] + (0.5 * F.R1[m]) * PF[2] + (F.R2[m] / 6.0) * PF[3];
     MP[m] = MP[m] + (0.5 * F.RM1[m]) * PF[2] + (R0[m] / 3.0) * PF[3] + (F.R1[m] / 6.0) * PF[4];
+  }
+}
+
+// htimes_rm3 for all nine (Qa, Qb): with qa in {0, Aa, Ba}, qb = {0, Ab, Bb} - D0,
+// (qa - qb).XX + (qa x qb).XM = qa.XX - qb.XX + qb.(XM x qa)
+GB_HD void htimes_rm3_all(const Fippi& F, const PairGeom<double>& g, double* h) {
+  const double* a[3] = {nullptr, g.Aa, g.Ba};
+  double qb[3][3], bx[3];
+  for (int c = 0; c < 3; c++) {
+    qb[0][c] = -g.D0[c];
+    qb[1][c] = g.Ab[c] - g.D0[c];
+    qb[2][c] = g.Bb[c] - g.D0[c];
+  }
+  for (int j = 0; j < 3; j++) bx[j] = vdot(qb[j], F.XX);
+  for (int i = 0; i < 3; i++) {
+    double x[3] = {0.0, 0.0, 0.0}, ax = 0.0;
+    if (i) {
+      vcross(F.XM, a[i], x);
+      ax = vdot(a[i], F.XX);
+    }
+    for (int j = 0; j < 3; j++) h[3 * i + j] = (ax - bx[j]) + (i ? vdot(qb[j], x) : 0.0);
   }
 }
 
