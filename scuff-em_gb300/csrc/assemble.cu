@@ -500,19 +500,21 @@ __global__ void __launch_bounds__(128) self_kernel(const DevNear* near, const in
   }
 }
 
-// Two lanes per pair and region, half of the first panel's points each: the
-// FP64 pipe issues a warp's operation in 64 cycles, so a pair's chain of
-// operations is what bounds a few thousand pairs (13400 operations per pair in
-// one lane: 0.71 ms at N = 960, 0.98 at 3840; 2200 in each of four: 0.17 and
-// 0.52).  After the moments are summed each lane forms five of the nine
-// (Qa, Qb) values; the regions' lanes add theirs.
+// Two lanes per pair and region, half of the first panel's points each, and a
+// warp per region (their wavenumbers take different branches): the FP64 pipe
+// issues a warp's operation in 64 cycles, so a pair's chain of operations is what
+// bounds a few thousand pairs (13400 in one lane, about 2000 in each of four).
+// After the moments are summed each lane forms five of the nine (Qa, Qb) values;
+// the second region's warp hands its own over through shared memory.
 template <int NREG>
 __global__ void __launch_bounds__(64) near_kernel(const DevNear* near, const int* list, int n, const double* pv,
                                                   const Fippi* fippi, RegionArgs ra, double* nearval) {
-  constexpr int LP = 2 * NREG;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = t / LP < n;  // the others keep the warp's shuffles company
-  const int i = list[live ? t / LP : n - 1], half = t & 1, r = NREG == 2 ? (t >> 1) & 1 : 0;
+  __shared__ cx<double> other[NREG == 2 ? 15 : 1][32];  // the second region's values
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = NREG == 2 ? warp : 0, half = lane & 1;
+  const int p = (blockIdx.x * (NREG == 2 ? 1 : 2) + (NREG == 2 ? 0 : warp)) * 16 + (lane >> 1);
+  const bool live = p < n;  // the others keep the warp's shuffles company
+  const int i = list[live ? p : n - 1];
   const DevNear d = near[i];
   PairGeom<double> g;
   for (int c = 0; c < 3; c++) {
@@ -554,22 +556,29 @@ __global__ void __launch_bounds__(64) near_kernel(const DevNear* near, const int
 #pragma unroll
     for (int c = 0; c < 9; c++) H1[c].re -= 0.079577471545947667884 * h[c];
   }
-  double* dst = nearval + 54 * (size_t)i;
+  cx<double> v[15];  // combinations 0 .. 4 or 5 .. 8, three values each
 #pragma unroll
-  for (int q = 0; q < 5; q++) {  // combinations 0 .. 4 or 5 .. 8
-    const int c1 = q < 4 ? 5 + q : 8, c = half ? c1 : q;
-    const cx<double> h0 = half ? H0[c1] : H0[q], h1 = half ? H1[c1] : H1[q];
-    cx<double> v[3] = {ra.pf1[r] * h0, ra.pfc[r] * h1, ra.pf3[r] * h0};
-#pragma unroll
-    for (int f = 0; f < 3; f++) {
-      if (!sum) v[f] = mk(0.0, 0.0);
-      if (NREG == 2) {
-        v[f].re += __shfl_xor_sync(0xffffffffu, v[f].re, 2);
-        v[f].im += __shfl_xor_sync(0xffffffffu, v[f].im, 2);
-      }
-      if (live && r == 0 && (q < 4 || !half)) *reinterpret_cast<double2*>(dst + 6 * c + 2 * f) = make_double2(v[f].re, v[f].im);
-    }
+  for (int q = 0; q < 5; q++) {
+    const int c1 = q < 4 ? 5 + q : 8;
+    const cx<double> h0 = half ? H0[c1] : H0[q], h1 = half ? H1[c1] : H1[q], z = mk(0.0, 0.0);
+    v[3 * q] = sum ? ra.pf1[r] * h0 : z;
+    v[3 * q + 1] = sum ? ra.pfc[r] * h1 : z;
+    v[3 * q + 2] = sum ? ra.pf3[r] * h0 : z;
   }
+  if (NREG == 2) {
+    if (warp == 1)
+#pragma unroll
+      for (int f = 0; f < 15; f++) other[f][lane] = v[f];
+    __syncthreads();
+    if (warp == 1) return;
+#pragma unroll
+    for (int f = 0; f < 15; f++) v[f] = v[f] + other[f][lane];
+  }
+  if (!live) return;
+  double2* dst = reinterpret_cast<double2*>(nearval + 54 * (size_t)i) + (half ? 15 : 0);
+#pragma unroll
+  for (int f = 0; f < 15; f++)
+    if (f < 12 || !half) dst[f] = make_double2(v[f].re, v[f].im);
 }
 
 // One warp per touching pair (ncv = 1, 2) in the short-wavelength regime
@@ -1593,7 +1602,7 @@ gbem_status assemble_device(Geometry* g, double wr, double wi, const double* eps
       }
       if (db->nother) {
         stats_launch(ST_NEAR);
-        const int blocks = (2 * ra.nreg * db->nother + 63) / 64;
+        const int blocks = (db->nother + (ra.nreg == 2 ? 15 : 31)) / (ra.nreg == 2 ? 16 : 32);
         if (ra.nreg == 2)
           near_kernel<2><<<blocks, 64, 0, s>>>(db->near, db->other_list, db->nother, g->d_pv, db->fippi, ra, db->nearval);
         else
