@@ -332,6 +332,10 @@ void free_geometry_device(Geometry* g) {
   }
   g->dblocks.clear();
   cudaFree(g->d_ffnode); cudaFree(g->d_ffgeo); cudaFree(g->ppv);
+  for (auto& d : g->dsurf) { cudaFree(d.V); cudaFree(d.E); cudaFree(d.L); }
+  g->dsurf.clear();
+  cudaFree(g->d_rhs);
+  g->d_rhs = nullptr;
   cudaFree(g->d_pvi); cudaFree(g->d_sbf); cudaFree(g->d_ssl);
   g->d_pvi = g->d_sbf = nullptr;
   g->d_ssl = nullptr;
@@ -2135,90 +2139,106 @@ struct RhsArgs {
   const int* E;     // 8 ints per edge
   const double* elen;
   int ne, bf_offset, pec, sign;  // sign: -1 incident field outside, +1 inside
-  cx<double> k, Z;               // wavenumber and wave impedance of the source region
-  cx<double> E0[3];
+  cx<double> k;                  // wavenumber of the source region
+  cx<double> E0[3], H0[3];       // field amplitudes, H0 = nh x E0 / Z
   double nh[3];
   cx<double>* rhs;
 };
 
-__device__ void pw_fields(const RhsArgs& a, const double* X, cx<double>* Ef, cx<double>* Hf) {
-  double ph = a.nh[0] * X[0] + a.nh[1] * X[1] + a.nh[2] * X[2];
-  cx<double> ex = cexpo(mk(-a.k.im * ph, a.k.re * ph));
-  for (int i = 0; i < 3; i++) Ef[i] = a.E0[i] * ex;
-  Hf[0] = cdiv(a.nh[1] * Ef[2] - a.nh[2] * Ef[1], a.Z);
-  Hf[1] = cdiv(a.nh[2] * Ef[0] - a.nh[0] * Ef[2], a.Z);
-  Hf[2] = cdiv(a.nh[0] * Ef[1] - a.nh[1] * Ef[0], a.Z);
+// One warp per edge, its 2 x 121 points dealt to the lanes: the FP64 pipe issues
+// a warp's operation in 64 cycles, so one thread per edge walking all points
+// took 1.4 ms at any size; a call for 480 edges took 1.47 ms and takes 0.06.
+__global__ void __launch_bounds__(128) rhs_kernel(RhsArgs a) {
+  constexpr int NQ = HO_N * HO_N;
+  __shared__ double rule[3 * NQ];
+  for (int q = threadIdx.x; q < 3 * NQ; q += blockDim.x) rule[q] = c_ho[q];
+  __syncthreads();
+  const int e = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (e >= a.ne) return;  // whole warps
+  const int* ed = a.E + 8 * e;
+  double V1[3], V2[3];
+  for (int i = 0; i < 3; i++) { V1[i] = a.V[3 * ed[0] + i]; V2[i] = a.V[3 * ed[1] + i]; }
+  cx<double> se = mk(0.0, 0.0), sh = mk(0.0, 0.0);  // P side minus M side
+  for (int p = lane; p < 2 * NQ; p += 32) {
+    const int side = p >= NQ, q = p - side * NQ, iq = side ? ed[3] : ed[2];
+    if (iq < 0) continue;
+    const double u = rule[3 * q], v = rule[3 * q + 1], w = side ? -rule[3 * q + 2] : rule[3 * q + 2];
+    double F[3], ph = 0.0;
+    for (int i = 0; i < 3; i++) {
+      const double Q = a.V[3 * iq + i];
+      F[i] = u * (V1[i] - Q) + v * (V2[i] - Q);
+      ph += a.nh[i] * (Q + F[i]);
+    }
+    double s, c, amp = w;
+    sincos(a.k.re * ph, &s, &c);
+    if (a.k.im != 0.0) amp *= exp(-a.k.im * ph);
+    const cx<double> ex = mk(amp * c, amp * s);
+    se = se + ex * (F[0] * a.E0[0] + F[1] * a.E0[1] + F[2] * a.E0[2]);
+    if (!a.pec) sh = sh + ex * (F[0] * a.H0[0] + F[1] * a.H0[1] + F[2] * a.H0[2]);
+  }
+  se = mk(warp_sum(se.re), warp_sum(se.im));
+  if (!a.pec) sh = mk(warp_sum(sh.re), warp_sum(sh.im));
+  if (lane) return;
+  // (L/2A) int (X-Q).E dA = L int_std (X-Q).E
+  const double ZVAC = 376.73031346177, L = a.elen[e], sg = (double)a.sign;
+  if (a.pec) a.rhs[a.bf_offset + e] = (sg * L / ZVAC) * se;
+  else {
+    a.rhs[a.bf_offset + 2 * e] = (sg * L / ZVAC) * se;
+    a.rhs[a.bf_offset + 2 * e + 1] = (sg * L) * sh;
+  }
 }
 
-__global__ void rhs_kernel(RhsArgs a) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= a.ne) return;
-  const int* ed = a.E + 8 * e;
-  const double* V1 = a.V + 3 * ed[0];
-  const double* V2 = a.V + 3 * ed[1];
-  cx<double> Ep = mk(0.0, 0.0), Hp = mk(0.0, 0.0);
-  for (int side = 0; side < 2; side++) {
-    int iq = side == 0 ? ed[2] : ed[3];
-    if (iq < 0) continue;
-    const double* Q = a.V + 3 * iq;
-    double A[3], B[3];
-    for (int i = 0; i < 3; i++) { A[i] = V1[i] - Q[i]; B[i] = V2[i] - Q[i]; }
-    cx<double> se = mk(0.0, 0.0), sh = mk(0.0, 0.0);
-    for (int q = 0; q < HO_N * HO_N; q++) {
-      double u = c_ho[3 * q], v = c_ho[3 * q + 1], w = c_ho[3 * q + 2];
-      double X[3], F[3];
-      for (int i = 0; i < 3; i++) { F[i] = u * A[i] + v * B[i]; X[i] = Q[i] + F[i]; }
-      cx<double> Ef[3], Hf[3];
-      pw_fields(a, X, Ef, Hf);
-      for (int i = 0; i < 3; i++) { se = se + (w * F[i]) * Ef[i]; sh = sh + (w * F[i]) * Hf[i]; }
-    }
-    // (L/2A) int (X-Q).E dA = L int_std (X-Q).E
-    double L = a.elen[e];
-    if (side == 0) { Ep = Ep + L * se; Hp = Hp + L * sh; }
-    else { Ep = Ep - L * se; Hp = Hp - L * sh; }
+// the surfaces' vertices, edges and edge lengths on the device
+static cudaError_t upload_surfaces(Geometry* g) {
+  if (!g->dsurf.empty()) return cudaSuccess;
+  std::vector<Geometry::SurfaceDev> d(g->S.size());
+  cudaError_t e = cudaSuccess;
+  for (size_t i = 0; i < d.size(); i++) {
+    const Surface& S = g->S[i];
+    if (e == cudaSuccess) e = dupload(&d[i].V, S.V.data(), S.V.size());
+    if (e == cudaSuccess) e = dupload(&d[i].E, S.E.data(), S.E.size());
+    if (e == cudaSuccess) e = dupload(&d[i].L, S.elen.data(), S.elen.size());
   }
-  const double ZVAC = 376.73031346177;
-  double sg = (double)a.sign;
-  if (a.pec) a.rhs[a.bf_offset + e] = (sg / ZVAC) * Ep;
-  else {
-    a.rhs[a.bf_offset + 2 * e] = (sg / ZVAC) * Ep;
-    a.rhs[a.bf_offset + 2 * e + 1] = sg * Hp;
-  }
+  if (e == cudaSuccess) g->dsurf = std::move(d);
+  else
+    for (auto& x : d) { cudaFree(x.V); cudaFree(x.E); cudaFree(x.L); }
+  return e;
 }
 
 gbem_status rhs_planewave_device(Geometry* g, double wr, double wi, const double* eps, const double* mu, const double* E0,
                                  const double* nh, void* d_rhs, cudaStream_t s) {
   gbem_status st = upload_geometry(g);
   if (st != GBEM_OK) return st;
-  cudaError_t e = cudaMemsetAsync(d_rhs, 0, sizeof(double) * 2 * g->N, s);
+  cudaError_t e = upload_surfaces(g);
+  if (e != cudaSuccess) return cuda_status(e, "rhs upload");
+  e = cudaMemsetAsync(d_rhs, 0, sizeof(double) * 2 * g->N, s);
   if (e != cudaSuccess) return cuda_status(e, "rhs memset");
-  for (Surface& S : g->S) {
+  for (size_t i = 0; i < g->S.size(); i++) {
+    const Surface& S = g->S[i];
     // the incident field lives in region 0 (the exterior medium)
     int sign;
     if (S.reg_ext == 0) sign = -1;
     else if (S.reg_int == 0) sign = 1;
     else continue;
+    if (!S.ne) continue;
     RhsArgs a;
-    double *dV = nullptr, *dL = nullptr;
-    int* dE = nullptr;
-    e = dupload(&dV, S.V.data(), S.V.size());
-    if (e == cudaSuccess) e = dupload(&dE, S.E.data(), S.E.size());
-    if (e == cudaSuccess) e = dupload(&dL, S.elen.data(), S.elen.size());
-    if (e != cudaSuccess) return cuda_status(e, "rhs upload");
-    a.V = dV; a.E = dE; a.elen = dL; a.ne = S.ne; a.bf_offset = S.bf_offset; a.pec = S.pec ? 1 : 0; a.sign = sign;
+    a.V = g->dsurf[i].V; a.E = g->dsurf[i].E; a.elen = g->dsurf[i].L;
+    a.ne = S.ne; a.bf_offset = S.bf_offset; a.pec = S.pec ? 1 : 0; a.sign = sign;
     cx<double> ep = cxd(eps[0], eps[1]), m = cxd(mu[0], mu[1]), em = ep * m;
     double rr = std::sqrt(std::hypot(em.re, em.im)), th = 0.5 * std::atan2(em.im, em.re);
     cx<double> rt = cxd(rr * std::cos(th), rr * std::sin(th));  // principal sqrt, as std::sqrt
     a.k = rt * cxd(wr, wi);
     cx<double> q = cdiv(m, ep);
     double rq = std::sqrt(std::hypot(q.re, q.im)), tq = 0.5 * std::atan2(q.im, q.re);
-    a.Z = 376.73031346177 * cxd(rq * std::cos(tq), rq * std::sin(tq));
-    for (int i = 0; i < 3; i++) { a.E0[i] = cxd(E0[2 * i], E0[2 * i + 1]); a.nh[i] = nh[i]; }
+    const cx<double> Z = 376.73031346177 * cxd(rq * std::cos(tq), rq * std::sin(tq));
+    for (int c = 0; c < 3; c++) { a.E0[c] = cxd(E0[2 * c], E0[2 * c + 1]); a.nh[c] = nh[c]; }
+    for (int c = 0; c < 3; c++) {
+      const int c1 = (c + 1) % 3, c2 = (c + 2) % 3;
+      a.H0[c] = cdiv(nh[c1] * a.E0[c2] - nh[c2] * a.E0[c1], Z);
+    }
     a.rhs = (cx<double>*)d_rhs;
-    if (S.ne) rhs_kernel<<<(S.ne + 127) / 128, 128, 0, s>>>(a);
+    rhs_kernel<<<(S.ne + 3) / 4, 128, 0, s>>>(a);
     e = cudaGetLastError();
-    cudaStreamSynchronize(s);
-    cudaFree(dV); cudaFree(dE); cudaFree(dL);
     if (e != cudaSuccess) return cuda_status(e, "rhs_kernel");
   }
   return GBEM_OK;

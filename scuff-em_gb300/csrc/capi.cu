@@ -1617,15 +1617,14 @@ gbem_status gbem_rhs_planewave(gbem_geometry* g, double omega_re, double omega_i
   if (!g || !eps || !mu || !E0 || !nhat || !rhs) { set_error("gbem_rhs_planewave: NULL argument"); return GBEM_EINVAL; }
   gbem_status st0 = ensure_stream(g);
   if (st0 != GBEM_OK) return st0;
-  void* d = nullptr;
-  CHECK_CUDA(cudaMalloc(&d, sizeof(double) * 2 * g->N), "rhs alloc");
-  gbem_status st = rhs_planewave_device(g, omega_re, omega_im, eps, mu, E0, nhat, d, g->stream);
+  std::lock_guard<std::mutex> l(g->rhs_mu);
+  if (!g->d_rhs) CHECK_CUDA(cudaMalloc(&g->d_rhs, sizeof(double) * 2 * std::max(1, g->N)), "rhs alloc");
+  gbem_status st = rhs_planewave_device(g, omega_re, omega_im, eps, mu, E0, nhat, g->d_rhs, g->stream);
   if (st == GBEM_OK) {
-    cudaError_t e = cudaMemcpyAsync(rhs, d, sizeof(double) * 2 * g->N, cudaMemcpyDeviceToHost, g->stream);
+    cudaError_t e = cudaMemcpyAsync(rhs, g->d_rhs, sizeof(double) * 2 * g->N, cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
     if (e != cudaSuccess) st = cuda_status(e, "rhs download");
   }
-  cudaFree(d);
   return st;
 }
 

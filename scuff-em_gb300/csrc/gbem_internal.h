@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <string>
+#include <mutex>
 #include <vector>
 #include <cstdint>
 #include "../../include/gbem.h"
@@ -98,6 +99,16 @@ struct Geometry {
   float* d_ffgeo = nullptr;   // per global panel: V0 - ff_origin, V1 - V0, V2 - V0 as float-float (18 floats)
   void* ppv = nullptr;        // pair-value scratch of the mixed far field
   size_t ppv_bytes = 0;
+  // per surface: vertices, edges and edge lengths (the right-hand sides'
+  // kernels; uploaded on first use), and the right-hand side itself
+  struct SurfaceDev {
+    double* V = nullptr;
+    int* E = nullptr;
+    double* L = nullptr;
+  };
+  std::vector<SurfaceDev> dsurf;
+  void* d_rhs = nullptr;
+  std::mutex rhs_mu;  // guards the two
   // adjoint tables, per global panel (built on first use)
   int* d_pvi = nullptr;       // 3: global vertex indices
   int* d_sbf = nullptr;       // 3: basis function of the edge at each vertex slot, -1 if none
