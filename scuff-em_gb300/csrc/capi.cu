@@ -864,7 +864,7 @@ gbem_status gbem_lu_solve(gbem_matrix* M, char trans, int nrhs, void* B, int ldb
     CHECK_CUDA(cudaMallocAsync(&tA, (size_t)N * N * 16, s), "solve alloc");
     CHECK_CUDA(cudaMallocAsync(&dBr, (size_t)N * nrhs * 8, s), "solve alloc");
     CHECK_CUDA(cudaMallocAsync(&dB, (size_t)N * nrhs * 16, s), "solve alloc");
-    CHECK_CUDA(cudaMallocAsync(&dY, (size_t)N * 8 * 16, s), "solve alloc");
+    CHECK_CUDA(cudaMallocAsync(&dY, lu_solve_ws_bytes(N, GBEM_C128), s), "solve alloc");
     CHECK_CUDA(cudaMemcpy2DAsync(dBr, (size_t)N * 8, B, (size_t)ldb * 8, (size_t)N * 8, nrhs, cudaMemcpyHostToDevice, s),
                "solve upload");
     make_complex<<<(unsigned)(((long long)N * N + 255) / 256), 256, 0, s>>>((const double*)M->d, M->ld, (double2*)tA, N,
@@ -888,7 +888,7 @@ gbem_status gbem_lu_solve(gbem_matrix* M, char trans, int nrhs, void* B, int ldb
   size_t es = esize(M->dtype);
   void *dB = nullptr, *dY = nullptr;
   CHECK_CUDA(cudaMallocAsync(&dB, (size_t)M->N * nrhs * es, M->stream), "solve alloc");
-  CHECK_CUDA(cudaMallocAsync(&dY, (size_t)M->N * 8 * es, M->stream), "solve alloc");
+  CHECK_CUDA(cudaMallocAsync(&dY, lu_solve_ws_bytes(M->N, M->dtype), M->stream), "solve alloc");
   CHECK_CUDA(cudaMemcpy2DAsync(dB, (size_t)M->N * es, B, (size_t)ldb * es, (size_t)M->N * es, nrhs,
                                cudaMemcpyHostToDevice, M->stream), "solve upload");
   gbem_status st = lu_solve_device(M->d, M->N, M->ld, M->dtype, M->d_perm, trans, nrhs, dB, M->N, dY, M->stream);
@@ -1169,7 +1169,7 @@ gbem_status gbem_lu_solve_host(const double* ZM, int N, int ld, const int* ipiv,
   gbem_status st = GBEM_OK;
   cudaError_t e = cudaMalloc(&dA, (size_t)N * N * 16);
   if (e == cudaSuccess) e = cudaMalloc(&dB, (size_t)N * nrhs * 16);
-  if (e == cudaSuccess) e = cudaMalloc(&dY, (size_t)N * 8 * 16);
+  if (e == cudaSuccess) e = cudaMalloc(&dY, lu_solve_ws_bytes(N, GBEM_C128));
   if (e == cudaSuccess) e = cudaMalloc((void**)&dperm, sizeof(int) * N);
   if (e == cudaSuccess)
     e = cudaMemcpy2DAsync(dA, (size_t)N * 16, ZM, (size_t)ld * 16, (size_t)N * 16, N, cudaMemcpyHostToDevice, s);
@@ -1401,7 +1401,7 @@ static gbem_status solve_mixed_impl(gbem_geometry* g, double omega_re, double om
     if (st == GBEM_OK) st = gbem_matrix_create(g, GBEM_C64, &F);
     if (st != GBEM_OK) return st;
     g->mixedM = M; g->mixedF = F;
-    size_t wsb = (size_t)N * nrhs * 16 * 4 + (size_t)N * nrhs * 8 + (size_t)N * 8 * 8 +
+    size_t wsb = (size_t)N * nrhs * 16 * 4 + (size_t)N * nrhs * 8 + lu_solve_ws_bytes(N, GBEM_C64) + 512 +
                  (size_t)RESID_MAX_SPLIT * 8 * N * 16 + 4096;
     cudaError_t e = cudaMalloc(&g->mixed_ws, wsb);
     if (e != cudaSuccess) return cuda_status(e, "gbem_solve_mixed alloc");
@@ -1415,7 +1415,8 @@ static gbem_status solve_mixed_impl(gbem_geometry* g, double omega_re, double om
   void* dR = w; w += (size_t)N * nrhs * 16;
   double* dn = (double*)w; w += (size_t)N * nrhs * 16;
   void* dD = w; w += (size_t)N * nrhs * 8;
-  void* dY = w; w += (size_t)N * 8 * 8;
+  w = (unsigned char*)g->mixed_ws + ((size_t)(w - (unsigned char*)g->mixed_ws) + 255) / 256 * 256;
+  void* dY = w; w += (lu_solve_ws_bytes(N, GBEM_C64) + 255) / 256 * 256;
   void* part = w;
   cudaError_t e = cudaSuccess;
   gbem_matrix* M128 = nullptr;

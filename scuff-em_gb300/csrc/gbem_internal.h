@@ -176,8 +176,9 @@ void cache_stats(const Geometry* g, long long* hits, long long* misses);
 // lu.cu
 gbem_status lu_factor_device(void* dA, int N, int ld, int dtype, int* d_ipiv, int* h_info, cudaStream_t s,
                              void** ws, size_t* ws_bytes);
+size_t lu_solve_ws_bytes(int N, int dtype);
 gbem_status lu_solve_device(const void* dA, int N, int ld, int dtype, const int* d_perm, char trans, int nrhs,
-                            void* dB, int ldb, void* dY, cudaStream_t s);
+                            void* dB, int ldb, void* ws, cudaStream_t s);
 // X = A^-1 B for many right-hand sides (blocked: block inverses + GEMM updates)
 gbem_status lu_solve_many_device(const void* dA, int N, int ld, int dtype, const int* d_perm, int nrhs, void* dB, int ldb,
                                  cudaStream_t s);

@@ -136,3 +136,26 @@ def test_complex_trace_matches_lapack(pec):
     X = sl.solve(A, B)
     tol = np.linalg.cond(A) * N * U * np.linalg.norm(X)
     assert abs(M.TraceMInvdM(B) - np.trace(X[:100])) <= tol
+
+
+@pytest.mark.parametrize("N,nrhs", [(1, 1), (31, 2), (32, 3), (33, 8), (64, 9), (65, 1), (200, 5), (609, 8), (777, 17)])
+def test_triangular_solve_edges(N, nrhs):
+    """Blocks of 32 rows, columns in groups of eight, more blocks than CTAs of
+    a group.  The solve applies the inverses of the diagonal blocks, so its
+    backward error is N u |L| |U| |x| times the blocks' condition, componentwise
+    || |D^-1| |D| ||."""
+    from gbem._lib import lib
+    rng = np.random.default_rng(N + nrhs)
+    A = rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))
+    B = rng.standard_normal((N, nrhs)) + 1j * rng.standard_normal((N, nrhs))
+    LU, piv = _factor(A)
+    X = np.asfortranarray(B.copy())
+    ipiv = (piv + 1).astype(np.int32)
+    assert lib().gbem_lu_solve_host(LU.ctypes.data, N, N, ipiv.ctypes.data, b"N", nrhs, X.ctypes.data, N) == 0
+    L, R = np.tril(LU, -1) + np.eye(N), np.triu(LU)
+    cond = 1.0
+    for k in range(0, N, 32):
+        for D in (L[k:k + 32, k:k + 32], R[k:k + 32, k:k + 32]):
+            cond = max(cond, (np.abs(np.linalg.inv(D)) @ np.abs(D)).sum(axis=1).max())
+    bound = 16 * N * U * cond * (np.abs(L) @ (np.abs(R) @ np.abs(X))).max(axis=0)
+    assert (np.abs(A @ X - B).max(axis=0) <= bound).all()

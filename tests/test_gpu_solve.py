@@ -215,3 +215,17 @@ def test_mixed_solve_with_odd_n():
     assert res <= 1e-10
     X64 = sl.solve(G.AssembleBEMMatrix(w).numpy(), B)
     assert np.abs(X - X64).max() / np.abs(X64).max() < 1e-5
+
+
+def test_mixed_solve_beyond_the_l2():
+    """N = 15360, five right-hand sides: the complex-FP32 triangular solves take
+    two columns at a time there, the last one by itself.  The residual that
+    solve_mixed returns is the FP64 one of the worst column."""
+    from gbem import RWGGeometry, mesh
+    from gbem.api import Material
+    V, P = mesh.icosphere(4)
+    G = RWGGeometry([{"V": V, "P": P, "material": Material(2.25 + 0.01j)}])
+    rng = np.random.default_rng(2)
+    B = rng.standard_normal((G.TotalBFs, 5)) + 1j * rng.standard_normal((G.TotalBFs, 5))
+    X, it, res = G.solve_mixed(2.0, B, tol=1e-10, max_iter=12)
+    assert res <= 1e-10 and np.isfinite(X).all()
