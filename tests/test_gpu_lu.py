@@ -202,3 +202,29 @@ def test_complex64_leaf_edges(N):
     assert np.abs(L).max() <= np.sqrt(2.0) * (1 + 1e-5)
     if N <= 65:
         assert np.array_equal(M.ipiv - 1, sl.lu_factor(A)[1])
+
+
+@pytest.mark.parametrize("N", [80, 95, 96, 97, 112, 127, 128, 161, 224, 255, 300])
+def test_complex64_panel_edges(N):
+    """C64 LU where the last leaf of a 32- or 64-row block also solves the
+    block row, and the panel's updates end in ragged tiles: FP32 throughout up
+    to one 128-column panel, so the backward error is within 4 N 2^-24 of
+    |L||U|; a second panel has split-BF16 updates (2^-16 per product)."""
+    from gbem import C64
+    from gbem.api import HMatrix
+    M = HMatrix(_strip(N), C64)
+    rng = np.random.default_rng(N)
+    A = (rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))).astype(np.complex64)
+    M.set(A)
+    assert M.LUFactorize() == 0
+    LU = M.numpy().astype(np.complex128)
+    L, U = np.tril(LU, -1) + np.eye(N), np.triu(LU)
+    perm = np.arange(N)
+    for i, p in enumerate(M.ipiv - 1):
+        perm[[i, p]] = perm[[p, i]]
+    u = 2.0 ** -24 if N <= 128 else 2.0 ** -16
+    err = np.abs(A.astype(np.complex128)[perm] - L @ U)
+    assert (err <= 4 * N * u * (np.abs(L) @ np.abs(U))).all()
+    b = rng.standard_normal(N) + 1j * rng.standard_normal(N)
+    x = M.LUSolve(b.astype(np.complex64)).astype(np.complex128)
+    assert np.linalg.norm(A.astype(np.complex128) @ x - b) / (np.linalg.norm(A, 2) * np.linalg.norm(x)) < 1e-3
