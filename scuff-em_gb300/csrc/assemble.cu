@@ -2254,11 +2254,14 @@ gbem_status rhs_planewave_device(Geometry* g, double wr, double wi, const double
 //  vjp_far_kernel   far pairs (rRel > 4), one thread per pair: reverse-mode
 //                   derivative of the 6x6-rule integrals (adjoint.cuh), the
 //                   edge-length factors La Lb included.
-//  vjp_near_kernel  near and common-vertex pairs, one warp per (pair,
-//                   vertex, coordinate) -- one vertex per pair follows from
-//                   translation invariance: central differences of the FP64
-//                   near-pair evaluation (static integrals recomputed for the
-//                   displaced vertices), contracted with the same weights.
+//  vjp_pair_kernel  near and touching pairs in the desingularised branch, one
+//                   CTA per pair, a lane per displaced evaluation: central
+//                   differences of the FP64 near-pair value (static integrals
+//                   recomputed for the displaced vertices), contracted with the
+//                   same weights; one vertex per pair follows from translation
+//                   invariance.
+//  vjp_near_kernel  the same for self pairs and the short-wavelength branches,
+//                   one warp per (pair, vertex, coordinate).
 //  rhs_vjp_kernel   Re sum conj(g_i) db_i/dV for plane-wave right-hand sides.
 // ---------------------------------------------------------------------------
 struct VjpTables {
@@ -2486,6 +2489,13 @@ struct VjpNearArgs {
   double rel_step;  // displacement = rel_step * the pair's larger panel radius
 };
 
+// whether every region takes the desingularised branch for this pair
+__device__ __forceinline__ bool pair_desing(const DevNear& d, const RegionArgs& ra) {
+  for (int r = 0; r < ra.nreg; r++)
+    if (hypot(ra.k[r].re * d.rmax, ra.k[r].im * d.rmax) > M_PI) return false;
+  return true;
+}
+
 __global__ void __launch_bounds__(128) vjp_near_kernel(VjpNearArgs a, RegionArgs ra) {
   // 15 warps per pair: vertices 1..5 of the pair's six slots (panel a's
   // vertex 0 follows from the others) x 3 coordinates; each warp evaluates
@@ -2504,6 +2514,7 @@ __global__ void __launch_bounds__(128) vjp_near_kernel(VjpNearArgs a, RegionArgs
   const VjpTables& t = a.t;
   const DevNear d = a.near[pair];
   const bool self = d.pa == d.pb;
+  if (!self && pair_desing(d, ra)) return;  // vjp_pair_kernel's
   // a pair's value does not change when both panels move together, so the
   // derivative for panel a's vertex 0 is minus the sum of the others': that
   // vertex is not displaced, each other direction subtracts its share from it
@@ -2542,6 +2553,328 @@ __global__ void __launch_bounds__(128) vjp_near_kernel(VjpNearArgs a, RegionArgs
   if (lane == 0) {
     atomicAdd(&t.grad[3 * (size_t)gv + c], dE);
     atomicAdd(&t.grad[3 * (size_t)g0 + c], -dE);
+  }
+}
+
+// Re sum_m C0 H0 + C1 H1 as a linear functional of a pair's integrals: real
+// weights of the static ones (their sums over the regions) and of the constant
+// part, complex ones of each region's desingularised moments
+struct PairFunctional {
+  double RM1[9], R1[9], R2[9], XM[3], XX[3], c;
+};
+
+// coefficients of the moments of one region (vec_combine, summed over (Qa, Qb)
+// with C0, C1): with c = sum C, qa = sum C alpha, qb = sum C beta, X = sum C1
+// alpha x beta and Q = sum C1 (D0 - alpha + beta)
+__device__ __forceinline__ void pair_functional(const PairGeom<double>& g, cx<double> k, const cx<double>* C0,
+                                                const cx<double>* C1, cx<double>* gG, cx<double>* gP, PairFunctional& f) {
+  const cx<double> m4ok2 = cdiv(mk(-4.0, 0.0), k * k);
+  const double* ea[2] = {g.Aa, g.Ba};
+  const double* eb[2] = {g.Ab, g.Bb};
+  const cx<double> zero = mk(0.0, 0.0);
+  cx<double> c0 = zero, c1 = zero;
+#pragma unroll
+  for (int m = 0; m < 9; m++) { c0 = c0 + C0[m]; c1 = c1 + C1[m]; }
+  cx<double> qa0[3], qb0[3], qa1[3], qb1[3], X[3], Q[3], qq = zero;
+  const cx<double> ra0[2] = {C0[3] + C0[4] + C0[5], C0[6] + C0[7] + C0[8]}, ra1[2] = {C1[3] + C1[4] + C1[5], C1[6] + C1[7] + C1[8]};
+  const cx<double> rb0[2] = {C0[1] + C0[4] + C0[7], C0[2] + C0[5] + C0[8]}, rb1[2] = {C1[1] + C1[4] + C1[7], C1[2] + C1[5] + C1[8]};
+#pragma unroll
+  for (int c = 0; c < 3; c++) {  // alpha_j = -(edge j) of panel a, beta_j of b; zero for j = 0
+    qa0[c] = zero - g.Aa[c] * ra0[0] - g.Ba[c] * ra0[1];
+    qa1[c] = zero - g.Aa[c] * ra1[0] - g.Ba[c] * ra1[1];
+    qb0[c] = zero - g.Ab[c] * rb0[0] - g.Bb[c] * rb0[1];
+    qb1[c] = zero - g.Ab[c] * rb1[0] - g.Bb[c] * rb1[1];
+    X[c] = zero;
+    Q[c] = g.D0[c] * c1 - qa1[c] + qb1[c];
+  }
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const int m = 3 * (i + 1) + j + 1;
+      double cr[3];
+      vcross(ea[i], eb[j], cr);
+      const double dot = vdot(ea[i], eb[j]);
+      qq = qq + dot * C0[m];
+      gG[m] = dot * c0;
+      gP[m] = cr[0] * Q[0] + cr[1] * Q[1] + cr[2] * Q[2];
+#pragma unroll
+      for (int c = 0; c < 3; c++) X[c] = X[c] + cr[c] * C1[m];
+    }
+  cx<double> bD[3], aD[3];  // qb1 x D0, qa1 x D0
+  cvcross(qb1, g.D0, bD);
+  cvcross(qa1, g.D0, aD);
+  gG[0] = qq + m4ok2 * c0;
+  gP[0] = rcdot(g.D0, X);
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    cx<double> ub = zero, ua = zero, pu = zero, pv = zero;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      ub = ub + ea[i][c] * qb0[c];
+      ua = ua + eb[i][c] * qa0[c];
+      pu = pu + ea[i][c] * (bD[c] + X[c]);
+      pv = pv - eb[i][c] * (aD[c] + X[c]);
+    }
+    gG[3 * (i + 1)] = ub;
+    gG[i + 1] = ua;
+    gP[3 * (i + 1)] = pu;
+    gP[i + 1] = pv;
+  }
+  // the static terms (add_taylor_terms, htimes_rm3)
+  const double inv4pi = 0.079577471545947667884;
+  const double R0[9] = {1.0 / 4, 1.0 / 12, 1.0 / 12, 1.0 / 12, 1.0 / 36, 1.0 / 36, 1.0 / 12, 1.0 / 36, 1.0 / 36};
+  const cx<double> ik = mk(-k.im, k.re), p1 = inv4pi * ik, p2 = p1 * ik, p3 = p2 * ik, p4 = p3 * ik;
+  auto re = [](cx<double> a, cx<double> b) { return a.re * b.re - a.im * b.im; };
+#pragma unroll
+  for (int m = 0; m < 9; m++) {
+    f.RM1[m] += inv4pi * gG[m].re + 0.5 * re(gP[m], p2);
+    f.R1[m] += 0.5 * re(gG[m], p2) + re(gP[m], p4) * (1.0 / 6.0);
+    f.R2[m] += re(gG[m], p3) * (1.0 / 6.0);
+    f.c += R0[m] * (re(gG[m], p1) + re(gP[m], p3) * (1.0 / 3.0));
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    f.XX[c] -= inv4pi * Q[c].re;
+    f.XM[c] -= inv4pi * (aD[c] + X[c]).re;
+  }
+}
+
+// One point of a non-touching pair's static integrals (fippi_far_acc),
+// contracted: bb[p] = the b-side weights of r^-1, r, r^2 at the point's a side
+__device__ __forceinline__ double fippi_far_dot(const double* Xo, const double* Ap, const double* Bp, const double* dV,
+                                                double a2, double ia, double up, const double (*bb)[3],
+                                                const PairFunctional& f) {
+  double Zo[3], Y[3];
+#pragma unroll
+  for (int m = 0; m < 3; m++) {
+    Zo[m] = dV[m] + up * Ap[m];
+    Y[m] = Xo[m] - Zo[m];
+  }
+  const double ia2 = ia * ia;
+  const double v0 = vdot(Bp, Y) * ia2;
+  double b2 = vdot(Y, Y) * ia2 - v0 * v0;
+  if (b2 < 0) b2 = 0;
+  double J[4][2], q[3];
+  seg_integrals(a2, ia, v0, b2, up, J);
+#pragma unroll
+  for (int m = 0; m < 3; m++) q[m] = Zo[m] * J[0][0] + Bp[m] * J[0][1];
+  double e = 0.0;
+#pragma unroll
+  for (int m = 0; m < 3; m++) {
+    const int m1 = (m + 1) % 3, m2 = (m + 2) % 3;
+    e += f.XM[m] * (Xo[m] * J[0][0] - q[m]) + f.XX[m] * (Xo[m1] * q[m2] - Xo[m2] * q[m1]);
+  }
+#pragma unroll
+  for (int p = 0; p < 3; p++) e += J[p + 1][0] * (bb[p][0] + up * bb[p][1]) + J[p + 1][1] * (bb[p][2] - bb[p][1]);
+  return e;
+}
+
+// What a Duffy point brings to every evaluation of a touching pair (all of it
+// independent of the vertices' positions): the monomials' radial integrals for
+// r^-1, r and r^2, the barycentric slopes of D = (x - x') / w, the vector of
+// the XX integral in panel a's edges, and the weights of XM and XX
+constexpr int TOUCH_PT = 35;
+__device__ __forceinline__ void touch_point(const int* pa, const int* pb, const DuffyPt& pt, double* o, int stride) {
+  const double o2 = pt.om.c[2], o3 = pt.om.c[3];
+  rpoly ua, va, ub, vb;
+  tcr_from_edge(pa, pt.sa0, pt.sa1, &ua, &va);
+  tcr_from_edge(pb, pt.sb0, pt.sb1, &ub, &vb);
+  const double a0[3] = {1.0, ua.c[0], va.c[0]}, a1[3] = {0.0, ua.c[1], va.c[1]};
+  const double b0[3] = {1.0, ub.c[0], vb.c[0]}, b1[3] = {0.0, ub.c[1], vb.c[1]};
+  constexpr double inv[9] = {0.0, 1.0, 1.0 / 2, 1.0 / 3, 1.0 / 4, 1.0 / 5, 1.0 / 6, 1.0 / 7, 1.0 / 8};
+  auto h = [&](int e) { return pt.W * (o2 * inv[e + 2] + o3 * inv[e + 3]); };
+#pragma unroll
+  for (int p = 0; p < 3; p++) {
+    const int e0 = p == 0 ? 0 : p + 1;
+    const double p0 = h(e0), p1 = h(e0 + 1), p2 = h(e0 + 2);
+    const double g0[3] = {p0, b0[1] * p0 + b1[1] * p1, b0[2] * p0 + b1[2] * p1};
+    const double g1[3] = {p1, b0[1] * p1 + b1[1] * p2, b0[2] * p1 + b1[2] * p2};
+#pragma unroll
+    for (int al = 0; al < 3; al++)
+#pragma unroll
+      for (int be = 0; be < 3; be++) o[(9 * p + 3 * al + be) * stride] = al ? a0[al] * g0[be] + a1[al] * g1[be] : g0[be];
+  }
+  const double om2 = o2 + 0.5 * o3, g1 = 0.5 * o2 + o3 / 3.0;
+  o[27 * stride] = ua.c[1]; o[28 * stride] = va.c[1]; o[29 * stride] = ub.c[1]; o[30 * stride] = vb.c[1];
+  o[31 * stride] = om2 * ua.c[0] + g1 * ua.c[1];
+  o[32 * stride] = om2 * va.c[0] + g1 * va.c[1];
+  o[33 * stride] = pt.W * om2;
+  o[34 * stride] = pt.W;
+}
+
+// The adjoint of a near or touching pair, one CTA per pair, where every region
+// is desingularised: a lane per displaced evaluation (15 directions, both
+// signs), the points dealt to the warps.  A lane first contracts the weights
+// with its displaced geometry (pair_functional), so a point costs it one
+// number: no moments to accumulate, none to sum over a warp (525 additions of
+// the 7100 FP64 operations of an evaluation), and what a point brings without
+// the positions is computed once for all evaluations.  The FP64 pipe bounds it:
+// the near pairs of the N = 960 sphere 77.5 -> 40 ms.
+__global__ void __launch_bounds__(128) vjp_pair_kernel(VjpNearArgs a, RegionArgs ra) {
+  __shared__ double sgx[N_FIP_ADJ], sgw[N_FIP_ADJ], srule6[18];
+  __shared__ cx<double> W[3][9];
+  __shared__ double sE[4][32];
+  __shared__ double spt[4][TOUCH_PT][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const DevNear d = a.near[blockIdx.x];
+  if (d.pa == d.pb || !pair_desing(d, ra)) return;
+  const VjpTables& t = a.t;
+  if (tid < N_FIP_ADJ) { sgx[tid] = c_gx8[tid]; sgw[tid] = c_gw8[tid]; }
+  if (tid < 18) srule6[tid] = c_lo64[tid];
+  if (tid < 9) {
+    cx<double> w3[3];
+    vjp_weights_m(t, d.pa, d.pb, a.bpe_a, a.bpe_b, true, tid, w3);
+    W[0][tid] = w3[0]; W[1][tid] = w3[1]; W[2][tid] = w3[2];
+  }
+  __syncthreads();
+  // this lane's evaluation (see vjp_near_kernel for the directions left out)
+  const int dir = min(lane >> 1, 14), v = 1 + dir / 3, c = dir % 3;
+  const int gv = v < 3 ? t.pvi[3 * d.pa + v] : t.pvi[3 * d.pb + v - 3], g0 = t.pvi[3 * d.pa];
+  bool live = lane < 30 && gv != g0;
+  if (v >= 3)
+    for (int q = 0; q < 3; q++) live = live && t.pvi[3 * d.pa + q] != gv;
+  const double step = a.rel_step * d.rmax, dv = lane & 1 ? -step : step;
+  // a sample's difference between the two signs (neighbouring lanes) before it
+  // is summed: the sums then round at the difference's size, not the energy's
+  auto diff = [](double e) { return e - __shfl_xor_sync(0xffffffffu, e, 1); };
+  double E = 0.0;
+  PairGeom<double> g;
+  PairFunctional f;
+  double Va[9], Vb[9];
+#pragma unroll
+  for (int q = 0; q < 9; q++) { Va[q] = t.pv[9 * (size_t)d.pa + q]; Vb[q] = t.pv[9 * (size_t)d.pb + q]; }
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const double da = t.pvi[3 * d.pa + q] == gv ? dv : 0.0, db = t.pvi[3 * d.pb + q] == gv ? dv : 0.0;
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+      if (e == c) { Va[3 * q + e] += da; Vb[3 * q + e] += db; }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 3; e++) {
+    g.D0[e] = Va[e] - Vb[e];
+    g.Aa[e] = Va[3 + e] - Va[e]; g.Ba[e] = Va[6 + e] - Va[e];
+    g.Ab[e] = Vb[3 + e] - Vb[e]; g.Bb[e] = Vb[6 + e] - Vb[e];
+  }
+  {
+    double la[3], lb[3];  // signed lengths of the edges opposite the Q's
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      double x = 0.0, y = 0.0;
+#pragma unroll
+      for (int e = 0; e < 3; e++) {
+        const double ea = Va[3 * ((q + 1) % 3) + e] - Va[3 * ((q + 2) % 3) + e];
+        const double eb = Vb[3 * ((q + 1) % 3) + e] - Vb[3 * ((q + 2) % 3) + e];
+        x += ea * ea; y += eb * eb;
+      }
+      la[q] = t.sbf[3 * d.pa + q] >= 0 ? (t.ssl[3 * d.pa + q] > 0.0 ? sqrt(x) : -sqrt(x)) : 0.0;
+      lb[q] = t.sbf[3 * d.pb + q] >= 0 ? (t.ssl[3 * d.pb + q] > 0.0 ? sqrt(y) : -sqrt(y)) : 0.0;
+    }
+#pragma unroll
+    for (int m = 0; m < 9; m++) f.RM1[m] = f.R1[m] = f.R2[m] = 0.0;
+    f.c = 0.0;
+#pragma unroll
+    for (int e = 0; e < 3; e++) f.XM[e] = f.XX[e] = 0.0;
+    for (int r = 0; r < ra.nreg; r++) {
+      const cx<double> k = ra.k[r];
+      if (k.re == 0.0 && k.im == 0.0) continue;
+      cx<double> C0[9], C1[9], gG[9], gP[9];
+#pragma unroll
+      for (int m = 0; m < 9; m++) {
+        const double fac = la[m / 3] * lb[m % 3];
+        C0[m] = fac * (ra.pf1[r] * W[0][m] + ra.pf3[r] * W[2][m]);
+        C1[m] = fac * (ra.pfc[r] * W[1][m]);
+      }
+      pair_functional(g, k, C0, C1, gG, gP, f);
+      // the desingularised part at this warp's nine samples
+#pragma unroll 1
+      for (int q = 9 * warp; q < 9 * warp + 9; q++) {
+        const int i = q / 6, j = q % 6;
+        const double u = srule6[3 * i], vv = srule6[3 * i + 1], up = srule6[3 * j], vp = srule6[3 * j + 1];
+        double r2 = 0.0;
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+          const double R = g.D0[e] + u * g.Aa[e] + vv * g.Ba[e] - up * g.Ab[e] - vp * g.Bb[e];
+          r2 += R * R;
+        }
+        cx<double> phi, psi;
+        desing_pp(r2, k, srule6[3 * i + 2] * srule6[3 * j + 2], &phi, &psi);
+        cx<double> T0 = mk(0.0, 0.0), T1 = T0;
+        const double ma[3] = {1.0, u, vv};
+#pragma unroll
+        for (int al = 0; al < 3; al++) {
+          T0 = T0 + ma[al] * (gG[3 * al] + up * gG[3 * al + 1] + vp * gG[3 * al + 2]);
+          T1 = T1 + ma[al] * (gP[3 * al] + up * gP[3 * al + 1] + vp * gP[3 * al + 2]);
+        }
+        E += diff((phi * T0 + psi * T1).re);
+      }
+    }
+  }
+  if (warp == 0) E += diff(f.c);
+  if (d.ncv == 0) {
+    double B[3], Bp[3], dV[3];
+#pragma unroll
+    for (int e = 0; e < 3; e++) { B[e] = g.Ba[e] - g.Aa[e]; Bp[e] = g.Bb[e] - g.Ab[e]; dV[e] = -g.D0[e]; }
+    const double a2 = vdot(Bp, Bp), ia = 1.0 / sqrt(a2);
+#pragma unroll 1
+    for (int q = 16 * warp; q < 16 * warp + 16; q++) {
+      const int i1 = q / N_FIP_ADJ, j = q % N_FIP_ADJ;
+      const double u = sgx[i1], vv = u * sgx[j], wu = sgw[i1] * sgw[j] * u;
+      double Xo[3], bb[3][3];
+#pragma unroll
+      for (int e = 0; e < 3; e++) {
+        Xo[e] = u * g.Aa[e] + vv * B[e];
+        bb[0][e] = f.RM1[e] + (u - vv) * f.RM1[3 + e] + vv * f.RM1[6 + e];
+        bb[1][e] = f.R1[e] + (u - vv) * f.R1[3 + e] + vv * f.R1[6 + e];
+        bb[2][e] = f.R2[e] + (u - vv) * f.R2[3 + e] + vv * f.R2[6 + e];
+      }
+#pragma unroll 1
+      for (int l = 0; l < N_FIP_ADJ; l++) E += diff((wu * sgw[l]) * fippi_far_dot(Xo, g.Ab, Bp, dV, a2, ia, sgx[l], bb, f));
+    }
+  } else {
+    const int np = duffy_npts(d.ncv, N_FIP_ADJ) / 4;  // this warp's
+    for (int q0 = np * warp; q0 < np * (warp + 1); q0 += 32) {
+      {
+        DuffyPt pt;
+        duffy_pt(d.ncv, q0 + lane, sgx, sgw, N_FIP_ADJ, pt);
+        touch_point(d.perm_a, d.perm_b, pt, &spt[warp][0][lane], 32);
+      }
+      __syncwarp();
+#pragma unroll 1
+      for (int p = 0; p < 32; p++) {
+        auto o = [&](int q) { return spt[warp][q][p]; };
+        double D[3], x[3];
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+          D[e] = o(27) * g.Aa[e] + o(28) * g.Ba[e] - o(29) * g.Ab[e] - o(30) * g.Bb[e];
+          x[e] = o(31) * g.Aa[e] + o(32) * g.Ba[e];
+        }
+        const double X2 = vdot(D, D), iX = rsqrt_d(X2), iX3 = iX * iX * iX;
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, sx = 0.0, sm = 0.0;
+#pragma unroll
+        for (int m = 0; m < 9; m++) { s0 += o(m) * f.RM1[m]; s1 += o(9 + m) * f.R1[m]; s2 += o(18 + m) * f.R2[m]; }
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+          const int e1 = (e + 1) % 3, e2 = (e + 2) % 3;
+          sm += f.XM[e] * D[e];
+          sx += f.XX[e] * (x[e1] * D[e2] - x[e2] * D[e1]);
+        }
+        E += diff(s0 * iX + s1 * (X2 * iX) + s2 * X2 + iX3 * (o(33) * sm - o(34) * sx));
+      }
+      __syncwarp();
+    }
+  }
+  sE[warp][lane] = E;
+  __syncthreads();
+  if (warp == 0) {
+    E = (sE[0][lane] + sE[1][lane]) + (sE[2][lane] + sE[3][lane]);
+    const double dE = E / (2.0 * step);
+    if (live && !(lane & 1)) {
+      atomicAdd(&t.grad[3 * (size_t)gv + c], dE);
+      atomicAdd(&t.grad[3 * (size_t)g0 + c], -dE);
+    }
   }
 }
 
@@ -2687,7 +3020,8 @@ gbem_status vertex_vjp_device(Geometry* g, double wr, double wi, const double* e
       na.rel_step = rel_step;
       const long long n = 15LL * 32 * db->nnear;  // one warp per (pair, displaced coordinate)
       vjp_near_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(na, ra);
-      stats_launch(ST_OTHER);
+      vjp_pair_kernel<<<(unsigned)db->nnear, 128, 0, s>>>(na, ra);
+      stats_launch(ST_OTHER, 2);
     }
     e = cudaGetLastError();
   }
