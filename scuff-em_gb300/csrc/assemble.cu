@@ -1100,8 +1100,8 @@ __global__ void __launch_bounds__(256) stamp_kernel(StampArgs sp) {
 // combinations of all nine (Qa, Qb) from eight scalars of the pair (h0_all,
 // h1_all), 180 operations from 2100; real arithmetic where the wavenumber is
 // imaginary (REALK); pairs below the diagonal skipped.  Measured against the
-// tile kernel: dielectric sphere, N = 3840, 36.7 -> 10.2 ms; PEC sphere, N =
-// 480, 1.13 -> 0.32; rounded cube, N = 6084, 97.1 -> 26.1.
+// tile kernel: dielectric sphere, N = 3840, 36.7 -> 9.4 ms; PEC sphere, N =
+// 480, 1.13 -> 0.32; rounded cube, N = 6084, 97.1 -> 24.4.
 // ---------------------------------------------------------------------------
 constexpr double PI64_HI = 0x1.921fb54400000p-5;  // pi/64, leading 33 bits
 constexpr double PI64_LO = 0x1.0b4611a626331p-39;
@@ -1132,25 +1132,43 @@ __device__ __forceinline__ void expi64(double x, const SinCosTab64& tab, double*
 // KIND 0: k real, 1: any k, 2: k imaginary (G and Psi real, E = double).
 // pa0/A/B: the row panel's V0 - V0 of the column panel and edges; ob: the
 // column panel's node offsets u' Ab + v' Bb; w4: the rule's weights over 4 pi.
-template <int KIND, typename E>
+// keep: where the first of two regions (SHARE = 1) leaves 1/r and r of the 36
+// samples for the second (2), 14 of whose operations per sample they are:
+// dielectric sphere, N = 3840, 9.85 -> 9.1 ms.
+constexpr int PP64_COLS = 8, PP64_SLOTS = 32 + PP64_COLS, PP64_THREADS = 32 * PP64_COLS;
+constexpr size_t PP64_KEEP = (size_t)36 * PP64_THREADS * sizeof(double2);
+
+template <int KIND, int SHARE, typename E>
 __device__ __forceinline__ void moments64(const double* D0, const double* A, const double* B, const double* ob, double kre,
-                                          double kim, const double* w4, const SinCosTab64& tab, E* MG, E* MP) {
+                                          double kim, const double* w4, const SinCosTab64& tab, double2* keep, E* MG,
+                                          E* MP) {
 #pragma unroll
   for (int m = 0; m < 9; m++) MG[m] = MP[m] = E{};
 #pragma unroll 1
   for (int i = 0; i < 6; i++) {
     const double u = c_lo64[3 * i], v = c_lo64[3 * i + 1], wi = c_lo64[3 * i + 2];
     double pa[3];
+    if (SHARE != 2) {
 #pragma unroll
-    for (int c = 0; c < 3; c++) pa[c] = fma(v, B[c], fma(u, A[c], D0[c]));
+      for (int c = 0; c < 3; c++) pa[c] = fma(v, B[c], fma(u, A[c], D0[c]));
+    }
     E SG[3], SP[3];
 #pragma unroll
     for (int b = 0; b < 3; b++) SG[b] = SP[b] = E{};
 #pragma unroll 2
     for (int j = 0; j < 6; j++) {
-      const double x = pa[0] - ob[3 * j], y = pa[1] - ob[3 * j + 1], z = pa[2] - ob[3 * j + 2];
-      const double r2 = fma(z, z, fma(y, y, x * x));
-      const double rinv = rsqrt(r2), r = r2 * rinv;
+      double rinv, r;
+      if (SHARE == 2) {
+        const double2 z = keep[(6 * i + j) * PP64_THREADS];
+        rinv = z.x;
+        r = z.y;
+      } else {
+        const double x = pa[0] - ob[3 * j], y = pa[1] - ob[3 * j + 1], z = pa[2] - ob[3 * j + 2];
+        const double r2 = fma(z, z, fma(y, y, x * x));
+        rinv = rsqrt(r2);
+        r = r2 * rinv;
+        if (SHARE == 1) keep[(6 * i + j) * PP64_THREADS] = make_double2(rinv, r);
+      }
       const double up = c_lo64[3 * j], vp = c_lo64[3 * j + 1];
       double amp = w4[j] * rinv;
       if (KIND != 0) amp *= exp(-kim * r);
@@ -1190,12 +1208,11 @@ struct PPair64Args {
   int nrow, ncp, sym;
   double2* out;       // [NC][9][ncp][nrow]; x = NaN: a near pair
 };
-constexpr int PP64_COLS = 8, PP64_SLOTS = 32 + PP64_COLS, PP64_THREADS = 32 * PP64_COLS;
-
 __device__ __forceinline__ cx<double> scaled(cx<double> f, cx<double> h) { return f * h; }
 __device__ __forceinline__ cx<double> scaled(cx<double> f, double h) { return h * f; }
 
-template <int NC, bool REALK>
+// TWO: both regions' wavenumbers may be nonzero (PP64_KEEP bytes of dynamic shared memory)
+template <int NC, bool REALK, bool TWO>
 __global__ void __launch_bounds__(PP64_THREADS, 1) ppair64_kernel(PPair64Args p, RegionArgs ra) {
   using E = typename std::conditional<REALK, double, cx<double>>::type;
   __shared__ double s_pv[PP64_SLOTS][9];
@@ -1204,7 +1221,9 @@ __global__ void __launch_bounds__(PP64_THREADS, 1) ppair64_kernel(PPair64Args p,
   __shared__ float s_cf[PP64_SLOTS][4];
   __shared__ SinCosTab64 s_tab;
   __shared__ double s_w4[6];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.y * 32 + threadIdx.x;
+  double2* keep = reinterpret_cast<double2*>(smem_raw) + tid;
   const int r0 = blockIdx.x * 32, c0 = blockIdx.y * PP64_COLS;
   auto panel_of = [&](int sl) -> int {
     if (sl < 32) return r0 + sl < p.nrow ? p.offa + r0 + sl : -1;
@@ -1254,12 +1273,18 @@ __global__ void __launch_bounds__(PP64_THREADS, 1) ppair64_kernel(PPair64Args p,
     const cx<double> k = ra.k[r];
     if (k.re == 0.0 && k.im == 0.0) continue;
     E MG[9], MP[9];
-    if constexpr (REALK) {
-      moments64<2>(g.D0, g.Aa, g.Ba, s_ob[threadIdx.y], 0.0, k.im, s_w4, s_tab, MG, MP);
-    } else {
-      if (k.im == 0.0) moments64<0>(g.D0, g.Aa, g.Ba, s_ob[threadIdx.y], k.re, 0.0, s_w4, s_tab, MG, MP);
-      else moments64<1>(g.D0, g.Aa, g.Ba, s_ob[threadIdx.y], k.re, k.im, s_w4, s_tab, MG, MP);
-    }
+    auto moments = [&](auto share) {
+      constexpr int SH = decltype(share)::value;
+      if constexpr (REALK) {
+        moments64<2, SH>(g.D0, g.Aa, g.Ba, s_ob[threadIdx.y], 0.0, k.im, s_w4, s_tab, keep, MG, MP);
+      } else {
+        if (k.im == 0.0) moments64<0, SH>(g.D0, g.Aa, g.Ba, s_ob[threadIdx.y], k.re, 0.0, s_w4, s_tab, keep, MG, MP);
+        else moments64<1, SH>(g.D0, g.Aa, g.Ba, s_ob[threadIdx.y], k.re, k.im, s_w4, s_tab, keep, MG, MP);
+      }
+    };
+    if constexpr (!TWO) moments(std::integral_constant<int, 0>());
+    else if (first) moments(std::integral_constant<int, 1>());
+    else moments(std::integral_constant<int, 2>());
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       g.Ab[c] = s_pv[ib][3 + c] - s_pv[ib][c]; g.Bb[c] = s_pv[ib][6 + c] - s_pv[ib][c];
@@ -1425,8 +1450,17 @@ static cudaError_t far_fp64(Geometry* g, const Block& b, DevBlock* db, const Til
     pp.offa = g->S[b.sa].panel_offset; pp.offb = g->S[b.sb].panel_offset;
     pp.nrow = st.nrow; pp.ncp = st.ncp; pp.sym = b.sym; pp.out = (double2*)g->ppv;
     const dim3 grid((st.nrow + 31) / 32, (st.ncp + PP64_COLS - 1) / PP64_COLS), block(32, PP64_COLS);
-    if (realk) ppair64_kernel<NC, true><<<grid, block, 0, s>>>(pp, ra);
-    else ppair64_kernel<NC, false><<<grid, block, 0, s>>>(pp, ra);
+    auto launch = [&](auto rk) {
+      constexpr bool RK = decltype(rk)::value;
+      if (ra.nreg < 2) {
+        ppair64_kernel<NC, RK, false><<<grid, block, 0, s>>>(pp, ra);
+      } else if ((e = allow_max_smem(ppair64_kernel<NC, RK, true>)) == cudaSuccess) {
+        ppair64_kernel<NC, RK, true><<<grid, block, PP64_KEEP, s>>>(pp, ra);
+      }
+    };
+    if (realk) launch(std::true_type());
+    else launch(std::false_type());
+    if (e != cudaSuccess) return e;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     Stamp64Args sp;
     sp.ta = ta; sp.tiles = st.tiles; sp.edge_a = db->edge_a; sp.edge_b = db->edge_b; sp.ecol = db->ecol;
