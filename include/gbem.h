@@ -187,6 +187,14 @@ gbem_status gbem_lu_solve(gbem_matrix *M, char trans, int nrhs, void *B, int ldb
 gbem_status gbem_lu_trace(gbem_matrix *M, const gbem_matrix *B, int ncols, double *trace);
 gbem_status gbem_lu_trace_host(gbem_matrix *M, const void *B, int ldb, int ncols, double *trace);
 
+/* The same trace for the rigid displacement of the first surface along axis
+ * (0, 1, 2), over that surface's basis functions: B holds the transposes of
+ * the gradients of the blocks (0, s), s >= 1 (gbem_assemble_block_gradient),
+ * assembled and transposed on the device.  M factored, F64 or C128 (F64: an
+ * imaginary omega, as there). */
+gbem_status gbem_lu_trace_displacement(gbem_matrix *M, int axis, double omega_re, double omega_im,
+                                       const double *eps, const double *mu, double *trace);
+
 /* log|det M| of a factored M (gbem_lu_factor): the sum of log|U(n,n)| over
  * the diagonal of its LU factor, the quantity GetLNDetMInvMInf sums from the
  * factors of M and of its diagonal T blocks for the Casimir energy

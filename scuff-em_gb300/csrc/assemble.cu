@@ -1101,7 +1101,7 @@ __global__ void __launch_bounds__(256) stamp_kernel(StampArgs sp) {
 // h1_all), 180 operations from 2100; real arithmetic where the wavenumber is
 // imaginary (REALK); pairs below the diagonal skipped.  Measured against the
 // tile kernel: dielectric sphere, N = 3840, 36.7 -> 9.4 ms; PEC sphere, N =
-// 480, 1.13 -> 0.32; rounded cube, N = 6084, 97.1 -> 24.4.
+// 480, 1.13 -> 0.32; rounded cube, N = 6084, 97.1 -> 24.1.
 // ---------------------------------------------------------------------------
 constexpr double PI64_HI = 0x1.921fb54400000p-5;  // pi/64, leading 33 bits
 constexpr double PI64_LO = 0x1.0b4611a626331p-39;

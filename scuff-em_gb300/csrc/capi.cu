@@ -252,6 +252,18 @@ static __global__ void log_abs_diag(const T* A, long long ld, int n, int cplx, d
 
 }  // namespace gbem
 
+// out(j, i) = in(i, j): in m x n (ld m), out with leading dimension ldo
+template <typename E>
+__global__ void __launch_bounds__(256) transpose_block(const E* in, int m, int n, E* out, long long ldo) {
+  __shared__ E t[32][33];
+  const int i0 = 32 * blockIdx.x, j0 = 32 * blockIdx.y, x = threadIdx.x, y = threadIdx.y;
+  for (int k = y; k < 32; k += 8)
+    if (i0 + x < m && j0 + k < n) t[k][x] = in[i0 + x + (long long)(j0 + k) * m];
+  __syncthreads();
+  for (int k = y; k < 32; k += 8)
+    if (j0 + x < n && i0 + k < m) out[j0 + x + (long long)(i0 + k) * ldo] = t[x][k];
+}
+
 extern "C" {
 
 const char* gbem_last_error(void) { return g_err; }
@@ -904,6 +916,28 @@ gbem_status gbem_lu_solve(gbem_matrix* M, char trans, int nrhs, void* B, int ldb
   return st;
 }
 
+// trace of M^-1 X over the first ncols diagonal entries; X (device, N x ncols)
+// is overwritten
+static gbem_status trace_solved(gbem_matrix* M, void* X, int ncols, double* trace) {
+  const int N = M->N, dt = M->dtype;
+  cudaStream_t s = M->stream;
+  double* d_out = nullptr;
+  cudaError_t e = cudaMallocAsync((void**)&d_out, 2 * sizeof(double), s);
+  if (e != cudaSuccess) return cuda_status(e, "gbem_lu_trace setup");
+  gbem_status st = lu_solve_many_device(M->d, N, M->ld, dt, M->d_perm, ncols, X, N, s);
+  if (st == GBEM_OK) {
+    if (dt == GBEM_C64) trace_diag<<<1, 1024, 0, s>>>((const cx<float>*)X, N, ncols, d_out);
+    else if (dt == GBEM_F64) trace_diag<<<1, 1024, 0, s>>>((const double*)X, N, ncols, d_out);
+    else trace_diag<<<1, 1024, 0, s>>>((const cx<double>*)X, N, ncols, d_out);
+    stats_launch(ST_OTHER);
+    e = cudaMemcpyAsync(trace, d_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) st = cuda_status(e, "gbem_lu_trace");
+  }
+  cudaFreeAsync(d_out, s);
+  return st;
+}
+
 // Tr over the first ncols diagonal entries of M^-1 B (GetTraceMInvdM,
 // applications/scuff-cas3D/CasimirIntegrand.cc:100-146): B holds the
 // derivative blocks of the BEM matrix in its first ncols columns.
@@ -916,29 +950,54 @@ static gbem_status trace_impl(gbem_matrix* M, const void* B, int ldb, int ncols,
   CHECK_CUDA(cudaSetDevice(M->g->device), "cudaSetDevice");
   const int N = M->N;
   cudaStream_t s = M->stream;
-  const int dt = M->dtype;
-  const size_t es = esize(dt);
+  const size_t es = esize(M->dtype);
   void* X = nullptr;
-  double* d_out = nullptr;
-  gbem_status st = GBEM_OK;
   cudaError_t e = cudaMallocAsync(&X, (size_t)N * ncols * es, s);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_out, 2 * sizeof(double), s);
   if (e == cudaSuccess)
     e = cudaMemcpy2DAsync(X, (size_t)N * es, B, (size_t)ldb * es, (size_t)N * es, ncols,
                           host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s);
-  if (e != cudaSuccess) st = cuda_status(e, "gbem_lu_trace setup");
-  if (st == GBEM_OK) st = lu_solve_many_device(M->d, N, M->ld, dt, M->d_perm, ncols, X, N, s);
-  if (st == GBEM_OK) {
-    if (dt == GBEM_C64) trace_diag<<<1, 1024, 0, s>>>((const cx<float>*)X, N, ncols, d_out);
-    else if (dt == GBEM_F64) trace_diag<<<1, 1024, 0, s>>>((const double*)X, N, ncols, d_out);
-    else trace_diag<<<1, 1024, 0, s>>>((const cx<double>*)X, N, ncols, d_out);
-    stats_launch(ST_OTHER);
-    e = cudaMemcpyAsync(trace, d_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) st = cuda_status(e, "gbem_lu_trace");
-  }
+  gbem_status st = e == cudaSuccess ? trace_solved(M, X, ncols, trace) : cuda_status(e, "gbem_lu_trace setup");
   if (X) cudaFreeAsync(X, s);
-  if (d_out) cudaFreeAsync(d_out, s);
+  cudaStreamSynchronize(s);
+  return st;
+}
+
+gbem_status gbem_lu_trace_displacement(gbem_matrix* M, int axis, double omega_re, double omega_im, const double* eps,
+                                       const double* mu, double* trace) {
+  if (!M || !eps || !mu || !trace || axis < 0 || axis > 2 || (M->dtype != GBEM_F64 && M->dtype != GBEM_C128)) {
+    set_error("gbem_lu_trace_displacement: bad arguments (axis 0..2, dtype F64 or C128)");
+    return GBEM_EINVAL;
+  }
+  if (!M->factored) { set_error("gbem_lu_trace_displacement: matrix is not factored"); return GBEM_EINVAL; }
+  gbem_geometry* g = (gbem_geometry*)M->g;
+  gbem_status st = ensure_stream(g);
+  if (st != GBEM_OK) return st;
+  const int N = M->N, m = surface_bfs(g, 0), ns = (int)g->S.size();
+  const size_t es = esize(M->dtype);
+  cudaStream_t s = g->stream;
+  int nmax = 1;
+  for (int b = 1; b < ns; b++) nmax = std::max(nmax, surface_bfs(g, b));
+  void *X = nullptr, *T = nullptr;
+  cudaError_t e = cudaMallocAsync(&X, (size_t)N * m * es, s);
+  if (e == cudaSuccess) e = cudaMallocAsync(&T, (size_t)m * nmax * es, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(X, 0, (size_t)N * m * es, s);
+  st = cuda_status(e, "gbem_lu_trace_displacement setup");
+  for (int b = 1, off = m; b < ns && st == GBEM_OK; off += surface_bfs(g, b), b++) {
+    const int n = surface_bfs(g, b);
+    void* out[3] = {nullptr, nullptr, nullptr};
+    out[axis] = T;
+    st = gbem_assemble_block_gradient(g, 0, b, omega_re, omega_im, eps, mu, out[0], out[1], out[2], m, 0, 0, M->dtype);
+    if (st != GBEM_OK) break;
+    const dim3 grid((m + 31) / 32, (n + 31) / 32), block(32, 8);
+    if (M->dtype == GBEM_F64) transpose_block<<<grid, block, 0, s>>>((const double*)T, m, n, (double*)X + off, N);
+    else transpose_block<<<grid, block, 0, s>>>((const cx<double>*)T, m, n, (cx<double>*)X + off, N);
+    stats_launch(ST_OTHER);
+    st = cuda_status(cudaGetLastError(), "transpose_block");
+  }
+  if (st == GBEM_OK && s != M->stream) st = cuda_status(cudaStreamSynchronize(s), "gbem_lu_trace_displacement");
+  if (st == GBEM_OK) st = trace_solved(M, X, m, trace);
+  if (X) cudaFreeAsync(X, s);
+  if (T) cudaFreeAsync(T, s);
   cudaStreamSynchronize(s);
   return st;
 }

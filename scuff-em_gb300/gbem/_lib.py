@@ -30,7 +30,7 @@ EXPORTS = [
     "gbem_lu_trace", "gbem_lu_trace_host", "gbem_assemble_block_dmdt", "gbem_assemble_block_dmdt_host",
     "gbem_solve_mixed_batch", "gbem_vertex_vjp_matrix", "gbem_vertex_vjp_rhs_planewave",
     "gbem_geometry_num_vertices", "gbem_cache_preload", "gbem_cache_store", "gbem_cache_clear", "gbem_cache_size",
-    "gbem_cache_lookup_stats",
+    "gbem_cache_lookup_stats", "gbem_lu_trace_displacement",
 ]
 
 
@@ -92,7 +92,7 @@ def lib():
             "gbem_assemble_block_gradient": ([P, I, I, D, D, P, P, P, P, P, I, I, I, I], I),
             "gbem_assemble_block_gradient_host": ([P, I, I, D, D, P, P, P, P, P, I, I, I, I], I),
             "gbem_power_emt": ([P, D, D, P, P, I, I, P, I, P, I, P, P], I),
-            "gbem_lu_trace": ([P, P, I, P], I),
+            "gbem_lu_trace": ([P, P, I, P], I), "gbem_lu_trace_displacement": ([P, I, D, D, P, P, P], I),
             "gbem_solve_mixed_batch": ([I, P, I], I),
             "gbem_assemble_block_dmdt": ([P, I, I, D, D, P, P, I, P, P, I, I, I, I], I),
             "gbem_assemble_block_dmdt_host": ([P, I, I, D, D, P, P, I, P, P, I, I, I, I], I),

@@ -124,6 +124,17 @@ class HMatrix:
             check(lib().gbem_lu_trace_host(self._h, B.ctypes.data, self.N, ncols or B.shape[1], tr.ctypes.data))
         return complex(tr[0], tr[1])
 
+    def TraceMInvDisplacement(self, geometry, Omega, axis=2):
+        """TraceMInvdM for the rigid displacement of the geometry's first
+        surface along an axis, over that surface's basis functions; dM is
+        assembled on the device."""
+        tr = np.zeros(2)
+        eps, mu = geometry.eps_mu(Omega)
+        Omega = complex(Omega)
+        check(lib().gbem_lu_trace_displacement(self._h, axis, Omega.real, Omega.imag, eps.ctypes.data, mu.ctypes.data,
+                                               tr.ctypes.data))
+        return complex(tr[0], tr[1])
+
     def LUSolve(self, B, Trans="N"):
         """Solve op(M) X = B for a vector or an N x nrhs array; returns X."""
         B = np.asarray(B)

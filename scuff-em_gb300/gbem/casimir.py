@@ -14,7 +14,8 @@ real; the reference forms (applications/scuff-cas3D/CasimirIntegrand.cc):
 Here M, the T blocks and dU/dz are assembled on the GPU (gbem_assemble and
 gbem_assemble_block_gradient in real storage), factored there
 (gbem_lu_factor), and log|det| and the trace are reduced there
-(gbem_lu_log_abs_det, gbem_lu_trace_host).
+(gbem_lu_log_abs_det, gbem_lu_trace_displacement): nothing of the size of a
+matrix passes through the host.
 """
 from __future__ import annotations
 
@@ -90,12 +91,6 @@ class CasimirIntegrand:
             ld = self.log_abs_det_blocks(xi) - M.LogAbsDet()
             E = -ld / (2.0 * math.pi) if math.isfinite(ld) else 0.0
         if zforce:
-            N1 = self.nbf[0]
-            dM = np.zeros((self.N, N1), dtype=np.float64, order="F")
-            for s in range(1, len(self.surfaces)):
-                g = self.G.AssembleBEMMatrixBlockGradient(0, s, 1j * xi, real=True, components=(2,))[2]
-                o = self.offset[s]
-                dM[o:o + self.nbf[s], :] = g.T
-            tr = 2.0 * M.TraceMInvdM(dM, N1).real
+            tr = 2.0 * M.TraceMInvDisplacement(self.G, 1j * xi).real
             F = -tr / (2.0 * math.pi) if math.isfinite(tr) else 0.0
         return E, F
