@@ -171,3 +171,15 @@ def test_block_row_solve_edges(N):
     A = rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))
     LU, piv = _factor(A)
     _check_backward(A, LU, piv)
+
+
+@pytest.mark.parametrize("N", [1, 2, 3, 4, 5, 15, 16, 17, 20, 31, 33, 47, 63, 65, 130, 512, 1023, 1025, 1041])
+def test_leaf_lanes_per_row(N):
+    """Panels whose rows are spread over four lanes (up to 64 rows a CTA), where
+    a leaf, a group of four columns or that range ends."""
+    import scipy.linalg as sl
+    rng = np.random.default_rng(7 * N)
+    A = rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))
+    LU, piv = _factor(A)
+    assert np.array_equal(piv, sl.lu_factor(A)[1])
+    _check_backward(A, LU, piv)
