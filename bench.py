@@ -539,7 +539,7 @@ def main():
             "frac": fl / (far_ms * 1e-3) / 1e12 / FP32_PEAK_TFLOPS,
             "peak_kind": "nominal FP32 (no measured FP32 figure in MEASURED_PEAKS.json)",
             "hbm_gbs": (N * N * 8 + G.np_total * 64 * 8) / (far_ms * 1e-3) / 1e9, "hbm_peak_gbs": hbm_peak,
-            "note": "float-float arithmetic issues ~640 FP32 instructions per sample against the 100-flop "
+            "note": "float-float arithmetic issues ~770 FP32 instructions per sample against the 100-flop "
                     "convention"}
     # solve and refinement: every sweep reads the complex64 factor once (its
     # forward and backward triangular solves) and the complex64 matrix once
@@ -549,10 +549,10 @@ def main():
         sweeps = statistics.median(iters)
         nbytes = 2 * sweeps * N * N * 8
         out["roofline_solve"] = {
-            "kernel": "trsv_coop (4 RHS) + residual_partial_df", "bound": "hbm",
+            "kernel": "trsv_words (4 RHS) + residual_partial_df", "bound": "hbm",
             "bytes_per_step": nbytes, "achieved_gbs": nbytes / (sol_ms * 1e-3) / 1e9, "peak_gbs": hbm_peak,
             "frac": nbytes / (sol_ms * 1e-3) / 1e9 / hbm_peak, "sweeps": sweeps,
-            "note": "latency-bound: one grid barrier per 64-row block in each triangular solve"}
+            "note": "latency-bound: a chain of 64-row blocks in each triangular solve"}
 
     # plain FP64 path (same geometry): assemble C128, LU, solve -- repeated,
     # with its own stage split
@@ -586,7 +586,9 @@ def main():
                                           "frac": a64 / FP64_PEAK_TFLOPS,
                                           "peak_kind": "nominal FP64 (no measured FP64 figure in "
                                                        "MEASURED_PEAKS.json)",
-                                          "kernel": "panel_kernel<double> + gemm_simt<double> (8N^3/3 flops)"}
+                                          "kernel": "panels on the FP64 pipe, trailing updates by integer slices "
+                                                    "on the tensor cores (oz_gemm_kernel): above 1 is possible "
+                                                    "(8N^3/3 flops)"}
         out["speedup_vs_fp64"] = out["value"] / out["fp64"]["value"]
         out["accuracy"] = {"rel_err_x_vs_fp64": rel_x,
                            "rel_err_extinction_power_vs_fp64": float(np.max(np.abs(pmx - p64) / np.abs(p64))),

@@ -166,8 +166,7 @@ gbem_status gbem_assemble_block_host(gbem_geometry *g, int nsa, int nsb, double 
 /* ---- dense LU ------------------------------------------------------------ */
 /* Replaces HMatrix::LUFactorize (libs/libhmat/LBWrappers.cc:151-171):
  * in-place LU with partial pivoting of a C128 (zgetrf semantics), F64
- * (dgetrf semantics, computed as complex128 with zero imaginary parts) or C64
- * matrix.  ipiv (optional, host, N ints) receives 1-based pivots; info is 0,
+ * (dgetrf semantics) or C64 matrix.  ipiv (optional, host, N ints) receives 1-based pivots; info is 0,
  * or k > 0 if U(k,k) is exactly zero. */
 gbem_status gbem_lu_factor(gbem_matrix *M, int *ipiv, int *info);
 

@@ -179,7 +179,7 @@ gbem_status lu_factor_device(void* dA, int N, int ld, int dtype, int* d_ipiv, in
 size_t lu_solve_ws_bytes(int N, int dtype);
 gbem_status lu_solve_device(const void* dA, int N, int ld, int dtype, const int* d_perm, char trans, int nrhs,
                             void* dB, int ldb, void* ws, cudaStream_t s);
-// X = A^-1 B for many right-hand sides (blocked: block inverses + GEMM updates)
+// X = A^-1 B for many right-hand sides (by halves, with GEMM updates)
 gbem_status lu_solve_many_device(const void* dA, int N, int ld, int dtype, const int* d_perm, int nrhs, void* dB, int ldb,
                                  cudaStream_t s);
 gbem_status residual_device(const void* dA, int lda, int dtype, int N, const double* dX, int ldx, const double* dB,
