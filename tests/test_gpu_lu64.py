@@ -163,10 +163,9 @@ def test_triangular_solve_edges(N, nrhs):
 
 @pytest.mark.parametrize("N", [272, 288, 304, 336, 400, 417, 560, 600, 1700])
 def test_block_row_solve_edges(N):
-    """The block rows right of a 256-column panel (substitution of 256 rows up
-    to 320 columns, of 128 rows up to 1280, by halves with tensor-core updates
-    beyond) and inside it, one, two and four columns per CTA, a last block of
-    half its rows."""
+    """The block rows right of a panel (substitution of 128 rows up to 1280
+    columns, by halves with tensor-core updates beyond) and inside it, one, two
+    and four columns per CTA, a last block of half its rows."""
     rng = np.random.default_rng(3 * N)
     A = rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))
     LU, piv = _factor(A)
