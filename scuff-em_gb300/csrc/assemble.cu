@@ -1234,7 +1234,7 @@ struct PPair64Args {
   const int* emax;
   int offa, offb;     // global index of the first panel of each surface
   int nrow, ncp, sym;
-  double2* out;       // [NC][9][ncp][nrow]; x = NaN: a near pair
+  double2* out;       // [NC][9][ncp][nrow]; x = NaN: a near pair, if it is listed as one
 };
 __device__ __forceinline__ cx<double> scaled(cx<double> f, cx<double> h) { return f * h; }
 __device__ __forceinline__ cx<double> scaled(cx<double> f, double h) { return h * f; }
@@ -1390,15 +1390,15 @@ __global__ void __launch_bounds__(256) stamp64_kernel(Stamp64Args sp) {
         for (int c = 0; c < NC; c++) v[w][c] = mk(0.0, 0.0);
         if (pa < 0 || pb < 0) continue;
         const double2* src = sp.ppv + (size_t)(3 * ja + jb) * cs + (size_t)cl * sp.nrow + pa;
+        // a NaN is a near pair (its value comes from near_kernel / self_kernel)
+        // where the pair is listed, else a far pair's own value, and stays one
         const double2 f0 = src[0];
-        if (!isnan(f0.x)) {
+        const int hit = isnan(f0.x) ? near_hit(a, a.row_panel_offset + pa, sp.offb + pb) : -1;
+        if (hit < 0) {
           v[w][0] = mk(f0.x, f0.y);
 #pragma unroll
           for (int c = 1; c < NC; c++) { const double2 f = src[c * fs]; v[w][c] = mk(f.x, f.y); }
         } else {
-          // near pair: values of near_kernel / self_kernel
-          const int hit = near_hit(a, a.row_panel_offset + pa, sp.offb + pb);
-          if (hit < 0) continue;  // cannot happen: every rRel<=4 pair is listed
           const double* nv = a.nearval + 54 * (size_t)(hit >> 1) + 6 * ((hit & 1) ? (3 * jb + ja) : (3 * ja + jb));
 #pragma unroll
           for (int c = 0; c < NC; c++) v[w][c] = mk(nv[2 * c], nv[2 * c + 1]);

@@ -185,3 +185,23 @@ def test_two_surfaces_every_pair_form_matches_oracle(omega):
             ok &= far[bf[:, a]][:, bf[:, b]]
     assert ok.mean() > 0.3
     assert np.abs(A - Ao)[ok].max() <= 1e-13 * np.abs(Ao).max()
+
+
+@pytest.mark.parametrize("bad", ["omega", "eps", "overflow"])
+@pytest.mark.parametrize("pec", [(True, True), (False, False), (True, False)])
+def test_non_finite_far_field_stays_visible(bad, pec):
+    """A wavenumber that is not a number, or one whose e^{ikr} overflows, gives
+    entries that are not finite, never zeros: the block of two bodies without
+    near pairs, and the far entries of a body's own block."""
+    from gbem import RWGGeometry, mesh
+    from gbem.api import Material
+    V, P = mesh.icosphere(1)
+    m = Material(2.25)
+    gs = [{"V": V + [0.0, 0.0, 12.0 * i], "P": P, "material": None if pec[i] else m} for i in range(2)]
+    G = RWGGeometry(gs, exterior=Material(np.nan) if bad == "eps" else None)
+    w = {"omega": complex(np.nan, 0.0), "eps": 1.0, "overflow": -400.0j}[bad]
+    for a, b in ((0, 1), (1, 0)):
+        M = G.AssembleBEMMatrixBlock(a, b, w)
+        assert not np.isfinite(M).any()
+    if bad != "overflow":  # (within a body the exponent stays in range)
+        assert not np.isfinite(G.AssembleBEMMatrixBlock(0, 0, w)).any()

@@ -184,3 +184,20 @@ def test_gradient_of_distant_bodies_in_every_form(omega, pec):
             real = G.AssembleBEMMatrixBlockGradient(a, b, omega, real=True)
             for mu in range(3):
                 assert np.array_equal(real[mu], grads[mu].real)
+
+
+@pytest.mark.parametrize("bad", ["omega", "eps", "overflow"])
+@pytest.mark.parametrize("pec", [(True, True), (False, False), (True, False)])
+def test_non_finite_gradient_stays_visible(bad, pec):
+    """The gradient of a block without near pairs is not finite, never zero,
+    where the wavenumber is not a number or e^{ikr} overflows."""
+    from gbem import RWGGeometry, mesh
+    from gbem.api import Material
+    V, P = mesh.icosphere(1)
+    m = Material(2.25)
+    G = RWGGeometry([{"V": V + [0.7 * i, 0.4 * i, 12.0 * i], "P": P, "material": None if pec[i] else m} for i in range(2)],
+                    exterior=Material(np.nan) if bad == "eps" else None)
+    w = {"omega": complex(np.nan, 0.0), "eps": 1.0, "overflow": -400.0j}[bad]
+    for a, b in ((0, 1), (1, 0)):
+        for g in G.AssembleBEMMatrixBlockGradient(a, b, w):
+            assert not np.isfinite(g).any()
