@@ -1047,15 +1047,15 @@ __global__ void __launch_bounds__(256) stamp_kernel(StampArgs sp) {
         const float* src = sp.ppv + (size_t)(3 * ja + jb) * cs + (size_t)cl * sp.nrow + pa;
         cff v0, v2 = cff_zero();
         cx<float> v1 = mk(0.0f, 0.0f);
+        // a NaN: a near pair (FP64 values of near_kernel / self_kernel) if it
+        // is listed, else a far pair's own value
         const float f0 = src[0];
-        if (!isnan(f0)) {
+        const int hit = isnan(f0) ? near_hit(a, a.row_panel_offset + pa, sp.offb + pb) : -1;
+        if (hit < 0) {
           v0 = cffv(ffv(f0, src[fs]), ffv(src[2 * fs], src[3 * fs]));
           if (NC > 1) v1 = mk(src[4 * fs], src[5 * fs]);
           if (NC > 2) v2 = cffv(ffv(src[6 * fs], src[7 * fs]), ffv(src[8 * fs], src[9 * fs]));
         } else {
-          // near pair: FP64 values of near_kernel / self_kernel
-          const int hit = near_hit(a, a.row_panel_offset + pa, sp.offb + pb);
-          if (hit < 0) continue;  // cannot happen: every rRel<=4 pair is listed
           const double* v = a.nearval + 54 * (size_t)(hit >> 1) + 6 * ((hit & 1) ? (3 * jb + ja) : (3 * ja + jb));
           v0 = cff_of(mk(v[0], v[1]));
           if (NC > 1) v1 = mk((float)v[2], (float)v[3]);

@@ -205,3 +205,16 @@ def test_non_finite_far_field_stays_visible(bad, pec):
         assert not np.isfinite(M).any()
     if bad != "overflow":  # (within a body the exponent stays in range)
         assert not np.isfinite(G.AssembleBEMMatrixBlock(0, 0, w)).any()
+
+
+@pytest.mark.parametrize("pec", [(True, True), (False, False), (True, False)])
+def test_non_finite_mixed_far_field_stays_visible(pec):
+    """The mixed form's entries between two distant bodies, likewise."""
+    from gbem import RWGGeometry, mesh
+    from gbem.api import Material
+    V, P = mesh.icosphere(1)
+    G = RWGGeometry([{"V": V + [0.0, 0.0, 12.0 * i], "P": P, "material": None if pec[i] else Material(2.25)}
+                     for i in range(2)])
+    n = G.NumBFs(0)
+    M = G.AssembleBEMMatrix(complex(np.nan, 0.0), precision="mixed").numpy()
+    assert not np.isfinite(M[:n, n:]).any() and not np.isfinite(M[n:, :n]).any()
