@@ -182,3 +182,30 @@ def test_leaf_lanes_per_row(N):
     LU, piv = _factor(A)
     assert np.array_equal(piv, sl.lu_factor(A)[1])
     _check_backward(A, LU, piv)
+
+
+@pytest.mark.parametrize("real", [False, True])
+@pytest.mark.parametrize("power", [-530, -520, -505, 505, 520, 900])
+def test_pivots_of_extreme_size(power, real):
+    """Pivots whose |z|^2 leaves the FP64 range: a matrix times a power of two
+    has the same L, and U times that power, exactly."""
+    N = 150
+    rng = np.random.default_rng(9)
+    A = rng.standard_normal((N, N))
+    if not real:
+        A = A + 1j * rng.standard_normal((N, N))
+    out = []
+    for s in (1.0, 2.0 ** power):
+        if real:
+            from gbem._lib import F64
+            from gbem.api import HMatrix
+            M = HMatrix(_strip(N), F64)
+            M.set(A * s)
+            assert M.LUFactorize() == 0
+            out.append((M.numpy(), M.ipiv))
+        else:
+            out.append(_factor(A * s))
+    (F0, p0), (F1, p1) = out
+    assert np.array_equal(p0, p1)
+    assert np.array_equal(np.tril(F0, -1), np.tril(F1, -1))
+    assert np.array_equal(np.triu(F0) * 2.0 ** power, np.triu(F1))
