@@ -72,8 +72,6 @@ constexpr int EXP_BAD = 1 << 20;  // scale exponent of a row or column that is n
 constexpr int VECS = 16;          // rows of A (columns of B) per packing CTA
 }  // namespace oz
 
-__device__ int g_oz_error = 0;
-
 // exponent field (at least 1) of a double's high word
 __device__ __forceinline__ int exp_field(unsigned hi) { return max((int)((hi >> 20) & 0x7ffu), 1); }
 
@@ -214,7 +212,8 @@ template <bool CPLX, int BN>
 __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__ CUtensorMap mapA,
                                                           const __grid_constant__ CUtensorMap mapB, double* C,
                                                           long long ldc, const int* ea, const int* eb, int m, int n,
-                                                          int kblocks, int pairs, int mt, int ntiles) {
+                                                          int kblocks, int pairs, int mt, int ntiles,
+                                                          int* wait_error) {
   pdl_wait();
   pdl_trigger();
   using TL = oz::Tile<BN>;
@@ -227,17 +226,19 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
   uint64_t* acc_empty = acc_full + 2;       // [2] drain -> MMA (8 warp arrivals)
   uint64_t* done = acc_empty + 2;           // all MMAs retired
   uint32_t* tmem_slot = (uint32_t*)(done + 1);
-  __shared__ int s_fail;
+  __shared__ int s_fail, s_skip;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = CPLX ? 2 * n : n;  // real output columns
   const int kbx = min(oz::KB, kblocks);
-  if (*(volatile int*)&g_oz_error) return;  // a CTA gave up on a wait: the rest of the grid does no work
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TL::STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }
     mbar_init(done, 1);
     s_fail = 0;
+    // once a CTA of this call has given up a wait, the rest do no work (read
+    // once, so that the whole CTA takes the same way)
+    s_skip = *(volatile int*)wait_error;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -250,7 +251,8 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == 0) {
+  if (s_skip) {
+  } else if (warp == 0) {
     if (lane == 0) {
       RingPos<TL::STAGES> r;
       int issued = 0;  // stages in use
@@ -342,7 +344,8 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
           const int acc = u & 1;
           ok = mbar_wait(&acc_full[acc], (uint32_t)((u >> 1) & 1));
           if (!ok) atomicExch(&s_fail, 1);
-          if (!ok || *(volatile int*)&s_fail) { ok = false; break; }
+          ok = __all_sync(0xffffffffu, ok && !*(volatile int*)&s_fail);  // the warp together: its TMEM reads are collective
+          if (!ok) break;
           tc_fence_after();
           const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN + half * CW);
 #pragma unroll
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN));
   }
-  if (threadIdx.x == 0 && s_fail) atomicExch(&g_oz_error, 1);
+  if (threadIdx.x == 0 && s_fail) atomicExch(wait_error, 1);
 }
 
 static size_t oz_round(size_t x) { return (x + 1023) & ~(size_t)1023; }
@@ -421,7 +424,7 @@ size_t oz_gemm_ws_bytes(int m, int n, int k, bool cplx) {
 // update does it
 template <bool CPLX>
 static bool update(double* C, long long ldc, const double* A, long long lda, const double* B, long long ldb, int m,
-                   int n, int k, void* ws, size_t ws_bytes, cudaStream_t s, cudaError_t* err) {
+                   int n, int k, void* ws, size_t ws_bytes, int* wait_error, cudaStream_t s, cudaError_t* err) {
   *err = cudaSuccess;
   if (m <= 0 || n <= 0 || k <= 0) return true;
   const int kreal = CPLX ? 2 * k : k;
@@ -454,28 +457,17 @@ static bool update(double* C, long long ldc, const double* A, long long lda, con
   if (*err != cudaSuccess) return false;
   const int ntiles = mt * ((nb + bn - 1) / bn);
   *err = launch_pdl(kernel, dim3(std::min(ntiles, nsm)), dim3(320), (size_t)smem, s, ma, mb, C, ldc, ea, eb, m, n,
-                    Kp / oz::BK, oz::ACC_TERMS / kreal, mt, ntiles);
+                    Kp / oz::BK, oz::ACC_TERMS / kreal, mt, ntiles, wait_error);
   return *err == cudaSuccess;
 }
 
 bool oz_gemm_update(cx<double>* C, long long ldc, const cx<double>* A, long long lda, const cx<double>* B, long long ldb,
-                    int m, int n, int k, void* ws, size_t ws_bytes, cudaStream_t s, cudaError_t* err) {
-  return update<true>((double*)C, ldc, (const double*)A, lda, (const double*)B, ldb, m, n, k, ws, ws_bytes, s, err);
+                    int m, int n, int k, void* ws, size_t ws_bytes, int* wait_error, cudaStream_t s, cudaError_t* err) {
+  return update<true>((double*)C, ldc, (const double*)A, lda, (const double*)B, ldb, m, n, k, ws, ws_bytes, wait_error, s, err);
 }
 bool oz_gemm_update(double* C, long long ldc, const double* A, long long lda, const double* B, long long ldb, int m,
-                    int n, int k, void* ws, size_t ws_bytes, cudaStream_t s, cudaError_t* err) {
-  return update<false>(C, ldc, A, lda, B, ldb, m, n, k, ws, ws_bytes, s, err);
-}
-
-// error word of the bounded waits (nonzero: a wait gave up)
-int oz_gemm_error(bool reset) {
-  int h = 0;
-  cudaMemcpyFromSymbol(&h, g_oz_error, sizeof(int));
-  if (reset && h) {
-    int z = 0;
-    cudaMemcpyToSymbol(g_oz_error, &z, sizeof(int));
-  }
-  return h;
+                    int n, int k, void* ws, size_t ws_bytes, int* wait_error, cudaStream_t s, cudaError_t* err) {
+  return update<false>(C, ldc, A, lda, B, ldb, m, n, k, ws, ws_bytes, wait_error, s, err);
 }
 
 }  // namespace gbem

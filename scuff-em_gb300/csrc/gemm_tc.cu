@@ -23,7 +23,8 @@
 //   warps 2-9 epilogue: tcgen05.ld 32 lanes x 32 columns at a time, C -= D
 //            (C loads issued before the TMEM read so they overlap)
 // Every mbarrier wait is bounded; on timeout the CTA records an error code,
-// drains its outstanding TMA copies (bounded), frees its TMEM and exits.
+// drains its outstanding TMA copies (bounded), frees its TMEM and exits.  The
+// word belongs to the factorisation (wait_error, beside its info).
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cstdint>
@@ -43,8 +44,6 @@ static_assert((2 * STAGES + 5) * 8 + 4 <= 256, "barrier area");
 constexpr uint32_t TMEM_COLS = 256;
 constexpr uint32_t IDESC = idesc_bf16(BM, BN);
 }  // namespace tc
-
-__device__ int g_tc_error = 0;
 
 // ---------------- split packing ----------------
 __device__ __forceinline__ void split_bf16(float x, __nv_bfloat16* hi, __nv_bfloat16* lo) {
@@ -126,7 +125,7 @@ __global__ void zero_pad(__nv_bfloat16* out, long long rows, int K6, int Kp) {
 __global__ void __launch_bounds__(320, 1) tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA,
                                                           const __grid_constant__ CUtensorMap mapB, cx<float>* C,
                                                           long long ldc, int m, int n, int kblocks, int mt,
-                                                          int ntiles) {
+                                                          int ntiles, int* wait_error) {
   pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -138,17 +137,17 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_kernel(const __grid_constant__
   uint64_t* acc_empty = acc_full + 2;       // [2] epilogue -> MMA (8 warp arrivals)
   uint64_t* drain = acc_empty + 2;          // all MMAs retired
   uint32_t* tmem_slot = (uint32_t*)(drain + 1);
-  __shared__ int s_fail;
+  __shared__ int s_fail, s_skip;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // once any CTA has given up on a wait, the rest of the grid does no work
-  if (*(volatile int*)&g_tc_error) return;
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < tc::STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }
     mbar_init(drain, 1);
     s_fail = 0;
+    // once a CTA of this call has given up a wait, the rest do no work (read
+    // once, so that the whole CTA takes the same way)
+    s_skip = *(volatile int*)wait_error;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -161,7 +160,8 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_kernel(const __grid_constant__
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == 0) {
+  if (s_skip) {
+  } else if (warp == 0) {
     if (lane == 0) {
       // producer: one ring of STAGES slots across all of this CTA's tiles
       RingPos<tc::STAGES> r;
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_kernel(const __grid_constant__
       const int row = tm * tc::BM + q * 32 + lane;
       const bool ok = mbar_wait(&acc_full[acc], (uint32_t)((i >> 1) & 1));
       if (!ok) atomicExch(&s_fail, 1);
-      if (!ok || *(volatile int*)&s_fail) break;
+      if (!__all_sync(0xffffffffu, ok && !*(volatile int*)&s_fail)) break;  // the warp together: its TMEM reads are collective
       tc_fence_after();
       const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * tc::TMEM_COLS);
       for (int c0 = half * (tc::BN / 2); c0 < (half + 1) * (tc::BN / 2); c0 += 32) {
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_kernel(const __grid_constant__
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * tc::TMEM_COLS));
   }
-  if (threadIdx.x == 0 && s_fail) atomicExch(&g_tc_error, 1);
+  if (threadIdx.x == 0 && s_fail) atomicExch(wait_error, 1);
 }
 
 // ---------------- host side ----------------
@@ -305,7 +305,7 @@ void tc_gemm_set_enabled(int on) { g_tc_mode = on ? 1 : 0; }
 void tc_gemm_thread_off(int off) { tl_tc_off = off; }
 
 bool tc_gemm_update(cx<float>* C, long long ldc, const cx<float>* A, long long lda, const cx<float>* B, long long ldb,
-                    int m, int n, int k, void* ws, size_t ws_bytes, cudaStream_t s, cudaError_t* err) {
+                    int m, int n, int k, void* ws, size_t ws_bytes, int* wait_error, cudaStream_t s, cudaError_t* err) {
   *err = cudaSuccess;
   if (g_tc_mode < 0) {
     const char* e = getenv("GBEM_LU_TC");
@@ -343,20 +343,9 @@ bool tc_gemm_update(cx<float>* C, long long ldc, const cx<float>* A, long long l
   const int mt = (m + tc::BM - 1) / tc::BM, ntn = (2 * n + tc::BN - 1) / tc::BN;
   const int ntiles = mt * ntn;
   launch_pdl(tc_gemm_kernel, dim3(std::min(ntiles, nsm)), dim3(320), (size_t)tc::SMEM_BYTES, s, ma, mb, C, ldc, m, n,
-             Kp / tc::BK, mt, ntiles);
+             Kp / tc::BK, mt, ntiles, wait_error);
   *err = cudaGetLastError();
   return *err == cudaSuccess;
-}
-
-// error word of the bounded waits (nonzero: a wait gave up)
-int tc_gemm_error(bool reset) {
-  int h = 0;
-  cudaMemcpyFromSymbol(&h, g_tc_error, sizeof(int));
-  if (reset) {
-    int z = 0;
-    cudaMemcpyToSymbol(g_tc_error, &z, sizeof(int));
-  }
-  return h;
 }
 
 }  // namespace gbem
