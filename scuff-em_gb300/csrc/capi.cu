@@ -884,7 +884,8 @@ gbem_status gbem_lu_solve(gbem_matrix* M, char trans, int nrhs, void* B, int ldb
     make_complex<<<(unsigned)(((long long)N * nrhs + 255) / 256), 256, 0, s>>>((const double*)dBr, N, (double2*)dB, N,
                                                                                N, nrhs);
     stats_launch(ST_OTHER, 3);
-    gbem_status st = lu_solve_device(tA, N, N, GBEM_C128, M->d_perm, trans, nrhs, dB, N, dY, s);
+    gbem_status st = lu_solve_begin(dY, s);
+    if (st == GBEM_OK) st = lu_solve_device(tA, N, N, GBEM_C128, M->d_perm, trans, nrhs, dB, N, dY, s);
     if (st == GBEM_OK) {
       take_real<<<(unsigned)(((long long)N * nrhs + 255) / 256), 256, 0, s>>>((const double2*)dB, N, (double*)dBr, N, N,
                                                                               nrhs);
@@ -892,6 +893,7 @@ gbem_status gbem_lu_solve(gbem_matrix* M, char trans, int nrhs, void* B, int ldb
                                         cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
       if (e != cudaSuccess) st = cuda_status(e, "solve download");
+      if (st == GBEM_OK) st = lu_solve_end(dY, s);
     }
     cudaFreeAsync(tA, s); cudaFreeAsync(dBr, s); cudaFreeAsync(dB, s); cudaFreeAsync(dY, s);
     cudaStreamSynchronize(s);
@@ -903,12 +905,14 @@ gbem_status gbem_lu_solve(gbem_matrix* M, char trans, int nrhs, void* B, int ldb
   CHECK_CUDA(cudaMallocAsync(&dY, lu_solve_ws_bytes(M->N, M->dtype), M->stream), "solve alloc");
   CHECK_CUDA(cudaMemcpy2DAsync(dB, (size_t)M->N * es, B, (size_t)ldb * es, (size_t)M->N * es, nrhs,
                                cudaMemcpyHostToDevice, M->stream), "solve upload");
-  gbem_status st = lu_solve_device(M->d, M->N, M->ld, M->dtype, M->d_perm, trans, nrhs, dB, M->N, dY, M->stream);
+  gbem_status st = lu_solve_begin(dY, M->stream);
+  if (st == GBEM_OK) st = lu_solve_device(M->d, M->N, M->ld, M->dtype, M->d_perm, trans, nrhs, dB, M->N, dY, M->stream);
   if (st == GBEM_OK) {
     cudaError_t e = cudaMemcpy2DAsync(B, (size_t)ldb * es, dB, (size_t)M->N * es, (size_t)M->N * es, nrhs,
                                       cudaMemcpyDeviceToHost, M->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(M->stream);
     if (e != cudaSuccess) st = cuda_status(e, "solve download");
+    if (st == GBEM_OK) st = lu_solve_end(dY, M->stream);
   }
   cudaFreeAsync(dB, M->stream);
   cudaFreeAsync(dY, M->stream);
@@ -1236,11 +1240,13 @@ gbem_status gbem_lu_solve_host(const double* ZM, int N, int ld, const int* ipiv,
     e = cudaMemcpy2DAsync(dB, (size_t)N * 16, B, (size_t)ldb * 16, (size_t)N * 16, nrhs, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(dperm, perm.data(), sizeof(int) * N, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) st = cuda_status(e, "gbem_lu_solve_host");
+  if (st == GBEM_OK) st = lu_solve_begin(dY, s);
   if (st == GBEM_OK) st = lu_solve_device(dA, N, N, GBEM_C128, dperm, trans, nrhs, dB, N, dY, s);
   if (st == GBEM_OK) {
     e = cudaMemcpy2DAsync(B, (size_t)ldb * 16, dB, (size_t)N * 16, (size_t)N * 16, nrhs, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) st = cuda_status(e, "gbem_lu_solve_host");
+    if (st == GBEM_OK) st = lu_solve_end(dY, s);
   }
   cudaFree(dA); cudaFree(dB); cudaFree(dY); cudaFree(dperm);
   cudaStreamDestroy(s);
@@ -1550,6 +1556,7 @@ static gbem_status solve_mixed_impl(gbem_geometry* g, double omega_re, double om
     }
     return rel <= tol;
   };
+  if (st == GBEM_OK) st = lu_solve_begin(dY, s);
   bool ok = refine(max_iter);
   if (st == GBEM_OK && !ok) {
     // the split-BF16 factor is too coarse for this matrix: factor it again
@@ -1582,6 +1589,7 @@ static gbem_status solve_mixed_impl(gbem_geometry* g, double omega_re, double om
                           x_host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) st = cuda_status(e, "gbem_solve_mixed download");
+    if (st == GBEM_OK) st = lu_solve_end(dY, s);
   }
   if (M128) gbem_matrix_destroy(M128);
   if (iters) *iters = it;

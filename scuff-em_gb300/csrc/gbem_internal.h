@@ -177,6 +177,10 @@ void cache_stats(const Geometry* g, long long* hits, long long* misses);
 gbem_status lu_factor_device(void* dA, int N, int ld, int dtype, int* d_ipiv, int* h_info, cudaStream_t s,
                              void** ws, size_t* ws_bytes);
 size_t lu_solve_ws_bytes(int N, int dtype);
+// before the first and after the last solve of a call on a workspace: whether
+// every bounded wait between them ended (GBEM_ETIMEOUT: the solutions are NaN)
+gbem_status lu_solve_begin(void* ws, cudaStream_t s);
+gbem_status lu_solve_end(const void* ws, cudaStream_t s);
 gbem_status lu_solve_device(const void* dA, int N, int ld, int dtype, const int* d_perm, char trans, int nrhs,
                             void* dB, int ldb, void* ws, cudaStream_t s);
 // X = A^-1 B for many right-hand sides (by halves, with GEMM updates)

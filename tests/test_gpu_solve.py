@@ -229,3 +229,56 @@ def test_mixed_solve_beyond_the_l2():
     B = rng.standard_normal((G.TotalBFs, 5)) + 1j * rng.standard_normal((G.TotalBFs, 5))
     X, it, res = G.solve_mixed(2.0, B, tol=1e-10, max_iter=12)
     assert res <= 1e-10 and np.isfinite(X).all()
+
+
+_GIVE_UP = r"""
+import ctypes, sys, numpy as np
+sys.path.insert(0, sys.argv[1])
+from gbem import C64, C128, RWGGeometry, mesh
+from gbem._lib import GBEM_ETIMEOUT, F64, GbemError, check, lib
+from gbem.api import HMatrix
+V, P = mesh.icosphere(2)
+G = RWGGeometry([{"V": V, "P": P, "material": None}])
+N = G.TotalBFs
+rng = np.random.default_rng(0)
+B = rng.standard_normal((N, 3)) + 1j * rng.standard_normal((N, 3))
+out = []
+def call(f):
+    try:
+        f()
+        out.append("ok")
+    except GbemError as e:
+        out.append("timeout" if e.status == GBEM_ETIMEOUT else str(e))
+for dt in (C128, C64, F64):
+    M = HMatrix(G, dt)
+    A = rng.standard_normal((N, N)) + N * np.eye(N)
+    M.set(A)
+    assert M.LUFactorize() == 0
+    b = B.real.copy() if dt == F64 else B.astype(M.np_dtype)
+    call(lambda: M.LUSolve(b))
+    if dt != F64:
+        x = np.asfortranarray(b)
+        call(lambda: check(lib().gbem_lu_solve_noalloc(M._h, b"N", 3, x.ctypes.data, N)))
+LU = np.asfortranarray(np.eye(N, dtype=np.complex128) * 2.0)
+ipiv = np.arange(1, N + 1, dtype=np.int32)
+X = np.asfortranarray(B)
+st = lib().gbem_lu_solve_host(LU.ctypes.data, N, N, ipiv.ctypes.data, b"N", 3, X.ctypes.data, N)
+out.append({0: "ok", GBEM_ETIMEOUT: "timeout"}.get(st, str(st)))
+call(lambda: G.solve_mixed(1.0, B, tol=1e-10, max_iter=4))
+print(" ".join(out))
+"""
+
+
+@pytest.mark.parametrize("spins,want", [("-1", "timeout"), ("4194304", "ok")])
+def test_triangular_solve_that_gives_up_says_so(spins, want):
+    """A wait of the triangular solves that runs out (here: the first time a
+    value is not there yet) gives GBEM_ETIMEOUT from every entry point that
+    solves, and the context stays usable.  The limit is read once per process."""
+    import os
+    import subprocess
+    import sys
+    repo = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", _GIVE_UP, os.path.join(repo, "scuff-em_gb300")],
+                         env=dict(os.environ, GBEM_TRSV_SPINS=spins), check=True, timeout=600, capture_output=True,
+                         text=True).stdout.split()
+    assert out == [want] * 7
