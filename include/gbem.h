@@ -190,7 +190,8 @@ gbem_status gbem_lu_trace_host(gbem_matrix *M, const void *B, int ldb, int ncols
  * (0, 1, 2), over that surface's basis functions: B holds the transposes of
  * the gradients of the blocks (0, s), s >= 1 (gbem_assemble_block_gradient),
  * assembled and transposed on the device.  M factored, F64 or C128 (F64: an
- * imaginary omega, as there). */
+ * imaginary omega, as there).  The surfaces are those of the geometry M was
+ * created on; eps and mu hold 2 doubles for each of its regions. */
 gbem_status gbem_lu_trace_displacement(gbem_matrix *M, int axis, double omega_re, double omega_im,
                                        const double *eps, const double *mu, double *trace);
 

@@ -127,7 +127,11 @@ class HMatrix:
     def TraceMInvDisplacement(self, geometry, Omega, axis=2):
         """TraceMInvdM for the rigid displacement of the geometry's first
         surface along an axis, over that surface's basis functions; dM is
-        assembled on the device."""
+        assembled on the device, from the surfaces of the matrix's own
+        geometry: another one must have the same surfaces (its materials
+        are taken)."""
+        if not geometry.same_surfaces(self.geometry):
+            raise ValueError("TraceMInvDisplacement: the geometry has other surfaces than the matrix's")
         tr = np.zeros(2)
         eps, mu = geometry.eps_mu(Omega)
         Omega = complex(Omega)
@@ -209,6 +213,14 @@ class RWGGeometry:
         if getattr(self, "_h", None):
             lib().gbem_geometry_destroy(self._h)
             self._h = None
+
+    def same_surfaces(self, other):
+        """Whether the other geometry has the same meshes and regions."""
+        if self is other:
+            return True
+        return (len(self.surfaces) == len(other.surfaces) and len(self.materials) == len(other.materials) and
+                all(a["pec"] == b["pec"] and a["interior"] == b["interior"] and np.array_equal(a["V"], b["V"]) and
+                    np.array_equal(a["P"], b["P"]) for a, b in zip(self.surfaces, other.surfaces)))
 
     def eps_mu(self, Omega):
         eps = np.array([[m.eps.real, m.eps.imag] for m in self.materials], dtype=np.float64).ravel()

@@ -68,3 +68,57 @@ def test_u_block_and_gradient_match_oracle(cas, golden):
     dUo = (ora_u(h) - ora_u(-h)).real / (2 * h)
     # central differences: truncation ~h^2 of the entries' third derivative
     assert np.abs(dUz[:, cols] - dUo).max() / np.abs(dUo).max() < 1e-6
+
+
+def _three_bodies(pec, gap):
+    from gbem import RWGGeometry, mesh
+    from gbem.api import Material
+    m = None if pec else Material(2.5)
+    V0, P0 = mesh.icosphere(1)
+    V1, P1 = mesh.rounded_cube(108, seed=4)
+    V2, P2 = mesh.icosphere(0)
+    return RWGGeometry([{"V": V0, "P": P0, "material": m},
+                        {"V": V1 + [0.2, 0.1, 1.5 + gap], "P": P1, "material": m},
+                        {"V": 0.7 * V2 - [1.8 + gap, 0.3, 0.0], "P": P2, "material": None}])
+
+
+@pytest.mark.parametrize("gap", [0.1, 4.0])
+@pytest.mark.parametrize("pec", [True, False])
+@pytest.mark.parametrize("omega", [0.5j, 1.1, 0.8 + 0.2j])
+def test_trace_of_a_displacement_equals_the_trace_of_its_blocks(omega, pec, gap):
+    """Bodies of unequal size, with (gap 0.1) and without near pairs, every axis,
+    real and complex storage: the trace with dM assembled on the device equals the
+    trace with the same gradient blocks put in place on the host.  The blocks
+    are the same numbers, and so is the solve: equal to the last bit."""
+    from gbem._lib import C128, F64
+    from gbem.api import HMatrix
+    G = _three_bodies(pec, gap)
+    off = np.concatenate([[0], np.cumsum([G.NumBFs(s) for s in range(3)])])
+    for dt in (F64, C128) if omega == 0.5j else (C128,):
+        M = G.AssembleBEMMatrix(omega, HMatrix(G, dt))
+        assert M.LUFactorize() == 0
+        for axis in range(3):
+            dM = np.zeros((G.TotalBFs, off[1]), dtype=M.np_dtype, order="F")
+            for s in (1, 2):
+                g = G.AssembleBEMMatrixBlockGradient(0, s, omega, real=dt == F64, components=(axis,))[axis]
+                dM[off[s]:off[s + 1]] = g.T
+            want = M.TraceMInvdM(dM, int(off[1]))
+            assert M.TraceMInvDisplacement(G, omega, axis) == want
+
+
+def test_trace_of_a_displacement_takes_its_own_geometry_only():
+    """The blocks come from the matrix's geometry: another one (fewer regions,
+    other meshes) is refused."""
+    from gbem import RWGGeometry, mesh
+    from gbem.api import Material
+    V, P = mesh.icosphere(0)
+    def geo(shift, m=None):
+        return RWGGeometry([{"V": V, "P": P, "material": m}, {"V": V + [0.0, 0.0, shift], "P": P, "material": m}])
+    G = geo(4.0, Material(2.0))
+    M = G.AssembleBEMMatrix(1.0)
+    assert M.LUFactorize() == 0
+    t = M.TraceMInvDisplacement(G, 1.0)
+    assert M.TraceMInvDisplacement(geo(4.0, Material(2.0)), 1.0) == t
+    for other in (geo(4.0), geo(5.0, Material(2.0)), RWGGeometry([{"V": V, "P": P, "material": Material(2.0)}])):
+        with pytest.raises(ValueError):
+            M.TraceMInvDisplacement(other, 1.0)
