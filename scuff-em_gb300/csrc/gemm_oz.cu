@@ -1,38 +1,55 @@
 // gemm_oz.cu -- the FP64 matrix update on the tensor cores:
 //     C (m x n) -= A (m x k) * B (k x n)
-// for complex128 or real double, column-major, to FP64 accuracy, with
-// tcgen05.mma (kind::f16) on integer slices of the operands (the error-free
+// for complex128 or real double, column-major, to FP64 accuracy entry by entry,
+// with tcgen05.mma (kind::f16) on integer slices of the operands (the error-free
 // splitting of Ozaki, Ogita, Oishi and Rump, "Error-free transformations of
 // matrix multiplication by using fast routines of matrix multiplication and
 // its applications", Numer. Algorithms 59, 2012).
 //
 // Each row of A and each column of B is scaled by the power of two above its
-// largest entry and rounded to a 55-bit fixed-point number, written as seven
+// largest entry and rounded to a 63-bit fixed-point number, written as eight
 // balanced base-256 digits (-128 .. 128, exact in bf16).  The product of two
 // digit matrices is an integer; its FP32 accumulator is exact while it stays
 // within 2^24, that is over 1024 products of at most 2^14.  The pairs (i, j)
 // of slices with i + j = d share the weight 2^-(8d - 2), so they add up in one
 // accumulator, as many pairs as the 1024 products allow; the groups d = 2 .. 9
-// (34 of the 49 pairs) are drained into one 64-bit integer per output, which
-// is rounded to FP64 once (integer arithmetic) and subtracted from C.  What is
-// left is the rounding to 55 bits, 2^-56 of the row's or column's maximum per
-// entry: for a row of L with entries below 1 and a column of U about
-// 2^-53 * 0.24 sqrt(k) of the column's typical entry, an FP64 chain's
-// 2^-53 * 0.3 sqrt(k).  (Without d = 9 it is three times that: the backward
-// error of an LU of normal entries, N = 768, was 1.06e-14 against 5.6e-15 for
-// FP64 chains.)
+// (36 of the 64 pairs) are drained into one 64-bit integer per output, which
+// is rounded to FP64 once (integer arithmetic) and subtracted from C.
 //
-// Measured, k = 256: 30 TFLOP/s FP64 at m = n = 15104 (1000 TFLOP/s of bf16,
-// 55 % of the measured rate) against 0.74 for the SIMT FP64 update; the
-// updates of an N = 3840 LU 6 ms against 194.  Error against long double for
-// normal entries, k = 256: 4.9e-18 of |a| |b| root mean square, FP64 FMAs
-// 4.3e-17; backward error of an LU of normal entries, N = 768: 3.3e-15 against
-// 5.6e-15 with FP64 updates (LAPACK 6.3e-15).
+// What fixed point leaves out is a fraction of (row maximum) x (column maximum),
+// where FP64 products lose a fraction of each |a_ik b_kj|.  The two differ where
+// a row's large entries meet a column's small ones: rows of different scale, a
+// weakly coupled set of unknowns, a dielectric at low frequency (electric and
+// magnetic currents in turn).  So a ninth slice holds the entries' sizes as
+// ordinary bf16 numbers, and its product, the first of a tile, is every output's
+// own sum S = sum |a_ik| |b_kj| in units of the two maxima.  An output with
+//   S >= 1        is summed in units of 2^-53;
+//   S <  1        in units of 2^-62 (modulo 2^64: the sum is below 2^62 of them);
+//   S <  2^-8     makes its tile add the pairs of d = 10, last;
+//   0 < S < 2^-10 is left to FP64 multiplications, by the draining warps.
+// What remains is 2^-51 of sum |a_ik| |b_kj| at most (random digits); FP64 chains
+// of 128 to 512 products lose up to 2^-49 of it (spheres, cubes).  The limit 2^-12
+// for FP64 multiplications left 2^-49.7 and saved 1 % of the Casimir integrand,
+// 2^-9 cost it 3 %.  Measured, N = 400, largest |P A - L U| / |L||U| of an LU, in
+// units of 2^-53:
+//                                          seven digits alone   now   LAPACK
+//   normal entries                                  1.8         1.8     1.9
+//   rows scaled over 1e12, the smallest first       300         2.1     1.7
+//   over 1e18, 1e30                             2.3e4, 7.7e7  2.1, 2.3  1.8, 2.1
+//   two sets coupled by 1e-6, 1e-12             5.9e4, 8.2e10 2.8, 2.5  3.3, 2.8
+// and of an update by itself, wide ranges of entries, k = 7 .. 256: 2 to 9, where
+// chains of FP64 FMAs have 2 to 15.  Error for normal entries, k = 256: 4.4e-18 of
+// |a| |b| root mean square, FP64 FMAs 4.3e-17; backward error of an LU of normal
+// entries, N = 768: 3.6e-15 (LAPACK 6.3e-15, FP64 updates 5.6e-15).
+//
+// Time, k = 256 complex: m = n = 3584 1.01 ms, 26 TFLOP/s FP64 (0.87 with seven
+// digits alone), against 0.74 TFLOP/s for the SIMT FP64 update; 1653 308 us (267);
+// 480 x 64, k = 64 35 us (31).
 //
 // What bounds it: the instructions of the single-thread TMA and MMA issuers
-// per k-step at every size, and the tensor pipe (34 bf16 products in place of
+// per k-step at every size, and the tensor pipe (37 bf16 products in place of
 // one FP64 one) not far behind.  The FP64 pipe it replaces runs 2 FMAs per
-// cycle and SM.
+// cycle and SM; outputs left to it take as long as gemm_simt took.
 //
 // A row or column that holds an infinity or NaN makes its row or column of C
 // NaN (the digits are zero there).
@@ -46,8 +63,9 @@
 namespace gbem {
 
 namespace oz {
-constexpr int NS = 7;             // slices (base-256 digits)
-constexpr int DMAX = 9;           // largest i + j of the slice pairs taken
+constexpr int NS = 8;             // slices (base-256 digits); slice NS + 1 holds the sizes
+constexpr int STEPS = 10;         // groups of slice pairs: sizes, d = 9 .. 2, and d = 10 where it is called for
+constexpr float S_FINE = 1.0f, S_MORE = 1.0f / 256, S_FP64 = 1.0f / 1024;  // see above
 constexpr int KMAX = 512;         // real products per output and slice pair
 constexpr int ACC_TERMS = 1024;   // products that add up exactly: 1024 * 2^14 = 2^24
 constexpr int BM = 128, BK = 64;
@@ -65,7 +83,7 @@ template <int BN> struct Tile {
   static constexpr int A_BYTES = KB * A_BLK, B_BYTES = KB * B_BLK, STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static constexpr uint32_t IDESC = idesc_bf16(BM, BN);
-  static_assert((2 * STAGES + 5) * 8 + 4 <= 256, "barrier area");
+  static_assert((2 * STAGES + 6) * 8 + 4 <= 256, "barrier area");
   static_assert(B_BLK % 1024 == 0, "swizzle atoms");
 };
 constexpr int EXP_BAD = 1 << 20;  // scale exponent of a row or column that is not finite
@@ -75,25 +93,41 @@ constexpr int VECS = 16;          // rows of A (columns of B) per packing CTA
 // exponent field (at least 1) of a double's high word
 __device__ __forceinline__ int exp_field(unsigned hi) { return max((int)((hi >> 20) & 0x7ffu), 1); }
 
-// |x| < 2^(F - 1022) as a signed 55-bit fixed-point number: round(x 2^(55 - (F - 1022)))
-__device__ __forceinline__ long long fixed55(double x, int F) {
+// |x| < 2^(F - 1022) as a signed 63-bit fixed-point number: round(x 2^(63 - (F - 1022)))
+__device__ __forceinline__ long long fixed63(double x, int F) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const int raw = (int)((b >> 52) & 0x7ffu), f = max(raw, 1);
   unsigned long long M = b & 0xfffffffffffffull;
   if (raw) M |= 1ull << 52;
   const int d = F - f;  // >= 0
   unsigned long long q;
-  if (d <= 2) q = M << (2 - d);
-  else if (d < 58) q = (M + (1ull << (d - 3))) >> (d - 2);
+  if (d <= 10) q = M << (10 - d);
+  else if (d < 66) q = (M + (1ull << (d - 11))) >> (d - 10);
   else q = 0;
   return (long long)b < 0 ? -(long long)q : (long long)q;
+}
+
+// its size as a bf16 number in units of 2^(F - 1022); no entry but zero is zero,
+// so that a sum of sizes is zero only where every product is
+__device__ __forceinline__ unsigned short size_bf16(double x, long long q) {
+  const float v = (float)(unsigned long long)(q < 0 ? -q : q) * 0x1p-63f;
+  const bool zero = (__double_as_longlong(x) << 1) == 0;
+  return zero ? (unsigned short)0 : __bfloat16_as_ushort(__float2bfloat16_rn(fmaxf(v, 0x1p-60f)));
+}
+
+// step of a tile (0: the sizes; 1 .. 8: d = 9 .. 2; 9: d = 10) -> its slice pairs (i, j), i0 <= i < i1, j = sum - i
+struct OzGroup { int i0, i1, sum; };
+__device__ __forceinline__ OzGroup oz_group(int step) {
+  if (step == 0) return {oz::NS + 1, oz::NS + 2, 2 * oz::NS + 2};
+  const int d = step < oz::STEPS - 1 ? 10 - step : 10;
+  return {max(1, d - oz::NS), min(oz::NS + 1, d), d};
 }
 
 // The digits of A's rows (part 0) and B's columns (part 1), one launch: CTAs
 // [0, na) take 16 rows of A each, the others 16 columns of B.  The vectors
 // are staged in shared memory (coalesced), their largest exponent is found,
-// and each vector's digits are written slice by slice, out[s][row][Kp],
-// zero beyond kreal.  A complex row of A is [Re | Im]; a complex column j of
+// and each vector's digits and sizes are written slice by slice,
+// out[s][row][Kp], zero beyond kreal.  A complex row of A is [Re | Im]; a complex column j of
 // B makes rows 2j = [Re | -Im] and 2j + 1 = [Im | Re], whose products with it
 // are the real and imaginary part.
 template <bool CPLX>
@@ -154,7 +188,9 @@ __global__ void __launch_bounds__(256) oz_pack(const double* A, long long lda, i
     const int r = q / groups, g = q - r * groups;
     const int v = rpv == 2 ? r >> 1 : r, odd = rpv == 2 ? r & 1 : 0;
     const int F = vexp[v];
-    long long b[4];  // bytes 0..5: digits 7..2 plus 128; above: the top digit
+    unsigned long long b[4];  // bytes 0..6: digits 8..2 plus 128
+    int top[4];
+    unsigned short sz[4];
     unsigned neg = 0;
 #pragma unroll
     for (int e = 0; e < 4; e++) {
@@ -172,15 +208,18 @@ __global__ void __launch_bounds__(256) oz_pack(const double* A, long long lda, i
       } else if (p < k) {
         x = t[p * 17 + v];
       }
-      b[e] = (F < 0 ? 0 : fixed55(x, F)) + 0x808080808080ll;
+      const long long q = F < 0 ? 0 : fixed63(x, F);
+      b[e] = ((unsigned long long)q & 0xffffffffffffffull) + 0x80808080808080ull;
+      top[e] = (int)(q >> 56) + (int)(b[e] >> 56);
+      sz[e] = F < 0 ? (unsigned short)0 : size_bf16(x, q);
     }
 #pragma unroll
-    for (int s = 0; s < oz::NS; s++) {  // slice s holds digit s + 1 (the top one first)
+    for (int s = 0; s <= oz::NS; s++) {  // slice s holds digit s + 1 (the top one first), the last the sizes
       unsigned short w[4];
 #pragma unroll
       for (int e = 0; e < 4; e++) {
-        const int dg = s == 0 ? (int)(b[e] >> 48) : (int)((b[e] >> (8 * (6 - s))) & 255) - 128;
-        w[e] = (unsigned short)(__float_as_uint((float)((neg >> e) & 1u ? -dg : dg)) >> 16);
+        const int dg = s == 0 ? top[e] : (int)((b[e] >> (8 * (7 - s) & 63)) & 255) - 128;
+        w[e] = s == oz::NS ? sz[e] : (unsigned short)(__float_as_uint((float)((neg >> e) & 1u ? -dg : dg)) >> 16);
       }
       uint2 pk;
       pk.x = (unsigned)w[0] | ((unsigned)w[1] << 16);
@@ -202,17 +241,72 @@ __device__ __forceinline__ double int_to_double(long long T, int e) {
   return a ? __longlong_as_double((long long)b) : 0.0;
 }
 
+// C(row, j) -= sum_k A(row, k) B(k, j) in FP64 for a warp's outputs marked in need
+// (bit c: its real column c; lane: its row).  Many of a column: each lane its own
+// row; few: the lanes share the products of one after the other.
+template <bool CPLX>
+__device__ __noinline__ void oz_fp64(double* C, long long ldc, const double* A, long long lda, const double* B, long long ldb,
+                                     int m, int n, int k, int row, int j0, unsigned need) {
+  constexpr int W = CPLX ? 2 : 1;
+  const int lane = threadIdx.x & 31, row0 = row - lane;
+  auto term = [&](int r, int j, int kk, double& x, double& y) {
+    const double* a = A + W * ((long long)r + (long long)kk * lda);
+    const double* b = B + W * ((long long)kk + (long long)j * ldb);
+    if (CPLX) {
+      const double2 u = *reinterpret_cast<const double2*>(a), v = *reinterpret_cast<const double2*>(b);
+      x = fma(-u.y, v.y, fma(u.x, v.x, x));
+      y = fma(u.y, v.x, fma(u.x, v.y, y));
+    } else {
+      x = fma(*a, *b, x);
+    }
+  };
+  auto put = [&](int r, int j, double x, double y) {
+    double* p = C + W * ((long long)r + (long long)j * ldc);
+    p[0] -= x;
+    if (CPLX) p[W - 1] -= y;
+  };
+  for (int c = 0; c < 32; c += W) {
+    const int j = j0 + c / W;
+    if (j >= n) break;
+    const bool mine = (need >> c) & (W == 2 ? 3u : 1u);
+    unsigned rows = __ballot_sync(0xffffffffu, mine);
+    if (__popc(rows) > 8) {
+      if (mine) {
+        double x = 0.0, y = 0.0;
+#pragma unroll 4
+        for (int kk = 0; kk < k; kk++) term(row, j, kk, x, y);
+        put(row, j, x, y);
+      }
+      __syncwarp();
+    } else {
+      for (; rows; rows &= rows - 1) {
+        const int r = row0 + __ffs(rows) - 1;
+        double x = 0.0, y = 0.0;
+        for (int kk = lane; kk < k; kk += 32) term(r, j, kk, x, y);
+        for (int o = 16; o > 0; o >>= 1) {
+          x += __shfl_xor_sync(0xffffffffu, x, o);
+          if (CPLX) y += __shfl_xor_sync(0xffffffffu, y, o);
+        }
+        if (lane == 0) put(r, j, x, y);
+      }
+    }
+  }
+}
+
 // One CTA per SM walks the 128 x BN output tiles (columns counted as reals;
 // m fastest, so the CTAs of a wave share their B tile).  Warp 0: TMA producer;
 // warp 1: TMEM and MMA issue; warps 2-9: drain.  A tile's accumulators follow
 // one another through two BN-column TMEM buffers: the MMAs of the next run
 // while the drain warps add the last one into their 64-bit integers (one row
-// and BN / 2 columns per thread).  pairs: slice pairs per accumulator.
+// and BN / 2 columns per thread).  The sizes come first: by the end of a tile its
+// draining warps have long decided whether d = 10 follows.  pairs: slice pairs
+// per accumulator.  A, B: the operands themselves, for the outputs left to FP64.
 template <bool CPLX, int BN>
 __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__ CUtensorMap mapA,
                                                           const __grid_constant__ CUtensorMap mapB, double* C,
-                                                          long long ldc, const int* ea, const int* eb, int m, int n,
-                                                          int kblocks, int pairs, int mt, int ntiles,
+                                                          long long ldc, const double* A, long long lda,
+                                                          const double* B, long long ldb, const int* ea,
+                                                          const int* eb, int m, int n, int k, int kblocks, int pairs, int mt, int ntiles,
                                                           int* wait_error) {
   pdl_wait();
   pdl_trigger();
@@ -225,8 +319,10 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
   uint64_t* acc_full = empty + TL::STAGES;  // [2] MMA -> drain
   uint64_t* acc_empty = acc_full + 2;       // [2] drain -> MMA (8 warp arrivals)
   uint64_t* done = acc_empty + 2;           // all MMAs retired
-  uint32_t* tmem_slot = (uint32_t*)(done + 1);
+  uint64_t* decided = done + 1;             // drain -> all: s_more of this tile is final (8 warp arrivals)
+  uint32_t* tmem_slot = (uint32_t*)(decided + 1);
   __shared__ int s_fail, s_skip;
+  __shared__ int s_more[2];  // by the parity of a CTA's tile number: the last tile (from 1) that takes d = 10
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = CPLX ? 2 * n : n;  // real output columns
   const int kbx = min(oz::KB, kblocks);
@@ -235,6 +331,8 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
     for (int s = 0; s < TL::STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }
     mbar_init(done, 1);
+    mbar_init(decided, 8);
+    s_more[0] = s_more[1] = 0;
     s_fail = 0;
     // once a CTA of this call has given up a wait, the rest do no work (read
     // once, so that the whole CTA takes the same way)
@@ -257,10 +355,15 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
       RingPos<TL::STAGES> r;
       int issued = 0;  // stages in use
       bool ok = true;
-      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+      for (int t = blockIdx.x, it = 0; t < ntiles && ok; t += gridDim.x, it++) {
         const int ya = (t % mt) * oz::BM, yb = (t / mt) * BN;
-        for (int d = oz::DMAX; d >= 2 && ok; d--)
-          for (int i = max(1, d - oz::NS); i <= min(oz::NS, d - 1) && ok; i++)
+        for (int step = 0; step < oz::STEPS && ok; step++) {
+          if (step == oz::STEPS - 1) {
+            if (!mbar_wait(decided, (uint32_t)(it & 1))) { atomicExch(&s_fail, 1); ok = false; }
+            if (!ok || *(volatile int*)&s_more[it & 1] != it + 1) break;
+          }
+          const OzGroup g = oz_group(step);
+          for (int i = g.i0; i < g.i1 && ok; i++)
             for (int kb = 0; kb < kblocks; kb += kbx, r.next()) {
               // a fresh barrier's previous phase counts as complete
               if (!mbar_wait(&empty[r.s], r.phase ^ 1u)) {
@@ -271,9 +374,10 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
               unsigned char* sa = tiles + r.s * TL::STAGE_BYTES;
               mbar_arrive_expect_tx(&full[r.s], kbx * (TL::A_BLK + TL::B_BLK));
               tma_load_3d(sa, &mapA, &full[r.s], 0, (i - 1) * m + ya, kb);
-              tma_load_3d(sa + TL::A_BYTES, &mapB, &full[r.s], 0, (d - i - 1) * nb + yb, kb);
+              tma_load_3d(sa + TL::A_BYTES, &mapB, &full[r.s], 0, (g.sum - i - 1) * nb + yb, kb);
               issued = min(issued + 1, TL::STAGES);
             }
+        }
       }
       // no TMA write may still be in flight when the CTA exits: the last
       // pass of every stage used
@@ -289,11 +393,15 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
       bool ok = true;
       int u = 0;
       const uint64_t desc0 = sdesc_sw128(smem_u32(tiles));  // addresses count 16 bytes in the low bits
-      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x)
-        for (int d = oz::DMAX; d >= 2 && ok; d--) {
-          const int ie = min(oz::NS + 1, d);
-          for (int i0 = max(1, d - oz::NS); i0 < ie && ok; i0 += pairs, u++) {
-            const int acc = u & 1, i1 = min(i0 + pairs, ie);
+      for (int t = blockIdx.x, it = 0; t < ntiles && ok; t += gridDim.x, it++)
+        for (int step = 0; step < oz::STEPS && ok; step++) {
+          if (step == oz::STEPS - 1) {
+            if (!mbar_wait(decided, (uint32_t)(it & 1))) { atomicExch(&s_fail, 1); ok = false; }
+            if (!ok || *(volatile int*)&s_more[it & 1] != it + 1) break;
+          }
+          const OzGroup g = oz_group(step);
+          for (int i0 = g.i0; i0 < g.i1 && ok; i0 += pairs, u++) {
+            const int acc = u & 1, i1 = min(i0 + pairs, g.i1);
             if (u >= 2 && !mbar_wait(&acc_empty[acc], (uint32_t)(((u >> 1) - 1) & 1))) {
               atomicExch(&s_fail, 1);
               ok = false;
@@ -326,21 +434,30 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
     // warp % 4 selects the TMEM lane quarter, the two warps of a quarter
     // split the 128 columns
     const int q = warp & 3, half = (warp - 2) >> 2;
-    constexpr int CH = CW < 32 ? CW : 32;
+    constexpr int CH = 16, NM = (CW + 31) / 32;
     int u = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+    for (int t = blockIdx.x, it = 0; t < ntiles && ok; t += gridDim.x, it++) {
       const int tm = t % mt, tn = t / mt;
-      const int row = tm * oz::BM + q * 32 + lane;
-      long long T[CW];
+      const int row = tm * oz::BM + q * 32 + lane, col0 = tn * BN + half * CW;  // col0: a real column
+      unsigned long long T[CW];  // modulo 2^64
+      unsigned fine[NM], low[NM];    // by column
+#pragma unroll
+      for (int h = 0; h < NM; h++) fine[h] = low[h] = 0;
 #pragma unroll
       for (int c = 0; c < CW; c++) T[c] = 0;
-      for (int d = oz::DMAX; d >= 2 && ok; d--) {
-        // units 2^-70 for d = 9, 2^-62 down to d = 4, then 2^-53: every sum
-        // stays below 2^63
-        const int sh = d >= 8 ? 0 : (d >= 4 ? 8 * (8 - d) : (d == 3 ? 31 : 39));
-        const int ie = min(oz::NS + 1, d);
-        for (int i0 = max(1, d - oz::NS); i0 < ie; i0 += pairs, u++) {
+      for (int step = 0; step < oz::STEPS && ok; step++) {
+        if (step == oz::STEPS - 1) {
+          ok = mbar_wait(decided, (uint32_t)(it & 1));
+          if (!ok) atomicExch(&s_fail, 1);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok || *(volatile int*)&s_more[it & 1] != it + 1) break;
+        }
+        const OzGroup g = oz_group(step);
+        // units: 2^-70 for d = 9, 2^-62 down to d = 4, then 2^-53, for a fine
+        // output still 2^-62; every sum of the former stays below 2^63
+        const int d = g.sum, sh = d >= 8 ? 0 : (d >= 4 ? 8 * (8 - d) : (d == 3 ? 31 : 39)), shf = d <= 3 ? sh + 9 : sh;
+        for (int i0 = g.i0; i0 < g.i1; i0 += pairs, u++) {
           const int acc = u & 1;
           ok = mbar_wait(&acc_full[acc], (uint32_t)((u >> 1) & 1));
           if (!ok) atomicExch(&s_fail, 1);
@@ -351,28 +468,60 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
 #pragma unroll
           for (int c0 = 0; c0 < CW; c0 += CH) {
             float v[CH];
-            if constexpr (CH == 32) tmem_ld32(tb + (uint32_t)c0, v);
-            else tmem_ld16(tb + (uint32_t)c0, v);
+            tmem_ld16(tb + (uint32_t)c0, v);
             if (c0 + CH == CW) {  // this warp's last read of the buffer
               tc_fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive(&acc_empty[acc]);
             }
+            if (step == 0) {
+              // (a zero sum needs nothing; rows beyond m hold other slices)
+              float least = oz::S_FINE;
 #pragma unroll
-            for (int c = 0; c < CH; c++) T[c0 + c] += (long long)__float2int_rn(v[c]) << sh;
+              for (int c = 0; c < CH; c++) {
+                if (v[c] < oz::S_FINE) fine[c0 / 32] |= 1u << (c0 + c) % 32;
+                least = fminf(least, v[c] > 0.0f && col0 + c0 + c < nb ? v[c] : oz::S_FINE);
+              }
+              if (row < m && least < oz::S_FP64) {
+#pragma unroll
+                for (int c = 0; c < CH; c++)
+                  if (v[c] < oz::S_FP64 && v[c] > 0.0f) low[c0 / 32] |= 1u << (c0 + c) % 32;
+              }
+              if (__any_sync(0xffffffffu, row < m && least < oz::S_MORE) && lane == 0) atomicMax(&s_more[it & 1], it + 1);
+            } else if (step == oz::STEPS - 1) {
+#pragma unroll
+              for (int c = 0; c < CH; c++)
+                if ((fine[c0 / 32] >> (c0 + c) % 32) & 1) T[c0 + c] += (unsigned long long)(long long)((__float2int_rn(v[c]) + (1 << 15)) >> 16);
+            } else if (sh == shf) {
+#pragma unroll
+              for (int c = 0; c < CH; c++) T[c0 + c] += (unsigned long long)(long long)__float2int_rn(v[c]) << sh;
+            } else {
+#pragma unroll
+              for (int c = 0; c < CH; c++)
+                T[c0 + c] += (unsigned long long)(long long)__float2int_rn(v[c]) << (((fine[c0 / 32] >> (c0 + c) % 32) & 1) ? shf : sh);
+            }
           }
         }
-        if (d == 9 || d == 4) {
-          const int down = d == 9 ? 8 : 9;
+        if (!ok) break;
+        if (step == 0) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(decided);
+        }
+        if (d == 9) {
 #pragma unroll
-          for (int c = 0; c < CW; c++) T[c] = (T[c] + (1 << (down - 1))) >> down;
+          for (int c = 0; c < CW; c++) T[c] = (unsigned long long)(((long long)T[c] + 128) >> 8);
+        }
+        if (d == 4) {
+#pragma unroll
+          for (int c = 0; c < CW; c++)
+            if (!((fine[c / 32] >> (c % 32)) & 1)) T[c] = (unsigned long long)(((long long)T[c] + 256) >> 9);
         }
       }
       if (!ok) break;
+      constexpr int W = CPLX ? 2 : 1;
+      const int j0 = col0 / W;
       if (row < m) {
         const int er = ea[row];
-        constexpr int W = CPLX ? 2 : 1;
-        const int j0 = (tn * BN + half * CW) / W;
 #pragma unroll
         for (int c = 0; c < CW; c += W) {
           const int j = j0 + c / W;
@@ -386,20 +535,25 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
           } else {
             z[0] = *p;
           }
-          if (e > -1000 && e < 960) {
+          if (e > -990 && e < 960) {
 #pragma unroll
-            for (int w = 0; w < W; w++) z[w] -= int_to_double(T[c + w], e);
+            for (int w = 0; w < W; w++) z[w] -= int_to_double((long long)T[c + w], e - (((fine[c / 32] >> ((c + w) % 32)) & 1) ? 9 : 0));
           } else if (er == oz::EXP_BAD || ec == oz::EXP_BAD) {
 #pragma unroll
             for (int w = 0; w < W; w++) z[w] = __longlong_as_double(0x7ff8000000000000ll);
           } else {
 #pragma unroll
-            for (int w = 0; w < W; w++) z[w] -= ldexp((double)T[c + w], e);
+            for (int w = 0; w < W; w++) z[w] -= ldexp((double)(long long)T[c + w], e - (((fine[c / 32] >> ((c + w) % 32)) & 1) ? 9 : 0));
           }
-          if (CPLX) *reinterpret_cast<double2*>(p) = make_double2(z[0], z[W - 1]);
-          else *p = z[0];
+          if (!((low[c / 32] >> (c % 32)) & (W == 2 ? 3u : 1u))) {
+            if (CPLX) *reinterpret_cast<double2*>(p) = make_double2(z[0], z[W - 1]);
+            else *p = z[0];
+          }
         }
       }
+#pragma unroll
+      for (int h = 0; h < NM; h++)
+        if (__any_sync(0xffffffffu, low[h] != 0)) oz_fp64<CPLX>(C, ldc, A, lda, B, ldb, m, n, k, row, j0 + h * 32 / W, low[h]);
     }
   }
   tc_fence_before();
@@ -415,7 +569,7 @@ static size_t oz_round(size_t x) { return (x + 1023) & ~(size_t)1023; }
 
 size_t oz_gemm_ws_bytes(int m, int n, int k, bool cplx) {
   const size_t Kp = ((size_t)(cplx ? 2 * k : k) + 63) / 64 * 64, nb = cplx ? 2 * (size_t)n : (size_t)n;
-  return oz_round(oz::NS * (size_t)m * Kp * 2) + oz_round(oz::NS * nb * Kp * 2) + oz_round(4 * (size_t)m) +
+  return oz_round((oz::NS + 1) * (size_t)m * Kp * 2) + oz_round((oz::NS + 1) * nb * Kp * 2) + oz_round(4 * (size_t)m) +
          oz_round(4 * (size_t)n) + 1024;
 }
 
@@ -426,13 +580,14 @@ template <bool CPLX>
 static bool update(double* C, long long ldc, const double* A, long long lda, const double* B, long long ldb, int m,
                    int n, int k, void* ws, size_t ws_bytes, int* wait_error, cudaStream_t s, cudaError_t* err) {
   *err = cudaSuccess;
+  if (!tensor_updates()) return false;  // GBEM_LU_TC=0
   if (m <= 0 || n <= 0 || k <= 0) return true;
   const int kreal = CPLX ? 2 * k : k;
   if (kreal > oz::KMAX || !ws || ws_bytes < oz_gemm_ws_bytes(m, n, k, CPLX)) return false;
   const int Kp = (kreal + 63) / 64 * 64, nb = CPLX ? 2 * n : n;
   unsigned char* w = (unsigned char*)(((uintptr_t)ws + 1023) & ~(uintptr_t)1023);
-  __nv_bfloat16* pa = (__nv_bfloat16*)w; w += oz_round(oz::NS * (size_t)m * Kp * 2);
-  __nv_bfloat16* pb = (__nv_bfloat16*)w; w += oz_round(oz::NS * (size_t)nb * Kp * 2);
+  __nv_bfloat16* pa = (__nv_bfloat16*)w; w += oz_round((oz::NS + 1) * (size_t)m * Kp * 2);
+  __nv_bfloat16* pb = (__nv_bfloat16*)w; w += oz_round((oz::NS + 1) * (size_t)nb * Kp * 2);
   int* ea = (int*)w; w += oz_round(4 * (size_t)m);
   int* eb = (int*)w;
   const int na = (m + oz::VECS - 1) / oz::VECS, nbk = (n + oz::VECS - 1) / oz::VECS;
@@ -442,21 +597,21 @@ static bool update(double* C, long long ldc, const double* A, long long lda, con
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int mt = (m + oz::BM - 1) / oz::BM;
   // narrow tiles where one wave of them covers C: a tile's k-steps and drain
-  // are then shorter (m = 3584, n = k = 32: 23 us with packing, 35 with
+  // are then shorter (m = 3584, n = k = 32, seven digits: 23 us with packing, 35 with
   // 128 columns); in two waves they lose (m = n = 704, k = 256: 170 against 113)
   const int bn = mt * ((nb + 31) / 32) <= nsm ? 32 : 128;
   const auto kernel = bn == 32 ? oz_gemm_kernel<CPLX, 32> : oz_gemm_kernel<CPLX, 128>;
   const int smem = bn == 32 ? oz::Tile<32>::SMEM_BYTES : oz::Tile<128>::SMEM_BYTES;
   if ((*err = allow_max_smem(kernel)) != cudaSuccess) return false;
   CUtensorMap ma, mb;
-  if (!make_bf16_map(&ma, pa, (long long)oz::NS * m, Kp, oz::BM, std::min(oz::KB, Kp / oz::BK)) ||
-      !make_bf16_map(&mb, pb, (long long)oz::NS * nb, Kp, bn, std::min(oz::KB, Kp / oz::BK)))
+  if (!make_bf16_map(&ma, pa, (oz::NS + 1LL) * m, Kp, oz::BM, std::min(oz::KB, Kp / oz::BK)) ||
+      !make_bf16_map(&mb, pb, (oz::NS + 1LL) * nb, Kp, bn, std::min(oz::KB, Kp / oz::BK)))
     return false;
   *err = launch_pdl(oz_pack<CPLX>, dim3(na + nbk), dim3(256), (size_t)k * 17 * (CPLX ? 16 : 8), s, A, lda, m, B, ldb, n,
                     k, Kp, na, pa, pb, ea, eb);
   if (*err != cudaSuccess) return false;
   const int ntiles = mt * ((nb + bn - 1) / bn);
-  *err = launch_pdl(kernel, dim3(std::min(ntiles, nsm)), dim3(320), (size_t)smem, s, ma, mb, C, ldc, ea, eb, m, n,
+  *err = launch_pdl(kernel, dim3(std::min(ntiles, nsm)), dim3(320), (size_t)smem, s, ma, mb, C, ldc, A, lda, B, ldb, ea, eb, m, n, k,
                     Kp / oz::BK, oz::ACC_TERMS / kreal, mt, ntiles, wait_error);
   return *err == cudaSuccess;
 }

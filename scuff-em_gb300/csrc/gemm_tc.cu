@@ -298,20 +298,22 @@ size_t tc_gemm_ws_bytes(int m, int n, int k) {
   return ((size_t)m + 2 * (size_t)n) * Kp * 2 + 4096;
 }
 
-static int g_tc_mode = -1;  // -1 unknown, 0 disabled, 1 enabled
+// GBEM_LU_TC=0: no tensor-core updates, complex FP32 or FP64
+bool tensor_updates() {
+  static const bool on = [] {
+    const char* e = getenv("GBEM_LU_TC");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
 static thread_local int tl_tc_off = 0;  // this host thread's LU takes the FP32 SIMT updates
 
-void tc_gemm_set_enabled(int on) { g_tc_mode = on ? 1 : 0; }
 void tc_gemm_thread_off(int off) { tl_tc_off = off; }
 
 bool tc_gemm_update(cx<float>* C, long long ldc, const cx<float>* A, long long lda, const cx<float>* B, long long ldb,
                     int m, int n, int k, void* ws, size_t ws_bytes, int* wait_error, cudaStream_t s, cudaError_t* err) {
   *err = cudaSuccess;
-  if (g_tc_mode < 0) {
-    const char* e = getenv("GBEM_LU_TC");
-    g_tc_mode = (e && e[0] == '0') ? 0 : 1;
-  }
-  if (g_tc_mode == 0 || tl_tc_off) return false;
+  if (!tensor_updates() || tl_tc_off) return false;
   if (m <= 0 || n <= 0 || k <= 0) return true;
   int Kp = pad64(6 * k);
   size_t need = ((size_t)m + 2 * (size_t)n) * Kp * 2;

@@ -114,6 +114,7 @@ constexpr uint32_t idesc_bf16(int m, int n) {
 // and kbox blocks of 64 columns (block after block in shared memory, 128-byte
 // swizzle); coordinates {0, row, block}
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
+bool tensor_updates();  // false: GBEM_LU_TC=0
 bool make_bf16_map(CUtensorMap* map, const void* ptr, long long rows, int cols, int box_rows, int kbox);
 
 }  // namespace gbem

@@ -184,6 +184,104 @@ def test_leaf_lanes_per_row(N):
     _check_backward(A, LU, piv)
 
 
+def _componentwise(A, LU, piv):
+    """max |P A - L U| / (|L| |U|) over sampled rows, in extended precision."""
+    N = A.shape[0]
+    perm = np.arange(N)
+    for i, p in enumerate(piv):
+        perm[[i, p]] = perm[[p, i]]
+    rows = np.unique(np.concatenate([np.linspace(0, N - 1, 24).astype(int), np.arange(max(0, N - 8), N)]))
+    ext = np.longdouble if not np.iscomplexobj(A) else np.clongdouble
+    L, R = (np.tril(LU, -1) + np.eye(N))[rows].astype(ext), np.triu(LU).astype(ext)
+    scale = np.abs(L) @ np.abs(R)
+    err = np.abs(A[perm][rows].astype(ext) - L @ R)
+    return float((err[scale > 0] / scale[scale > 0]).max())
+
+
+def _graded(kind, N, rng, real):
+    A = rng.standard_normal((N, N))
+    if not real:
+        A = A + 1j * rng.standard_normal((N, N))
+    if kind[0] == "rows":        # row scales spread evenly, the smallest first
+        return A * 10.0 ** np.linspace(-kind[1], 0.0, N)[:, None]
+    if kind[0] == "both":
+        s = 10.0 ** rng.uniform(-kind[1], 0.0, N)
+        return A * s[:, None] * rng.permutation(s)
+    if kind[0] == "coupled":     # two sets of unknowns in turn, weakly coupled
+        i = np.arange(N)
+        return A * np.where((i[:, None] + i) % 2, 10.0 ** -kind[1], 1.0)
+    if kind[0] == "entries":
+        return A * 10.0 ** rng.uniform(-kind[1], 0.0, (N, N))
+    i = np.arange(N)             # "arrow": zero except a band, a full row and a full column
+    return A * ((np.abs(i[:, None] - i) < 40) | (i[:, None] > N - 4) | (i > N - 4)) * 10.0 ** np.linspace(-kind[1], 0.0, N)[:, None]
+
+
+@pytest.mark.parametrize("real", [False, True])
+@pytest.mark.parametrize("kind", [("rows", 0), ("rows", 12), ("rows", 18), ("rows", 30), ("both", 20), ("coupled", 2),
+                                  ("coupled", 6), ("coupled", 12), ("entries", 8), ("arrow", 18)])
+def test_factor_is_as_accurate_as_lapack_entry_by_entry(kind, real):
+    """|P A - L U| against |L| |U|, entry by entry, where rows, columns or
+    blocks differ in scale: within eight times LAPACK's own factorisation of the
+    same matrix (another order of the same FP64 sums) and eight roundings."""
+    import scipy.linalg as sl
+    N = 400
+    A = _graded(kind, N, np.random.default_rng(int(kind[1]) + 100 * real), real)
+    lu_ref, piv_ref = sl.lu_factor(A)
+    ref = _componentwise(A, lu_ref, piv_ref)
+    if real:
+        from gbem._lib import F64
+        from gbem.api import HMatrix
+        M = HMatrix(_strip(N), F64)
+        M.set(A)
+        assert M.LUFactorize() == 0
+        LU, piv = M.numpy(), M.ipiv - 1
+    else:
+        LU, piv = _factor(A)
+    got = _componentwise(A, LU, piv)
+    print("componentwise error / u: %.2f (LAPACK %.2f)" % (got / U, ref / U))
+    assert got <= 8 * ref + 8 * U
+
+
+def test_wide_tiles_are_as_accurate_as_lapack_entry_by_entry():
+    """The same where the trailing update takes 128-column tiles (N = 1300),
+    some of them with graded rows, some with even ones, a ragged last one."""
+    import scipy.linalg as sl
+    N = 1300
+    rng = np.random.default_rng(5)
+    A = rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))
+    A[:700] *= 10.0 ** np.linspace(-18.0, 0.0, 700)[:, None]
+    lu_ref, piv_ref = sl.lu_factor(A)
+    LU, piv = _factor(A)
+    got, ref = _componentwise(A, LU, piv), _componentwise(A, lu_ref, piv_ref)
+    print("componentwise error / u: %.2f (LAPACK %.2f)" % (got / U, ref / U))
+    assert got <= 8 * ref + 8 * U
+
+
+_NO_TENSOR = r"""
+import sys
+sys.path[:0] = [sys.argv[1], sys.argv[1] + "/tests", sys.argv[1] + "/scuff-em_gb300"]
+import numpy as np, scipy.linalg as sl
+import test_gpu_lu64 as t
+A = t._graded(("rows", 18), 400, np.random.default_rng(1), False)
+LU, piv = t._factor(A)
+assert t._componentwise(A, LU, piv) <= 8 * t._componentwise(A, *sl.lu_factor(A)) + 8 * t.U
+np.save(sys.argv[2], LU)
+"""
+
+
+def test_tensor_updates_can_be_switched_off(tmp_path):
+    """GBEM_LU_TC=0 takes every update in FP64 multiplications: as accurate, and
+    not the same last bits as the slices'."""
+    import os
+    import subprocess
+    import sys
+    repo = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for tc in ("0", "1"):
+        subprocess.run([sys.executable, "-c", _NO_TENSOR, repo, str(tmp_path / ("lu%s.npy" % tc))],
+                       env=dict(os.environ, GBEM_LU_TC=tc), check=True, timeout=600)
+    assert not np.array_equal(np.load(tmp_path / "lu0.npy"), np.load(tmp_path / "lu1.npy"))
+
+
 @pytest.mark.parametrize("real", [False, True])
 @pytest.mark.parametrize("power", [-530, -520, -505, 505, 520, 900])
 def test_pivots_of_extreme_size(power, real):
