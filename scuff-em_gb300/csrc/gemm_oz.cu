@@ -7,44 +7,48 @@
 // its applications", Numer. Algorithms 59, 2012).
 //
 // Each row of A and each column of B is scaled by the power of two above its
-// largest entry and rounded to a 63-bit fixed-point number, written as eight
+// largest entry and rounded to a 71-bit fixed-point number, written as nine
 // balanced base-256 digits (-128 .. 128, exact in bf16).  The product of two
 // digit matrices is an integer; its FP32 accumulator is exact while it stays
 // within 2^24, that is over 1024 products of at most 2^14.  The pairs (i, j)
 // of slices with i + j = d share the weight 2^-(8d - 2), so they add up in one
 // accumulator, as many pairs as the 1024 products allow; the groups d = 2 .. 9
-// (36 of the 64 pairs) are drained into one 64-bit integer per output, which
-// is rounded to FP64 once (integer arithmetic) and subtracted from C.
+// (36 pairs) are drained into one 64-bit integer per output, which is rounded to
+// FP64 once (integer arithmetic) and subtracted from C.
 //
 // What fixed point leaves out is a fraction of (row maximum) x (column maximum),
 // where FP64 products lose a fraction of each |a_ik b_kj|.  The two differ where
 // a row's large entries meet a column's small ones: rows of different scale, a
-// weakly coupled set of unknowns, a dielectric at low frequency (electric and
-// magnetic currents in turn).  So a ninth slice holds the entries' sizes as
+// weakly coupled set of unknowns, low frequencies (of a dielectric, electric and
+// magnetic currents in turn).  So one more slice holds the entries' sizes as
 // ordinary bf16 numbers, and its product, the first of a tile, is every output's
-// own sum S = sum |a_ik| |b_kj| in units of the two maxima.  An output with
-//   S >= 1        is summed in units of 2^-53;
-//   S <  1        in units of 2^-62 (modulo 2^64: the sum is below 2^62 of them);
-//   S <  2^-8     makes its tile add the pairs of d = 10, last;
-//   0 < S < 2^-10 is left to FP64 multiplications, by the draining warps.
-// What remains is 2^-51 of sum |a_ik| |b_kj| at most (random digits); FP64 chains
-// of 128 to 512 products lose up to 2^-49 of it (spheres, cubes).  The limit 2^-12
-// for FP64 multiplications left 2^-49.7 and saved 1 % of the Casimir integrand,
-// 2^-9 cost it 3 %.  Measured, N = 400, largest |P A - L U| / |L||U| of an LU, in
-// units of 2^-53:
+// own sum S = sum |a_ik| |b_kj| in units of the two maxima.  Outputs with
+//   S >= 1      are summed in units of 2^-53, with
+//   S <  1      in units of 2^-62 (modulo 2^64: the sum is below 2^62 of them);
+//   S <  2^-8   add the pairs of d = 10 to their tile, last;
+//   S <  2^-10  are left to FP64 multiplications by the draining warp where it has
+//               few (FEW); where it has more, its outputs with
+//     S < 2^-8  are summed in units of 2^-70, with
+//     S < 2^-16 in units of 2^-78 (and d = 11 is added),
+//     S < 2^-20 left to FP64 multiplications.
+// Whatever is left out is then a rounding or two of sum |a_ik| |b_kj|, which FP64
+// chains of 128 to 512 products exceed.  Measured, N = 400, largest |P A - L U| /
+// |L||U| of an LU, in units of 2^-53:
 //                                          seven digits alone   now   LAPACK
 //   normal entries                                  1.8         1.8     1.9
-//   rows scaled over 1e12, the smallest first       300         2.1     1.7
-//   over 1e18, 1e30                             2.3e4, 7.7e7  2.1, 2.3  1.8, 2.1
+//   rows scaled over 1e12, the smallest first       300         1.8     1.7
+//   over 1e18, 1e30                             2.3e4, 7.7e7  2.1, 1.4  1.8, 2.1
 //   two sets coupled by 1e-6, 1e-12             5.9e4, 8.2e10 2.8, 2.5  3.3, 2.8
-// and of an update by itself, wide ranges of entries, k = 7 .. 256: 2 to 9, where
-// chains of FP64 FMAs have 2 to 15.  Error for normal entries, k = 256: 4.4e-18 of
-// |a| |b| root mean square, FP64 FMAs 4.3e-17; backward error of an LU of normal
-// entries, N = 768: 3.6e-15 (LAPACK 6.3e-15, FP64 updates 5.6e-15).
+// and of an update by itself, entries over 2^60, k = 7 .. 256: 1 to 4, chains of
+// FP64 FMAs 2 to 15.  Error for normal entries, k = 256: 4.4e-18 of |a| |b| root
+// mean square, FP64 FMAs 4.3e-17; backward error of an LU of normal entries,
+// N = 768: 3.6e-15 (LAPACK 6.3e-15, FP64 updates 5.6e-15).
 //
-// Time, k = 256 complex: m = n = 3584 1.01 ms, 26 TFLOP/s FP64 (0.87 with seven
-// digits alone), against 0.74 TFLOP/s for the SIMT FP64 update; 1653 308 us (267);
-// 480 x 64, k = 64 35 us (31).
+// Time, k = 256 complex: m = n = 3584 1.05 ms, 25 TFLOP/s FP64 (0.87 with seven
+// digits alone), against 0.74 TFLOP/s for the SIMT FP64 update; 1653 319 us (267);
+// 480 x 64, k = 64 33 us (31).  LU of dielectric spheres, N = 3840, kR = 2, 0.5, 0.1:
+// 37, 42, 58 ms; 36 with seven digits alone, 290 with SIMT updates; with every
+// output below 2^-10 left to FP64 37, 59 and, at 0.05 (76 now), 182.
 //
 // What bounds it: the instructions of the single-thread TMA and MMA issuers
 // per k-step at every size, and the tensor pipe (37 bf16 products in place of
@@ -63,9 +67,11 @@
 namespace gbem {
 
 namespace oz {
-constexpr int NS = 8;             // slices (base-256 digits); slice NS + 1 holds the sizes
-constexpr int STEPS = 10;         // groups of slice pairs: sizes, d = 9 .. 2, and d = 10 where it is called for
-constexpr float S_FINE = 1.0f, S_MORE = 1.0f / 256, S_FP64 = 1.0f / 1024;  // see above
+constexpr int NS = 9;             // slices (base-256 digits); slice NS + 1 holds the sizes
+constexpr int STEPS = 11;         // groups of slice pairs: sizes, d = 9 .. 2, and d = 10, 11 where they are called for
+// outputs by the sum of their products' sizes (see above)
+constexpr float S_FINE = 1.0f, S_10 = 0x1p-8f, S_FEW = 0x1p-10f, S_11 = 0x1p-16f, S_FP64 = 0x1p-20f;
+constexpr int FEW = 8;            // outputs below S_FEW that a warp leaves to FP64 rather than go below units of 2^-62
 constexpr int KMAX = 512;         // real products per output and slice pair
 constexpr int ACC_TERMS = 1024;   // products that add up exactly: 1024 * 2^14 = 2^24
 constexpr int BM = 128, BK = 64;
@@ -93,34 +99,43 @@ constexpr int VECS = 16;          // rows of A (columns of B) per packing CTA
 // exponent field (at least 1) of a double's high word
 __device__ __forceinline__ int exp_field(unsigned hi) { return max((int)((hi >> 20) & 0x7ffu), 1); }
 
-// |x| < 2^(F - 1022) as a signed 63-bit fixed-point number: round(x 2^(63 - (F - 1022)))
-__device__ __forceinline__ long long fixed63(double x, int F) {
+// |x| < 2^(F - 1022) as a 71-bit fixed-point number, round(|x| 2^(71 - (F - 1022))):
+// its leading 39 and its last 32 bits, in balanced digits -- bytes 0..3 of hi are the
+// digits 5..2 plus 128, above them the top digit; bytes 0..3 of lo the digits 9..6
+// plus 128 -- and its size as a bf16 number in units of 2^(F - 1022): no entry but
+// zero has size zero, so that a sum of sizes is zero only where every product is
+struct OzDigits { unsigned long long hi; unsigned lo; unsigned short size; };
+__device__ __forceinline__ OzDigits oz_digits(double x, int F) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int raw = (int)((b >> 52) & 0x7ffu), f = max(raw, 1);
+  const int raw = (int)((b >> 52) & 0x7ffu), d = F - max(raw, 1);  // d >= 0
   unsigned long long M = b & 0xfffffffffffffull;
   if (raw) M |= 1ull << 52;
-  const int d = F - f;  // >= 0
-  unsigned long long q;
-  if (d <= 10) q = M << (10 - d);
-  else if (d < 66) q = (M + (1ull << (d - 11))) >> (d - 10);
-  else q = 0;
-  return (long long)b < 0 ? -(long long)q : (long long)q;
+  unsigned long long hi, lo;
+  if (d <= 18) {
+    hi = M >> (14 + d);
+    lo = M << (18 - d) & 0xffffffffull;
+  } else {
+    lo = d < 74 ? (M + (1ull << (d - 19))) >> (d - 18) : 0;
+    hi = lo >> 32;
+    lo &= 0xffffffffull;
+  }
+  lo += 0x80808080ull;
+  OzDigits r;
+  r.lo = (unsigned)lo;
+  r.hi = hi + (lo >> 32) + 0x80808080ull;
+  const float v = (float)M * __int_as_float((74 - min(d, 60)) << 23);  // M 2^-53 2^-d
+  r.size = M ? __bfloat16_as_ushort(__float2bfloat16_rn(fmaxf(v, 0x1p-60f))) : (unsigned short)0;
+  return r;
 }
 
-// its size as a bf16 number in units of 2^(F - 1022); no entry but zero is zero,
-// so that a sum of sizes is zero only where every product is
-__device__ __forceinline__ unsigned short size_bf16(double x, long long q) {
-  const float v = (float)(unsigned long long)(q < 0 ? -q : q) * 0x1p-63f;
-  const bool zero = (__double_as_longlong(x) << 1) == 0;
-  return zero ? (unsigned short)0 : __bfloat16_as_ushort(__float2bfloat16_rn(fmaxf(v, 0x1p-60f)));
-}
-
-// step of a tile (0: the sizes; 1 .. 8: d = 9 .. 2; 9: d = 10) -> its slice pairs (i, j), i0 <= i < i1, j = sum - i
+// step of a tile (0: the sizes; 1 .. 8: d = 9 .. 2; 9, 10: d = 10, 11) -> its slice pairs (i, j), i0 <= i < i1, j = sum - i
 struct OzGroup { int i0, i1, sum; };
-__device__ __forceinline__ OzGroup oz_group(int step) {
+// (d = 10 without the ninth digits where units of 2^-62 are the finest: narrow)
+__device__ __forceinline__ OzGroup oz_group(int step, bool narrow) {
   if (step == 0) return {oz::NS + 1, oz::NS + 2, 2 * oz::NS + 2};
-  const int d = step < oz::STEPS - 1 ? 10 - step : 10;
-  return {max(1, d - oz::NS), min(oz::NS + 1, d), d};
+  const int d = step < 9 ? 10 - step : step + 1;
+  const int cut = d == 10 && narrow ? 1 : 0;
+  return {max(1, d - oz::NS) + cut, min(oz::NS + 1, d) - cut, d};
 }
 
 // The digits of A's rows (part 0) and B's columns (part 1), one launch: CTAs
@@ -188,9 +203,7 @@ __global__ void __launch_bounds__(256) oz_pack(const double* A, long long lda, i
     const int r = q / groups, g = q - r * groups;
     const int v = rpv == 2 ? r >> 1 : r, odd = rpv == 2 ? r & 1 : 0;
     const int F = vexp[v];
-    unsigned long long b[4];  // bytes 0..6: digits 8..2 plus 128
-    int top[4];
-    unsigned short sz[4];
+    OzDigits z[4];
     unsigned neg = 0;
 #pragma unroll
     for (int e = 0; e < 4; e++) {
@@ -208,18 +221,18 @@ __global__ void __launch_bounds__(256) oz_pack(const double* A, long long lda, i
       } else if (p < k) {
         x = t[p * 17 + v];
       }
-      const long long q = F < 0 ? 0 : fixed63(x, F);
-      b[e] = ((unsigned long long)q & 0xffffffffffffffull) + 0x80808080808080ull;
-      top[e] = (int)(q >> 56) + (int)(b[e] >> 56);
-      sz[e] = F < 0 ? (unsigned short)0 : size_bf16(x, q);
+      if (F < 0) x = 0.0;
+      neg ^= (unsigned)(__double2hiint(x) < 0) << e;
+      z[e] = oz_digits(x, F < 0 ? 1 : F);
     }
 #pragma unroll
     for (int s = 0; s <= oz::NS; s++) {  // slice s holds digit s + 1 (the top one first), the last the sizes
       unsigned short w[4];
 #pragma unroll
       for (int e = 0; e < 4; e++) {
-        const int dg = s == 0 ? top[e] : (int)((b[e] >> (8 * (7 - s) & 63)) & 255) - 128;
-        w[e] = s == oz::NS ? sz[e] : (unsigned short)(__float_as_uint((float)((neg >> e) & 1u ? -dg : dg)) >> 16);
+        const int dg = s == 0 ? (int)(z[e].hi >> 32)
+                              : (int)((s < 5 ? z[e].hi >> (8 * (4 - s)) : (unsigned long long)(z[e].lo >> (8 * (8 - min(s, 8))))) & 255) - 128;
+        w[e] = s == oz::NS ? z[e].size : (unsigned short)(__float_as_uint((float)((neg >> e) & 1u ? -dg : dg)) >> 16);
       }
       uint2 pk;
       pk.x = (unsigned)w[0] | ((unsigned)w[1] << 16);
@@ -239,6 +252,13 @@ __device__ __forceinline__ double int_to_double(long long T, int e) {
   unsigned long long b = ((unsigned long long)(1023 + 63 - 1 + e - lz) << 52) + q;
   b |= (unsigned long long)T & 0x8000000000000000ull;
   return a ? __longlong_as_double((long long)b) : 0.0;
+}
+
+// x 2^s modulo 2^64, 0 <= s <= 64
+__device__ __forceinline__ unsigned long long shl64(long long x, int s) {
+  unsigned long long y;
+  asm("shl.b64 %0, %1, %2;" : "=l"(y) : "l"(x), "r"(s));
+  return y;
 }
 
 // C(row, j) -= sum_k A(row, k) B(k, j) in FP64 for a warp's outputs marked in need
@@ -299,7 +319,7 @@ __device__ __noinline__ void oz_fp64(double* C, long long ldc, const double* A, 
 // one another through two BN-column TMEM buffers: the MMAs of the next run
 // while the drain warps add the last one into their 64-bit integers (one row
 // and BN / 2 columns per thread).  The sizes come first: by the end of a tile its
-// draining warps have long decided whether d = 10 follows.  pairs: slice pairs
+// draining warps have long decided whether d = 10 and 11 follow.  pairs: slice pairs
 // per accumulator.  A, B: the operands themselves, for the outputs left to FP64.
 template <bool CPLX, int BN>
 __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__ CUtensorMap mapA,
@@ -322,7 +342,12 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
   uint64_t* decided = done + 1;             // drain -> all: s_more of this tile is final (8 warp arrivals)
   uint32_t* tmem_slot = (uint32_t*)(decided + 1);
   __shared__ int s_fail, s_skip;
-  __shared__ int s_more[2];  // by the parity of a CTA's tile number: the last tile (from 1) that takes d = 10
+  // the last of a CTA's tiles (from 1, by parity) that takes d = 10, d = 11, and
+  // d = 10 with the ninth digits
+  __shared__ int s_more[3][2];
+  // by drain thread and 32 columns: outputs in units of 2^-70, of 2^-78, left to
+  // FP64, left to FP64 if they are few
+  __shared__ unsigned s_low[(CW + 31) / 32][4][256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = CPLX ? 2 * n : n;  // real output columns
   const int kbx = min(oz::KB, kblocks);
@@ -332,13 +357,13 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
     for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }
     mbar_init(done, 1);
     mbar_init(decided, 8);
-    s_more[0] = s_more[1] = 0;
+    for (int q = 0; q < 6; q++) s_more[q / 2][q % 2] = 0;
     s_fail = 0;
-    // once a CTA of this call has given up a wait, the rest do no work (read
-    // once, so that the whole CTA takes the same way)
-    s_skip = *(volatile int*)wait_error;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // once a CTA of this call has given up a wait, the rest do no work (read once, so
+  // that the whole CTA takes the same way; by a thread with nothing else to do here)
+  if (threadIdx.x == 64) s_skip = *(volatile int*)wait_error;
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(2 * BN));
@@ -358,11 +383,11 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
       for (int t = blockIdx.x, it = 0; t < ntiles && ok; t += gridDim.x, it++) {
         const int ya = (t % mt) * oz::BM, yb = (t / mt) * BN;
         for (int step = 0; step < oz::STEPS && ok; step++) {
-          if (step == oz::STEPS - 1) {
-            if (!mbar_wait(decided, (uint32_t)(it & 1))) { atomicExch(&s_fail, 1); ok = false; }
-            if (!ok || *(volatile int*)&s_more[it & 1] != it + 1) break;
+          if (step >= 9) {
+            if (step == 9 && !mbar_wait(decided, (uint32_t)(it & 1))) { atomicExch(&s_fail, 1); ok = false; }
+            if (!ok || *(volatile int*)&s_more[step - 9][it & 1] != it + 1) break;
           }
-          const OzGroup g = oz_group(step);
+          const OzGroup g = oz_group(step, step == 9 && *(volatile int*)&s_more[2][it & 1] != it + 1);
           for (int i = g.i0; i < g.i1 && ok; i++)
             for (int kb = 0; kb < kblocks; kb += kbx, r.next()) {
               // a fresh barrier's previous phase counts as complete
@@ -395,11 +420,11 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
       const uint64_t desc0 = sdesc_sw128(smem_u32(tiles));  // addresses count 16 bytes in the low bits
       for (int t = blockIdx.x, it = 0; t < ntiles && ok; t += gridDim.x, it++)
         for (int step = 0; step < oz::STEPS && ok; step++) {
-          if (step == oz::STEPS - 1) {
-            if (!mbar_wait(decided, (uint32_t)(it & 1))) { atomicExch(&s_fail, 1); ok = false; }
-            if (!ok || *(volatile int*)&s_more[it & 1] != it + 1) break;
+          if (step >= 9) {
+            if (step == 9 && !mbar_wait(decided, (uint32_t)(it & 1))) { atomicExch(&s_fail, 1); ok = false; }
+            if (!ok || *(volatile int*)&s_more[step - 9][it & 1] != it + 1) break;
           }
-          const OzGroup g = oz_group(step);
+          const OzGroup g = oz_group(step, step == 9 && *(volatile int*)&s_more[2][it & 1] != it + 1);
           for (int i0 = g.i0; i0 < g.i1 && ok; i0 += pairs, u++) {
             const int acc = u & 1, i1 = min(i0 + pairs, g.i1);
             if (u >= 2 && !mbar_wait(&acc_empty[acc], (uint32_t)(((u >> 1) - 1) & 1))) {
@@ -433,7 +458,7 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
   } else {
     // warp % 4 selects the TMEM lane quarter, the two warps of a quarter
     // split the 128 columns
-    const int q = warp & 3, half = (warp - 2) >> 2;
+    const int q = warp & 3, half = (warp - 2) >> 2, dt = threadIdx.x - 64;
     constexpr int CH = 16, NM = (CW + 31) / 32;
     int u = 0;
     bool ok = true;
@@ -441,21 +466,23 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
       const int tm = t % mt, tn = t / mt;
       const int row = tm * oz::BM + q * 32 + lane, col0 = tn * BN + half * CW;  // col0: a real column
       unsigned long long T[CW];  // modulo 2^64
-      unsigned fine[NM], low[NM];    // by column
+      unsigned fine[NM];         // by column: S < S_FINE
+      bool some = false;         // outputs of this warp take finer units
 #pragma unroll
-      for (int h = 0; h < NM; h++) fine[h] = low[h] = 0;
+      for (int h = 0; h < NM; h++) fine[h] = 0;
 #pragma unroll
       for (int c = 0; c < CW; c++) T[c] = 0;
       for (int step = 0; step < oz::STEPS && ok; step++) {
-        if (step == oz::STEPS - 1) {
-          ok = mbar_wait(decided, (uint32_t)(it & 1));
+        if (step >= 9) {
+          if (step == 9) ok = mbar_wait(decided, (uint32_t)(it & 1));
           if (!ok) atomicExch(&s_fail, 1);
           ok = __all_sync(0xffffffffu, ok);
-          if (!ok || *(volatile int*)&s_more[it & 1] != it + 1) break;
+          if (!ok || *(volatile int*)&s_more[step - 9][it & 1] != it + 1) break;
         }
-        const OzGroup g = oz_group(step);
+        const OzGroup g = oz_group(step, step == 9 && *(volatile int*)&s_more[2][it & 1] != it + 1);
         // units: 2^-70 for d = 9, 2^-62 down to d = 4, then 2^-53, for a fine
-        // output still 2^-62; every sum of the former stays below 2^63
+        // output still 2^-62; every sum of the former stays below 2^63.  (Some: 2^-62,
+        // 2^-70 or 2^-78 from the first, then 2^-53 for those that are not fine.)
         const int d = g.sum, sh = d >= 8 ? 0 : (d >= 4 ? 8 * (8 - d) : (d == 3 ? 31 : 39)), shf = d <= 3 ? sh + 9 : sh;
         for (int i0 = g.i0; i0 < g.i1; i0 += pairs, u++) {
           const int acc = u & 1;
@@ -475,23 +502,50 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
               if (lane == 0) mbar_arrive(&acc_empty[acc]);
             }
             if (step == 0) {
-              // (a zero sum needs nothing; rows beyond m hold other slices)
+              // (a zero sum needs nothing; beyond C's edge they are zero)
               float least = oz::S_FINE;
 #pragma unroll
               for (int c = 0; c < CH; c++) {
                 if (v[c] < oz::S_FINE) fine[c0 / 32] |= 1u << (c0 + c) % 32;
-                least = fminf(least, v[c] > 0.0f && col0 + c0 + c < nb ? v[c] : oz::S_FINE);
+                least = fminf(least, v[c] > 0.0f ? v[c] : oz::S_FINE);
               }
-              if (row < m && least < oz::S_FP64) {
+              unsigned l10 = 0, l11 = 0, l64 = 0, few = 0;
+              if (least < oz::S_10) {
 #pragma unroll
-                for (int c = 0; c < CH; c++)
-                  if (v[c] < oz::S_FP64 && v[c] > 0.0f) low[c0 / 32] |= 1u << (c0 + c) % 32;
+                for (int c = 0; c < CH; c++) {
+                  const unsigned bit = v[c] > 0.0f ? 1u << (c0 + c) % 32 : 0u;
+                  if (v[c] < oz::S_10) l10 |= bit;
+                  if (v[c] < oz::S_FEW) few |= bit;
+                  if (v[c] < oz::S_11) l11 |= bit;
+                  if (v[c] < oz::S_FP64) l64 |= bit;
+                }
               }
-              if (__any_sync(0xffffffffu, row < m && least < oz::S_MORE) && lane == 0) atomicMax(&s_more[it & 1], it + 1);
-            } else if (step == oz::STEPS - 1) {
+              const int h = c0 / 32;
+              if (c0 % 32 == 0) s_low[h][0][dt] = s_low[h][1][dt] = s_low[h][2][dt] = s_low[h][3][dt] = 0;
+              if (l10) {
+                s_low[h][0][dt] |= l10;
+                s_low[h][1][dt] |= l11;
+                s_low[h][2][dt] |= l64;
+                s_low[h][3][dt] |= few;
+              }
+            } else if (some) {
+              const unsigned l10 = s_low[c0 / 32][0][dt], l11 = s_low[c0 / 32][1][dt];
+#pragma unroll
+              for (int c = 0; c < CH; c++) {
+                const int bit = (c0 + c) % 32;
+                const bool f = (fine[c0 / 32] >> bit) & 1;
+                // 2^-(8d - 2) in units of 2^-62, 2^-70 or 2^-78 (or 2^-53)
+                const int r = 64 - 8 * d + (((l10 >> bit) & 1) << 3) + (((l11 >> bit) & 1) << 3) - (d <= 3 && !f ? 9 : 0);
+                const long long x = (long long)__float2int_rn(v[c]);
+                const unsigned long long y = r >= 0 ? shl64(x, r) : (unsigned long long)((x + (1ll << (-r - 1))) >> -r);
+                if (d < 10 || f) T[c0 + c] += y;
+              }
+            } else if (step == 9) {
 #pragma unroll
               for (int c = 0; c < CH; c++)
                 if ((fine[c0 / 32] >> (c0 + c) % 32) & 1) T[c0 + c] += (unsigned long long)(long long)((__float2int_rn(v[c]) + (1 << 15)) >> 16);
+            } else if (step == 10) {
+              // nothing of d = 11 counts here
             } else if (sh == shf) {
 #pragma unroll
               for (int c = 0; c < CH; c++) T[c0 + c] += (unsigned long long)(long long)__float2int_rn(v[c]) << sh;
@@ -504,10 +558,34 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
         }
         if (!ok) break;
         if (step == 0) {
+          // how small the warp's outputs are: d = 10 for some; beyond FEW below
+          // S_FEW, finer units too
+          unsigned any10 = 0, any11 = 0, nfew = 0;
+#pragma unroll
+          for (int h = 0; h < NM; h++) {
+            any10 |= s_low[h][0][dt];
+            any11 |= s_low[h][1][dt];
+            nfew += __popc(s_low[h][3][dt]);
+          }
+          some = __reduce_add_sync(0xffffffffu, nfew) > oz::FEW;
+          any10 = __any_sync(0xffffffffu, any10 != 0);
+          any11 = __any_sync(0xffffffffu, any11 != 0);
+          if (!some) {
+#pragma unroll
+            for (int h = 0; h < NM; h++) {
+              s_low[h][0][dt] = s_low[h][1][dt] = 0;
+              s_low[h][2][dt] = s_low[h][3][dt];
+            }
+          }
+          if (lane == 0) {
+            if (any10) atomicMax(&s_more[0][it & 1], it + 1);
+            if (some && any11) atomicMax(&s_more[1][it & 1], it + 1);
+            if (some) atomicMax(&s_more[2][it & 1], it + 1);
+          }
           __syncwarp();
           if (lane == 0) mbar_arrive(decided);
         }
-        if (d == 9) {
+        if (d == 9 && !some) {
 #pragma unroll
           for (int c = 0; c < CW; c++) T[c] = (unsigned long long)(((long long)T[c] + 128) >> 8);
         }
@@ -520,6 +598,13 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
       if (!ok) break;
       constexpr int W = CPLX ? 2 : 1;
       const int j0 = col0 / W;
+      unsigned l10[NM], l11[NM], l64[NM];
+#pragma unroll
+      for (int h = 0; h < NM; h++) {
+        l10[h] = s_low[h][0][dt];
+        l11[h] = s_low[h][1][dt];
+        l64[h] = s_low[h][2][dt];
+      }
       if (row < m) {
         const int er = ea[row];
 #pragma unroll
@@ -527,6 +612,11 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
           const int j = j0 + c / W;
           if (j >= n) break;
           const int ec = eb[j], e = er + ec - 53;
+          // the unit of the sum, 2^-53 less 0, 9, 17 or 25
+          auto unit = [&](int cc) {
+            const int h = cc / 32, bit = cc % 32;
+            return e - (((fine[h] >> bit) & 1) * 9 + ((((l10[h] >> bit) & 1) + ((l11[h] >> bit) & 1)) << 3));
+          };
           double* p = C + W * ((long long)row + (long long)j * ldc);
           double z[W];
           if (CPLX) {
@@ -535,17 +625,17 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
           } else {
             z[0] = *p;
           }
-          if (e > -990 && e < 960) {
+          if (e > -970 && e < 960) {
 #pragma unroll
-            for (int w = 0; w < W; w++) z[w] -= int_to_double((long long)T[c + w], e - (((fine[c / 32] >> ((c + w) % 32)) & 1) ? 9 : 0));
+            for (int w = 0; w < W; w++) z[w] -= int_to_double((long long)T[c + w], unit(c + w));
           } else if (er == oz::EXP_BAD || ec == oz::EXP_BAD) {
 #pragma unroll
             for (int w = 0; w < W; w++) z[w] = __longlong_as_double(0x7ff8000000000000ll);
           } else {
 #pragma unroll
-            for (int w = 0; w < W; w++) z[w] -= ldexp((double)(long long)T[c + w], e - (((fine[c / 32] >> ((c + w) % 32)) & 1) ? 9 : 0));
+            for (int w = 0; w < W; w++) z[w] -= ldexp((double)(long long)T[c + w], unit(c + w));
           }
-          if (!((low[c / 32] >> (c % 32)) & (W == 2 ? 3u : 1u))) {
+          if (!((l64[c / 32] >> (c % 32)) & (W == 2 ? 3u : 1u))) {
             if (CPLX) *reinterpret_cast<double2*>(p) = make_double2(z[0], z[W - 1]);
             else *p = z[0];
           }
@@ -553,7 +643,7 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
       }
 #pragma unroll
       for (int h = 0; h < NM; h++)
-        if (__any_sync(0xffffffffu, low[h] != 0)) oz_fp64<CPLX>(C, ldc, A, lda, B, ldb, m, n, k, row, j0 + h * 32 / W, low[h]);
+        if (__any_sync(0xffffffffu, l64[h] != 0)) oz_fp64<CPLX>(C, ldc, A, lda, B, ldb, m, n, k, row, j0 + h * 32 / W, l64[h]);
     }
   }
   tc_fence_before();

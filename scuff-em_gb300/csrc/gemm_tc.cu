@@ -145,11 +145,11 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_kernel(const __grid_constant__
     for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }
     mbar_init(drain, 1);
     s_fail = 0;
-    // once a CTA of this call has given up a wait, the rest do no work (read
-    // once, so that the whole CTA takes the same way)
-    s_skip = *(volatile int*)wait_error;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // once a CTA of this call has given up a wait, the rest do no work (read once, so
+  // that the whole CTA takes the same way; by a thread with nothing else to do here)
+  if (threadIdx.x == 64) s_skip = *(volatile int*)wait_error;
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(2 * tc::TMEM_COLS));
