@@ -104,7 +104,13 @@ gbem_status gbem_matrix_upload(gbem_matrix *m, const void *host, int ldh);
  * RWGGeometry::UpdateCachedEpsMuValues caches, RWGGeometry.cc:1093-1113).
  * precision: gbem_precision.  The matrix dtype must be C128 or F64 for FP64
  * and C64 for MIXED; F64 (the reference's real storage, used at purely
- * imaginary Omega where the matrix is real) keeps the real part. */
+ * imaginary Omega where the matrix is real) keeps the real part.
+ * The geometry keeps the far field's scratch from its first assembly until it is
+ * destroyed: FP64 (and gradient blocks of bodies without near pairs) 144 bytes
+ * per panel pair of a column stripe and per channel -- one channel between PEC
+ * bodies, three between dielectrics, stripes of at most 3 * 2^20 pairs: up to
+ * 0.45 and 1.36 GB -- and the mixed form up to 1.1 GB.  Where the FP64 scratch
+ * cannot be had, a slower kernel that needs none runs. */
 gbem_status gbem_assemble(gbem_geometry *g, double omega_re, double omega_im,
                           const double *eps, const double *mu, int precision,
                           gbem_matrix *M);
@@ -166,8 +172,12 @@ gbem_status gbem_assemble_block_host(gbem_geometry *g, int nsa, int nsb, double 
 /* ---- dense LU ------------------------------------------------------------ */
 /* Replaces HMatrix::LUFactorize (libs/libhmat/LBWrappers.cc:151-171):
  * in-place LU with partial pivoting of a C128 (zgetrf semantics), F64
- * (dgetrf semantics) or C64 matrix.  ipiv (optional, host, N ints) receives 1-based pivots; info is 0,
- * or k > 0 if U(k,k) is exactly zero. */
+ * (dgetrf semantics) or C64 matrix.  ipiv (optional, host, N ints) receives
+ * 1-based pivots; info is 0, or k > 0 if U(k,k) is exactly zero.  The matrix
+ * keeps the factorisation's workspace until it is destroyed: for C128 about
+ * 120 w N bytes (w: the widest panel, 128 or 256 columns; 0.24 GB at N = 15360),
+ * for F64 a third of that; where it cannot be had, the FP64 updates run without
+ * it, more slowly. */
 gbem_status gbem_lu_factor(gbem_matrix *M, int *ipiv, int *info);
 
 /* Replaces HMatrix::LUSolve(HMatrix *X, char Trans, int nrhs)
