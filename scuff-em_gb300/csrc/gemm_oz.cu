@@ -44,16 +44,22 @@
 // mean square, FP64 FMAs 4.3e-17; backward error of an LU of normal entries,
 // N = 768: 3.6e-15 (LAPACK 6.3e-15, FP64 updates 5.6e-15).
 //
-// Time, k = 256 complex: m = n = 3584 1.05 ms, 25 TFLOP/s FP64 (0.87 with seven
-// digits alone), against 0.74 TFLOP/s for the SIMT FP64 update; 1653 319 us (267);
-// 480 x 64, k = 64 33 us (31).  LU of dielectric spheres, N = 3840, kR = 2, 0.5, 0.1:
-// 37, 42, 58 ms; 36 with seven digits alone, 290 with SIMT updates; with every
-// output below 2^-10 left to FP64 37, 59 and, at 0.05 (76 now), 182.
+// Time, k = 256 complex: m = n = 3584 0.96 ms, 27 TFLOP/s FP64 (0.87 with seven
+// digits alone), against 0.74 TFLOP/s for the SIMT FP64 update; 1653 302 us (267);
+// 480 x 64, k = 64 33 us (31); real 3584 372 us (402).  LU of dielectric spheres,
+// N = 3840, kR = 2, 0.5, 0.1: 37, 41, 57 ms; 36 with seven digits alone, 290 with SIMT
+// updates; with every output below 2^-10 left to FP64 37, 59 and, at 0.05 (76 now),
+// 182.
 //
-// What bounds it: the instructions of the single-thread TMA and MMA issuers
-// per k-step at every size, and the tensor pipe (37 bf16 products in place of
-// one FP64 one) not far behind.  The FP64 pipe it replaces runs 2 FMAs per
-// cycle and SM; outputs left to it take as long as gemm_simt took.
+// What bounds it: large updates, the draining warps' instructions -- ncu, m = n =
+// 3584, k = 256: tensor pipe 43 % active, of the drain's stalls a quarter waits for
+// instructions (64 outputs of a thread are 64 copies of the code) and a third for
+// TMEM, C and spilled words; one conversion for every exponent in place of three
+// branches 1.04 -> 0.96 ms.  Small ones, the single-thread TMA and MMA issuers'
+// instructions per k-step.  Output tiles are walked in bands of 16 rows of tiles: with
+// columns of 118 the slices of A no longer fit the L2 (m = n = 15104, k = 128: 12.8 ->
+// 10.7 ms).  The FP64 pipe it replaces runs 2 FMAs per cycle and SM; outputs left to it
+// take as long as gemm_simt took.
 //
 // A row or column that holds an infinity or NaN makes its row or column of C
 // NaN (the digits are zero there).
@@ -93,6 +99,7 @@ template <int BN> struct Tile {
   static_assert(B_BLK % 1024 == 0, "swizzle atoms");
 };
 constexpr int EXP_BAD = 1 << 20;  // scale exponent of a row or column that is not finite
+constexpr int BAND = 16;          // rows of output tiles walked together (8 and 32 within 1 %)
 constexpr int VECS = 16;          // rows of A (columns of B) per packing CTA
 }  // namespace oz
 
@@ -242,16 +249,30 @@ __global__ void __launch_bounds__(256) oz_pack(const double* A, long long lda, i
   }
 }
 
-// T 2^e rounded to 53 bits, -1000 < e < 960, in integer arithmetic: the FP64
-// pipe (2 operations per cycle and SM) is left with the one subtraction.
+// T 2^e rounded to 53 bits (below 2^-1022 cut off, above the range infinite; NaN for
+// the exponent of a row or column that is not finite), in integer arithmetic: the
+// FP64 pipe (2 operations per cycle and SM) is left with the one subtraction.  One
+// path for every exponent: a drain warp runs its 64 copies once a tile, and what it
+// waits for most is instructions.
 __device__ __forceinline__ double int_to_double(long long T, int e) {
   const unsigned long long a = T < 0 ? 0ull - (unsigned long long)T : (unsigned long long)T;
   const int lz = __clzll((long long)a);
   const unsigned long long m = a << (lz & 63);
   const unsigned long long q = (m >> 11) + ((m >> 10) & 1ull);  // 2^52 .. 2^53
-  unsigned long long b = ((unsigned long long)(1023 + 63 - 1 + e - lz) << 52) + q;
+  const int E = 1023 + 63 - 1 + e - lz;                          // the exponent field, less what q brings
+  unsigned long long b = E >= 0 ? ((unsigned long long)E << 52) + q : q >> min(-E, 63);
+  if (E > 2045) b = 0x7ff0000000000000ull;
+  if (!a) b = 0;
   b |= (unsigned long long)T & 0x8000000000000000ull;
-  return a ? __longlong_as_double((long long)b) : 0.0;
+  if (e > oz::EXP_BAD / 2) b = 0x7ff8000000000000ull;
+  return __longlong_as_double((long long)b);
+}
+
+// the t-th output tile of mt x (ntiles / mt)
+struct OzTile { int m, n; };
+__device__ __forceinline__ OzTile oz_tile(int t, int mt, int ntiles) {
+  const int nt = ntiles / mt, b = t / (oz::BAND * nt), r = t - b * oz::BAND * nt, h = min(oz::BAND, mt - b * oz::BAND);
+  return {b * oz::BAND + r % h, r / h};
 }
 
 // x 2^s modulo 2^64, 0 <= s <= 64
@@ -314,7 +335,8 @@ __device__ __noinline__ void oz_fp64(double* C, long long ldc, const double* A, 
 }
 
 // One CTA per SM walks the 128 x BN output tiles (columns counted as reals;
-// m fastest, so the CTAs of a wave share their B tile).  Warp 0: TMA producer;
+// in bands of BAND rows of tiles, m fastest, so the CTAs of a wave share their B
+// tiles and a band of A).  Warp 0: TMA producer;
 // warp 1: TMEM and MMA issue; warps 2-9: drain.  A tile's accumulators follow
 // one another through two BN-column TMEM buffers: the MMAs of the next run
 // while the drain warps add the last one into their 64-bit integers (one row
@@ -381,7 +403,8 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
       int issued = 0;  // stages in use
       bool ok = true;
       for (int t = blockIdx.x, it = 0; t < ntiles && ok; t += gridDim.x, it++) {
-        const int ya = (t % mt) * oz::BM, yb = (t / mt) * BN;
+        const OzTile tile = oz_tile(t, mt, ntiles);
+        const int ya = tile.m * oz::BM, yb = tile.n * BN;
         for (int step = 0; step < oz::STEPS && ok; step++) {
           if (step >= 9) {
             if (step == 9 && !mbar_wait(decided, (uint32_t)(it & 1))) { atomicExch(&s_fail, 1); ok = false; }
@@ -463,8 +486,8 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
     int u = 0;
     bool ok = true;
     for (int t = blockIdx.x, it = 0; t < ntiles && ok; t += gridDim.x, it++) {
-      const int tm = t % mt, tn = t / mt;
-      const int row = tm * oz::BM + q * 32 + lane, col0 = tn * BN + half * CW;  // col0: a real column
+      const OzTile tile = oz_tile(t, mt, ntiles);
+      const int row = tile.m * oz::BM + q * 32 + lane, col0 = tile.n * BN + half * CW;  // col0: a real column
       unsigned long long T[CW];  // modulo 2^64
       unsigned fine[NM];         // by column: S < S_FINE
       bool some = false;         // outputs of this warp take finer units
@@ -607,37 +630,38 @@ __global__ void __launch_bounds__(320, 1) oz_gemm_kernel(const __grid_constant__
       }
       if (row < m) {
         const int er = ea[row];
+        constexpr int EB = 4;  // C's elements in flight: their loads are a trip to memory each
 #pragma unroll
-        for (int c = 0; c < CW; c += W) {
-          const int j = j0 + c / W;
-          if (j >= n) break;
-          const int ec = eb[j], e = er + ec - 53;
-          // the unit of the sum, 2^-53 less 0, 9, 17 or 25
-          auto unit = [&](int cc) {
-            const int h = cc / 32, bit = cc % 32;
-            return e - (((fine[h] >> bit) & 1) * 9 + ((((l10[h] >> bit) & 1) + ((l11[h] >> bit) & 1)) << 3));
-          };
-          double* p = C + W * ((long long)row + (long long)j * ldc);
-          double z[W];
-          if (CPLX) {
-            const double2 zz = *reinterpret_cast<const double2*>(p);
-            z[0] = zz.x; z[W - 1] = zz.y;
-          } else {
-            z[0] = *p;
+        for (int cb = 0; cb < CW; cb += EB * W) {
+          double z[EB][W];
+          int ec[EB];
+#pragma unroll
+          for (int b = 0; b < EB; b++) {
+            const int j = min(j0 + cb / W + b, n - 1);
+            const double* p = C + W * ((long long)row + (long long)j * ldc);
+            ec[b] = eb[j];
+            if (CPLX) {
+              const double2 zz = *reinterpret_cast<const double2*>(p);
+              z[b][0] = zz.x; z[b][W - 1] = zz.y;
+            } else {
+              z[b][0] = *p;
+            }
           }
-          if (e > -970 && e < 960) {
 #pragma unroll
-            for (int w = 0; w < W; w++) z[w] -= int_to_double((long long)T[c + w], unit(c + w));
-          } else if (er == oz::EXP_BAD || ec == oz::EXP_BAD) {
+          for (int b = 0; b < EB; b++) {
+            const int c = cb + b * W, j = j0 + c / W, e = er + ec[b] - 53;
+            // the unit of the sum, 2^-53 less 0, 9, 17 or 25
+            auto unit = [&](int cc) {
+              const int h = cc / 32, bit = cc % 32;
+              return e - (((fine[h] >> bit) & 1) * 9 + ((((l10[h] >> bit) & 1) + ((l11[h] >> bit) & 1)) << 3));
+            };
 #pragma unroll
-            for (int w = 0; w < W; w++) z[w] = __longlong_as_double(0x7ff8000000000000ll);
-          } else {
-#pragma unroll
-            for (int w = 0; w < W; w++) z[w] -= ldexp((double)(long long)T[c + w], unit(c + w));
-          }
-          if (!((l64[c / 32] >> (c % 32)) & (W == 2 ? 3u : 1u))) {
-            if (CPLX) *reinterpret_cast<double2*>(p) = make_double2(z[0], z[W - 1]);
-            else *p = z[0];
+            for (int w = 0; w < W; w++) z[b][w] -= int_to_double((long long)T[c + w], unit(c + w));
+            if (j < n && !((l64[c / 32] >> (c % 32)) & (W == 2 ? 3u : 1u))) {
+              double* p = C + W * ((long long)row + (long long)j * ldc);
+              if (CPLX) *reinterpret_cast<double2*>(p) = make_double2(z[b][0], z[b][W - 1]);
+              else *p = z[b][0];
+            }
           }
         }
       }

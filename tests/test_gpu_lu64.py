@@ -307,3 +307,37 @@ def test_pivots_of_extreme_size(power, real):
     assert np.array_equal(p0, p1)
     assert np.array_equal(np.tril(F0, -1), np.tril(F1, -1))
     assert np.array_equal(np.triu(F0) * 2.0 ** power, np.triu(F1))
+
+
+@pytest.mark.parametrize("real", [False, True])
+@pytest.mark.parametrize("power", [-1015, -960, 960, 1015])
+def test_updates_at_the_ends_of_the_range(power, real):
+    """Sums of the updates that are subnormal or close to overflow: the backward
+    error of the scaled factors, entry by entry, with one subnormal spacing of
+    2^-1074 for each of the N subtractions beside the relative error."""
+    N = 300
+    rng = np.random.default_rng(13)
+    A = rng.standard_normal((N, N))
+    if not real:
+        A = A + 1j * rng.standard_normal((N, N))
+    A = A * 2.0 ** power
+    if real:
+        from gbem._lib import F64
+        from gbem.api import HMatrix
+        M = HMatrix(_strip(N), F64)
+        M.set(A)
+        assert M.LUFactorize() == 0
+        LU, piv = M.numpy(), M.ipiv - 1
+    else:
+        LU, piv = _factor(A)
+    perm = np.arange(N)
+    for i, p in enumerate(piv):
+        perm[[i, p]] = perm[[p, i]]
+    L, R = np.tril(LU, -1) + np.eye(N), np.triu(LU)
+    assert np.isfinite(R).all() and np.abs(L).max() <= np.sqrt(2.0) * (1 + 1e-12)
+    # in units of 2^power, where every product is a normal number
+    R0 = R * 2.0 ** (-power // 2) * 2.0 ** (-power - (-power // 2))
+    A0 = A * 2.0 ** (-power // 2) * 2.0 ** (-power - (-power // 2))
+    tiny = 2.0 ** max(-1074 - power, -1074)
+    bound = 8 * N * (U * (np.abs(L) @ np.abs(R0) + np.abs(A0[perm])) + tiny)
+    assert (np.abs(A0[perm] - L @ R0) <= bound).all()
