@@ -44,9 +44,9 @@
 // mean square, FP64 FMAs 4.3e-17; backward error of an LU of normal entries,
 // N = 768: 3.6e-15 (LAPACK 6.3e-15, FP64 updates 5.6e-15).
 //
-// Time, k = 256 complex: m = n = 3584 0.96 ms, 27 TFLOP/s FP64 (0.87 with seven
-// digits alone), against 0.74 TFLOP/s for the SIMT FP64 update; 1653 302 us (267);
-// 480 x 64, k = 64 33 us (31); real 3584 372 us (402).  LU of dielectric spheres,
+// Time, k = 256 complex: m = n = 3584 0.97 ms, 27 TFLOP/s FP64 (0.87 with seven
+// digits alone), against 0.74 TFLOP/s for the SIMT FP64 update; 1653 306 us (267);
+// 480 x 64, k = 64 33 us (31); real 3584 401 us (402).  LU of dielectric spheres,
 // N = 3840, kR = 2, 0.5, 0.1: 37, 41, 57 ms; 36 with seven digits alone, 290 with SIMT
 // updates; with every output below 2^-10 left to FP64 37, 59 and, at 0.05 (76 now),
 // 182.
@@ -55,7 +55,7 @@
 // 3584, k = 256: tensor pipe 43 % active, of the drain's stalls a quarter waits for
 // instructions (64 outputs of a thread are 64 copies of the code) and a third for
 // TMEM, C and spilled words; one conversion for every exponent in place of three
-// branches 1.04 -> 0.96 ms.  Small ones, the single-thread TMA and MMA issuers'
+// branches 1.04 -> 0.97 ms.  Small ones, the single-thread TMA and MMA issuers'
 // instructions per k-step.  Output tiles are walked in bands of 16 rows of tiles: with
 // columns of 118 the slices of A no longer fit the L2 (m = n = 15104, k = 128: 12.8 ->
 // 10.7 ms).  The FP64 pipe it replaces runs 2 FMAs per cycle and SM; outputs left to it
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(256) oz_pack(const double* A, long long lda, i
   }
 }
 
-// T 2^e rounded to 53 bits (below 2^-1022 cut off, above the range infinite; NaN for
+// T 2^e rounded to 53 bits (fewer below 2^-1022; above the range infinite; NaN for
 // the exponent of a row or column that is not finite), in integer arithmetic: the
 // FP64 pipe (2 operations per cycle and SM) is left with the one subtraction.  One
 // path for every exponent: a drain warp runs its 64 copies once a tile, and what it
@@ -258,11 +258,12 @@ __device__ __forceinline__ double int_to_double(long long T, int e) {
   const unsigned long long a = T < 0 ? 0ull - (unsigned long long)T : (unsigned long long)T;
   const int lz = __clzll((long long)a);
   const unsigned long long m = a << (lz & 63);
-  const unsigned long long q = (m >> 11) + ((m >> 10) & 1ull);  // 2^52 .. 2^53
-  const int E = 1023 + 63 - 1 + e - lz;                          // the exponent field, less what q brings
-  unsigned long long b = E >= 0 ? ((unsigned long long)E << 52) + q : q >> min(-E, 63);
+  const int E = 1023 + 63 - 1 + e - lz;  // the exponent field, less what q brings
+  const int r = 11 - max(min(E, 0), -53);
+  const unsigned long long q = ((m >> (r - 1)) + 1) >> 1;  // 2^52 .. 2^53, less where E < 0
+  unsigned long long b = ((unsigned long long)max(E, 0) << 52) + q;
   if (E > 2045) b = 0x7ff0000000000000ull;
-  if (!a) b = 0;
+  if (!a || E < -53) b = 0;
   b |= (unsigned long long)T & 0x8000000000000000ull;
   if (e > oz::EXP_BAD / 2) b = 0x7ff8000000000000ull;
   return __longlong_as_double((long long)b);
