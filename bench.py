@@ -8,13 +8,14 @@ One step = one full solve: assemble the BEM matrix (warm: the
 frequency-independent near-pair table is built once, before timing), factor,
 solve the 4 right-hand sides and refine to 1e-10 relative residual.
 
-  python bench.py [--gpus N] [--steps K] [--warmup W] [--impl gbem|reference]
+  python bench.py [--gpus N] [--steps K] [--warmup W] [--impl gbem|reference|cpu]
 
-Prints one JSON line.  --impl reference times the CPU implementation of the
-path on all host cores (the oracle port of the reference's assembly and
-LAPACK's zgetrf/zgetrs; the reference binary built from its sources does not
-exist on the GPU host): one full-size solve cut into W + K slices, each step
-a real part of it (oracle/cpu_solve.py).
+Prints one JSON line.  --impl reference says that the unmodified reference is not
+available: it is a C++ project without a Python package, so nothing of it can be
+installed for this script to call.  --impl cpu times the repository's own CPU
+restatement of the path on all host cores (the oracle's assembly and LAPACK's
+zgetrf/zgetrs): one full-size solve cut into W + K slices, each step a real
+part of it (oracle/cpu_solve.py).
 """
 from __future__ import annotations
 
@@ -176,7 +177,15 @@ def cpu_sample(cores, subdiv=4):
 
 
 def run_reference(args):
-    """The reference's CPU path on all host cores (oracle assembly with
+    """The unmodified reference's arm: not available."""
+    if int(os.environ.get("RANK", "0")) == 0:
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "HomerReid/scuff-em is a C++ autotools project without a Python package: pip has nothing to "
+                          "install, and its libraries are not on this machine (--impl cpu times the CPU restatement)"}))
+
+
+def run_cpu(args):
+    """The path on all host cores (oracle assembly with
     OpenMP, LAPACK LU from OpenBLAS): one full-size solve cut into W + K
     slices.  Every step assembles a column stripe holding 1/(W+K) of the
     upper triangle's edge pairs (warm: the near-pair integrals are memoised
@@ -226,7 +235,7 @@ def run_reference(args):
     print(json.dumps({"metric": METRIC, "value": v, "unit": "solves/s", "n_gpus": args.gpus, "steps": K,
                       "warmup": W, "ms_per_step": ms_step, "higher_is_better": True,
                       "scaling": "weak", "vs_baseline": None, "dtype": "c128", "data": "synthetic",
-                      "impl": "reference", "cpu_baseline": cb,
+                      "impl": "cpu", "cpu_baseline": cb,
                       "e2e": {"value": v, "unit": "solves/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
                       "config": bench_config(args.subdiv, job.N, 4, args.gpus),
                       "method": "oracle port of the reference's assembly (OpenMP) + LAPACK zgetrf/zgetrs "
@@ -387,7 +396,7 @@ def main():
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--steps", type=int, default=5)
     ap.add_argument("--warmup", type=int, default=3)
-    ap.add_argument("--impl", default="gbem", choices=["gbem", "reference"])
+    ap.add_argument("--impl", default="gbem", choices=["gbem", "reference", "cpu"])
     ap.add_argument("--subdiv", type=int, default=4)
     ap.add_argument("--pec", action="store_true",
                     help="a PEC sphere instead of the dielectric one (N = 30 * 4^s; for profiling runs)")
@@ -402,6 +411,8 @@ def main():
         args.no_fp64 = True  # the accuracy report assumes the dielectric's K/N interleaving
     if args.impl == "reference":
         return run_reference(args)
+    if args.impl == "cpu":
+        return run_cpu(args)
     if args.workload == "batch":
         return run_batch(args)
     if args.workload == "large":

@@ -34,3 +34,16 @@ def test_slices_cover_one_solve():
     from oracle import oracle
     M = oracle.assemble([job.S], [(0, 1)], [False], job.omega, job.eps, [1.0, 1.0])
     assert np.array_equal(np.triu(job.M), np.triu(M))
+
+
+def test_reference_arm_says_it_is_unavailable():
+    """bench.py's reference arm never times anything else in its place."""
+    import json
+    import os
+    import subprocess
+    import sys
+    repo = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, os.path.join(repo, "bench.py"), "--impl", "reference", "--gpus", "1", "--steps", "2",
+                          "--warmup", "1"], check=True, capture_output=True, text=True, timeout=300).stdout
+    line = json.loads(out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
