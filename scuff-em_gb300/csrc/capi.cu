@@ -1285,6 +1285,17 @@ __global__ void add_c128(double2* x, const double2* d, size_t n) {
   if (i < n) { x[i].x += d[i].x; x[i].y += d[i].y; }
 }
 
+// the largest |r| / |b| of the columns, from their squares; infinite where one is
+// not a number (which would compare as converged)
+static double worst_residual(const std::vector<double>& rn, const std::vector<double>& bn) {
+  double rel = 0.0;
+  for (size_t c = 0; c < rn.size(); c++) {
+    const double q = std::sqrt(rn[c] / (bn[c] > 0 ? bn[c] : 1.0));
+    rel = q >= rel ? q : std::isnan(q) ? INFINITY : rel;
+  }
+  return rel;
+}
+
 // GMRES-based refinement, for matrices whose conditioning defeats plain
 // refinement with the complex64 factor (kappa(A) u_f >~ 1: low frequencies,
 // fine meshes).  Each outer step solves the correction equation A d = r,
@@ -1333,8 +1344,7 @@ static gbem_status gmres_refine(const void* dA, int adtype, gbem_matrix* F, int 
     cudaError_t ee = cudaMemcpyAsync(rn.data(), dn, sizeof(double) * nrhs, cudaMemcpyDeviceToHost, s);
     if (ee == cudaSuccess) ee = cudaStreamSynchronize(s);
     if (ee != cudaSuccess) return cuda_status(ee, "GMRES residual");
-    *rel = 0.0;
-    for (int r = 0; r < nrhs; r++) *rel = std::fmax(*rel, std::sqrt(rn[r] / (bn[r] > 0 ? bn[r] : 1.0)));
+    *rel = worst_residual(rn, bn);
     return GBEM_OK;
   };
   double rel = *rel_out;
@@ -1548,8 +1558,7 @@ static gbem_status solve_mixed_impl(gbem_geometry* g, double omega_re, double om
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
       if (e != cudaSuccess) { st = cuda_status(e, "refinement"); break; }
       it++;
-      rel = 0;
-      for (int r = 0; r < nrhs; r++) rel = std::fmax(rel, std::sqrt(rn[r] / (bn[r] > 0 ? bn[r] : 1.0)));
+      rel = worst_residual(rn, bn);
       if (rel <= tol) return true;
       if (sw >= 1 && !(rel < 0.2 * prev)) return false;
       prev = rel;
@@ -1579,8 +1588,9 @@ static gbem_status solve_mixed_impl(gbem_geometry* g, double omega_re, double om
       tc_gemm_thread_off(0);
     }
     if (st == GBEM_OK) ok = refine(max_iter);
-    // then GMRES-based refinement preconditioned by that factor
-    if (st == GBEM_OK && !ok)
+    // then GMRES-based refinement preconditioned by that factor (which cannot
+    // start from a residual that is not finite)
+    if (st == GBEM_OK && !ok && std::isfinite(rel))
       st = gmres_refine(dA, adt, F, N, nrhs, (const double2*)dB, (double2*)dX, (double2*)dR, (float2*)dD, dY, part, bn,
                         tol, max_iter, &it, &rel, s);
   }

@@ -282,3 +282,23 @@ def test_triangular_solve_that_gives_up_says_so(spins, want):
                          env=dict(os.environ, GBEM_TRSV_SPINS=spins), check=True, timeout=600, capture_output=True,
                          text=True).stdout.split()
     assert out == [want] * 7
+
+
+@pytest.mark.parametrize("which", ["frequency", "right-hand side", "second right-hand side"])
+@pytest.mark.parametrize("refined", [False, True])
+def test_solution_that_is_not_a_number_is_not_converged(which, refined):
+    """A residual that is not a number does not count as below the tolerance: it
+    is reported as infinite (the status is GBEM_ENOCONV, which the Python calls
+    leave to their caller's look at the residual)."""
+    from gbem import RWGGeometry, mesh
+    V, P = mesh.icosphere(1)
+    G = RWGGeometry([{"V": V, "P": P, "material": None}])
+    rng = np.random.default_rng(0)
+    B = rng.standard_normal((G.TotalBFs, 2)) + 1j * rng.standard_normal((G.TotalBFs, 2))
+    if which != "frequency":
+        B[3, 0 if which == "right-hand side" else 1] = np.nan
+    solve = G.solve_refined if refined else G.solve_mixed
+    X, it, res = solve(complex(np.nan, 0.0) if which == "frequency" else 1.0, B, tol=1e-10, max_iter=5)
+    assert res == np.inf and not np.isfinite(X).all()
+    X, it, res = solve(1.0, np.nan_to_num(B), tol=1e-10, max_iter=8)
+    assert res <= 1e-10 and np.isfinite(X).all()
